@@ -524,6 +524,29 @@ def test_large_m_many_waves():
     assert np.abs(vals - want).max() <= cc.TOL_16BIT * np.abs(want).max()
 
 
+# --------------------------------------------------------------------------- channel counts that no k-chunk divides
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("c_bytes", [32, 48, 64, 80, 112, 128, 144, 240, 272])
+@pytest.mark.parametrize("r,s,stride", [(3, 3, 1), (1, 1, 1), (2, 3, 2)])
+def test_ragged_channel_counts(c_bytes, r, s, stride, dtype):
+    """Rows of channels either side of every k-chunk width (32, 64, 128 bytes and more than one chunk). The weights after a
+    tap's last channel are another tap's, so one infinite weight must reach only the outputs whose tap it is."""
+    C = c_bytes // (4 if dtype == "f32" else 2)
+    x = cc.uniform((2, C, 9, 11), 21, "rag/x", 0.1, 1.0)
+    w = cc.kaiming((72, C, r, s), 21, "rag/w")
+    b = cc.normal((72,), 21, "rag/b", 0.1)
+    check(x, w, b, None, stride, (r // 2, s // 2), 1, "bias+relu", dtype)
+    w[5, 0, r - 1, s - 1] = np.inf             # first channel of the last tap: right behind the tap before it
+    got = run_gpu(x, w, b, None, stride, (r // 2, s // 2), 1, "bias", dtype)
+    hit = np.zeros((2, 1, 9, 11), np.float32) + 1
+    ones = np.zeros((1, 1, r, s), np.float32)
+    ones[0, 0, r - 1, s - 1] = 1
+    reached = oracle.conv2d(hit, ones, None, None, stride, (r // 2, s // 2), 1, "none")[:, 0] != 0
+    # padding pixels are zeros: 0 * inf is NaN where the tap lies outside the image, inf where it does not
+    assert np.isposinf(got[:, 5][reached]).all() and np.isnan(got[:, 5][~reached]).all()
+    assert np.isfinite(np.delete(got, 5, axis=1)).all()
+
+
 # --------------------------------------------------------------------------- tiles split over K (opt-in schedule)
 _SPLIT_K_SCRIPT = r"""
 import sys

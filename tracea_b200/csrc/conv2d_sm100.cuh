@@ -66,15 +66,17 @@ struct ConvKernelArgs {
   // k-chunking: one chunk = chunk_elems channels of one tap
   int chunk_elems;        // elements per chunk (chunk_bytes / element size)
   int chunk_bytes;        // 128, 64, 32 or 16
-  int chunks_per_tap;     // C / chunk_elems
+  int chunks_per_tap;     // ceil(C / chunk_elems); the last chunk's channels past C read zeros on both sides
   int total_chunks;       // R * S * chunks_per_tap
-  int C;                  // input channels (c coordinate >= C reads zeros)
+  int C;                  // chunks_per_tap * chunk_elems (c coordinate >= C reads zeros)
   int a_tiled;            // 1: A is a plain [M][C] matrix (1x1, stride 1, no padding) read by tiled TMA
-  // B's column (element index inside one output channel's weight row) of tap (r, s), channel c is
-  // b_k0 + r * (row stride) + s * (tap stride) + c. The loader walks it incrementally: +chunk_elems per k-step,
-  // +b_jump_s at every tap boundary, +b_jump_r more at every filter-row boundary. Dense [R][S][C] rows: all 0.
-  // Non-zero jumps are only used with 128-byte chunks (one chunk per stage).
-  int b_k0, b_jump_s, b_jump_r;
+  // B is a 3-D map {column, tap, output channel}. The loader walks the column incrementally: +chunk_elems per k-step,
+  // +b_jump_s at every tap boundary, +b_jump_r more at every filter-row boundary; the tap coordinate moves by
+  // b_tap_step at a tap boundary. Three forms: taps contiguous in one row, all jumps and b_tap_step 0; channel counts
+  // that no k-chunk divides, one map row per tap (b_tap_step 1, b_jump_s back to column 0), so that the last chunk of a
+  // tap ends in zeros instead of in the next tap's weights; taps at any stride of the row, from column b_k0 with jumps
+  // (only used with 128-byte chunks, one chunk per stage).
+  int b_k0, b_jump_s, b_jump_r, b_tap_step;
   // tiling / pipeline
   int num_m_tiles, num_n_tiles;
   int panel_width;  // column tiles per panel of the tile order (>= 1; num_n_tiles = one panel = row-major order)
@@ -779,7 +781,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
         if (one_chunk) {
           // common case: one 128-byte chunk per stage = 64 (16-bit) or 32 (fp32) channels of one tap.
           // Position of k-step k_begin: tap (r, s), channel chunk cc (a whole tile starts at 0, 0, 0)
-          int c_coord = 0, k_coord = args.b_k0, tap_s = 0;
+          int c_coord = 0, k_coord = args.b_k0, tap_s = 0, tap_coord = 0;
           uint32_t off_w = 0, off_h = 0;
           if (item.k_begin != 0) {
             const int tap = item.k_begin / args.chunks_per_tap;
@@ -790,6 +792,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
             off_w = static_cast<uint32_t>(tap_s * args.dil_w);
             off_h = static_cast<uint32_t>(tap_r * args.dil_h);
             k_coord += item.k_begin * args.chunk_elems + tap * args.b_jump_s + tap_r * args.b_jump_r;
+            tap_coord = tap * args.b_tap_step;
           }
           for (int it = item.k_begin; it < item.k_end; ++it) {
             if (issued == args.test_producer_stop) {   // test hook: go silent, leave normally
@@ -812,16 +815,16 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               next_free = tma_stage_probe_pair(stage_addr, stage_addr + kABytes, full_addr,
                                                full_leader0 + (full_addr - full_bar0), leader ? 2u * kStageBytes : 0u,
                                                &tmap_x, c_coord, w_start, h_start, img0, (uint16_t)off_w,
-                                               (uint16_t)off_h, &tmap_w, k_coord, n_coord, nempty, nphase ^ 1u);
+                                               (uint16_t)off_h, &tmap_w, k_coord, tap_coord, n_coord, nempty, nphase ^ 1u);
             } else if constexpr (kRows2) {
               next_free = tma_stage_probe_rows2(stage_addr, stage_addr + kABlockBytes, stage_addr + kABytes, full_addr,
                                                 kStageBytes, &tmap_x, c_coord, w_start, h_start, img0, w_start1,
                                                 h_start1, img1, (uint16_t)off_w, (uint16_t)off_h, &tmap_w, k_coord,
-                                                n_coord, nempty, nphase ^ 1u);
+                                                tap_coord, n_coord, nempty, nphase ^ 1u);
             } else {
               next_free = tma_stage_probe(stage_addr, stage_addr + kABytes, full_addr, kStageBytes, &tmap_x, c_coord,
                                           w_start, h_start, img0, (uint16_t)off_w, (uint16_t)off_h, &tmap_w, k_coord,
-                                          n_coord, nempty, nphase ^ 1u);
+                                          tap_coord, n_coord, nempty, nphase ^ 1u);
             }
             k_coord += args.chunk_elems;
             c_coord += args.chunk_elems;
@@ -829,6 +832,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               c_coord = 0;
               off_w += args.dil_w;
               k_coord += args.b_jump_s;
+              tap_coord += args.b_tap_step;
               if (++tap_s == args.S) { tap_s = 0; off_w = 0; off_h += args.dil_h; k_coord += args.b_jump_r; }
             }
             ++issued;
@@ -837,7 +841,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
           }
         } else {
           // narrow k-chunks (several per stage): whole tiles only, the host never splits these over K
-          int chunk = 0, tap_r = 0, tap_s = 0, cc = 0;
+          int chunk = 0, tap_r = 0, tap_s = 0, cc = 0, b_col = 0, tap_coord = 0;
           for (int it = 0; it < k_iters; ++it) {
             if (!mbar_wait_bounded(empty_addr, phase ^ 1u, abort_p, args.wait_limit)) {
               report_error(args, abort_p, kErrProducerWait, (uint32_t)it);
@@ -851,8 +855,8 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               // chunks past the end of Kgemm read zeros: channel coordinate C / column Kgemm are out of range
               const bool pad_chunk = chunk >= args.total_chunks;
               const int c_coord = pad_chunk ? args.C : cc * args.chunk_elems;
-              const int k_coord = pad_chunk ? args.total_chunks * args.chunk_elems
-                                            : chunk * args.chunk_elems;
+              // (the last tap's row ends at or before column args.C, a single contiguous row at total_chunks chunks)
+              const int k_coord = pad_chunk ? args.total_chunks * args.chunk_elems : b_col;
               if (args.a_tiled) {
                 tma_load_2d(a_dst + j * a_chunk_bytes, &tmap_x, full_addr, c_coord, m0);
               } else {
@@ -860,10 +864,13 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
                                    w_start, h_start, img0, (uint16_t)(tap_s * args.dil_w),
                                    (uint16_t)(tap_r * args.dil_h));
               }
-              tma_load_2d(b_dst + j * b_chunk_bytes, &tmap_w, full_addr, k_coord, n_coord);
+              tma_load_3d(b_dst + j * b_chunk_bytes, &tmap_w, full_addr, k_coord, tap_coord, n_coord);
               if (!pad_chunk) {
+                b_col += args.chunk_elems;
                 if (++cc == args.chunks_per_tap) {
                   cc = 0;
+                  b_col += args.b_jump_s;
+                  tap_coord += args.b_tap_step;
                   if (++tap_s == args.S) { tap_s = 0; ++tap_r; }
                 }
               }

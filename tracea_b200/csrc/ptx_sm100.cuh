@@ -177,6 +177,16 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint
       : "memory");
 }
 
+// Tiled 3-D load: coordinates {c0 (innermost), c1, c2}.
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      :
+      : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+
 // im2col-mode 4-D load over an NHWC tensor: coordinates {c, w, h, n} give the first base pixel
 // (already including the negative padding corner), {off_w, off_h} the filter-tap offset.
 __device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const void* tmap, uint32_t bar,
@@ -395,25 +405,25 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
 __device__ __forceinline__ bool tma_stage_probe_pair(uint32_t a_dst, uint32_t b_dst, uint32_t full_bar_local,
                                                      uint32_t full_bar_leader, uint32_t expect_bytes,
                                                      const void* tmap_x, int c, int w, int h, int n, uint16_t off_w,
-                                                     uint16_t off_h, const void* tmap_w, int k0, int n0,
+                                                     uint16_t off_h, const void* tmap_w, int k0, int tap, int n0,
                                                      uint32_t next_empty_bar, uint32_t next_parity) {
   uint32_t free_next;
   asm volatile(
       "{\n"
       ".reg .pred pn, pl;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 pn, [%16], %17;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 pn, [%17], %18;\n"
       "setp.ne.b32 pl, %4, 0;\n"
       "@pl mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %4;\n"
       "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
       " [%1], [%6, {%7, %8, %9, %10}], [%5], {%11, %12};\n"
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%2], [%13, {%14, %15}], [%5];\n"
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%2], [%13, {%14, %15, %16}], [%5];\n"
       "selp.u32 %0, 1, 0, pn;\n"
       "}\n"
       : "=r"(free_next)
       : "r"(a_dst), "r"(b_dst), "r"(full_bar_local), "r"(expect_bytes), "r"(full_bar_leader),
         "l"(reinterpret_cast<uint64_t>(tmap_x)), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h),
-        "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(n0), "r"(next_empty_bar), "r"(next_parity)
+        "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(tap), "r"(n0), "r"(next_empty_bar), "r"(next_parity)
       : "memory");
   return free_next != 0;
 }
@@ -423,24 +433,24 @@ __device__ __forceinline__ bool tma_stage_probe_pair(uint32_t a_dst, uint32_t b_
 // of B, then read the probe.
 __device__ __forceinline__ bool tma_stage_probe(uint32_t a_dst, uint32_t b_dst, uint32_t full_bar, uint32_t stage_bytes,
                                                 const void* tmap_x, int c, int w, int h, int n, uint16_t off_w,
-                                                uint16_t off_h, const void* tmap_w, int k0, int n0,
+                                                uint16_t off_h, const void* tmap_w, int k0, int tap, int n0,
                                                 uint32_t next_empty_bar, uint32_t next_parity) {
   uint32_t free_next;
   asm volatile(
       "{\n"
       ".reg .pred pn;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 pn, [%15], %16;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 pn, [%16], %17;\n"
       "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %4;\n"
       "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
       " [%1], [%5, {%6, %7, %8, %9}], [%3], {%10, %11};\n"
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%2], [%12, {%13, %14}], [%3];\n"
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%2], [%12, {%13, %14, %15}], [%3];\n"
       "selp.u32 %0, 1, 0, pn;\n"
       "}\n"
       : "=r"(free_next)
       : "r"(a_dst), "r"(b_dst), "r"(full_bar), "r"(stage_bytes), "l"(reinterpret_cast<uint64_t>(tmap_x)), "r"(c),
-        "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h), "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(n0),
-        "r"(next_empty_bar), "r"(next_parity)
+        "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h), "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(tap),
+        "r"(n0), "r"(next_empty_bar), "r"(next_parity)
       : "memory");
   return free_next != 0;
 }
@@ -450,26 +460,26 @@ __device__ __forceinline__ bool tma_stage_probe(uint32_t a_dst, uint32_t b_dst, 
 __device__ __forceinline__ bool tma_stage_probe_rows2(uint32_t a0_dst, uint32_t a1_dst, uint32_t b_dst,
                                                       uint32_t full_bar, uint32_t stage_bytes, const void* tmap_x,
                                                       int c, int w0, int h0, int n0i, int w1, int h1, int n1i,
-                                                      uint16_t off_w, uint16_t off_h, const void* tmap_w, int k0,
+                                                      uint16_t off_w, uint16_t off_h, const void* tmap_w, int k0, int tap,
                                                       int ncol, uint32_t next_empty_bar, uint32_t next_parity) {
   uint32_t free_next;
   asm volatile(
       "{\n"
       ".reg .pred pn;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 pn, [%19], %20;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 pn, [%20], %21;\n"
       "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n"
       "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
       " [%1], [%6, {%7, %8, %9, %10}], [%4], {%14, %15};\n"
       "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
       " [%2], [%6, {%7, %11, %12, %13}], [%4], {%14, %15};\n"
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%3], [%16, {%17, %18}], [%4];\n"
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%3], [%16, {%17, %18, %19}], [%4];\n"
       "selp.u32 %0, 1, 0, pn;\n"
       "}\n"
       : "=r"(free_next)
       : "r"(a0_dst), "r"(a1_dst), "r"(b_dst), "r"(full_bar), "r"(stage_bytes), "l"(reinterpret_cast<uint64_t>(tmap_x)),
         "r"(c), "r"(w0), "r"(h0), "r"(n0i), "r"(w1), "r"(h1), "r"(n1i), "h"(off_w), "h"(off_h),
-        "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(ncol), "r"(next_empty_bar), "r"(next_parity)
+        "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(tap), "r"(ncol), "r"(next_empty_bar), "r"(next_parity)
       : "memory");
   return free_next != 0;
 }

@@ -378,6 +378,18 @@ int pick_bn(long long m_tiles, int k_out, int num_sms) {
   return best;
 }
 
+// Bytes of one pixel's channels per copy (the width of a k-chunk). A tap of row_bytes takes ceil(row_bytes / chunk)
+// chunks, and what the last one brings in past the channels is zeros. The TMA unit's rate is in rows, not bytes -- a
+// 64-byte and a 128-byte chunk cost it the same -- so the widest chunk wins although it is partly padding: 3x3 C->128 on
+// 32 images of 28x28 in chunks of 128 / 64 / 32 / 16 bytes: C = 96 (192-byte rows) 12.8 / 18.3 / 28.6 / 46.0 us, C = 112
+// 13.9 / 22.2 / 32.1 / 51.7, C = 48 10.5 / 14.1 / 16.9 / 25.6. Rows that fit a narrower chunk whole take that, which saves
+// the tensor work on the padding (C = 24: 14.7 us in 64-byte chunks, 19.8 in 128-byte ones).
+int pick_chunk_bytes(long long row_bytes) {
+  int chunk = 16;
+  while (chunk < 128 && chunk < row_bytes) chunk *= 2;
+  return chunk;
+}
+
 int pick_stages(int bn, bool pair, bool rows2, bool shared_bias) {
   const int stage_bytes = tb200::conv_smem_bytes(bn, 1, pair, rows2) - tb200::conv_smem_bytes(bn, 0, pair, rows2);
   const int fixed = tb200::conv_smem_bytes(bn, 0, pair, rows2, shared_bias);
@@ -1052,24 +1064,19 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     x.stride[3] = Cp;
   }
 
-  // ---- k-chunking: the widest power-of-two row (<= 128 B) that divides one pixel's channels
+  // ---- k-chunking: how many bytes of one pixel's channels one copy brings in (see pick_chunk_bytes)
   // In window mode the kernel sees a conv with one tap per filter row over "pixels" of 8 * Cp channels.
   const long long Cg = window ? 8 * Cp : Cp;      // channel extent of the kernel's view
   const long long Sg = window ? 1 : S;            // taps per filter row of the kernel's view
   const long long row_bytes = Cg * es;
-  int chunk_bytes = 16;
-  for (int cb = 128; cb >= 16; cb >>= 1) {
-    if (row_bytes % cb == 0) {
-      chunk_bytes = cb;
-      break;
-    }
-  }
+  int chunk_bytes = pick_chunk_bytes(row_bytes);
   const int forced_chunk = knobs().force_chunk;
-  if (forced_chunk == 16 || forced_chunk == 32 || forced_chunk == 64 || forced_chunk == 128) {
-    if (row_bytes % forced_chunk == 0) chunk_bytes = forced_chunk;
-  }
+  if (forced_chunk == 16 || forced_chunk == 32 || forced_chunk == 64 || forced_chunk == 128) chunk_bytes = forced_chunk;
   const int chunk_elems = chunk_bytes / es;
-  const int chunks_per_tap = static_cast<int>(Cg / chunk_elems);
+  const int chunks_per_tap = static_cast<int>((Cg + chunk_elems - 1) / chunk_elems);
+  // the last chunk of a tap is partly past the channels: fine for the activations (the TMA unit fills channels >= C with
+  // zeros), but the weights then need a map with one row per tap, unless there is only one tap
+  const bool ragged_taps = row_bytes % chunk_bytes != 0 && R * Sg > 1;
   const long long total_chunks_ll = R * Sg * chunks_per_tap;
   if (total_chunks_ll > 0x7fffffffLL / 128) TB_FAIL(TRACEA_UNSUPPORTED_CONFIG, "R*S*C too large");
 
@@ -1084,7 +1091,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   const bool w_dense = C == Cp && (w_in.stride[1] == 1) && w_in.stride[3] == C &&
                        w_in.stride[2] == S * C && w_in.stride[0] == R * S * C && aligned16(w_in.ptr);
   bool w_direct = w_dense, w_remap = false;
-  if (!w_dense && !window && C == Cp && w_in.stride[1] == 1 && chunk_bytes == 128) {
+  if (!w_dense && !window && C == Cp && w_in.stride[1] == 1 && chunk_bytes == 128 && !ragged_taps) {
     const long long ss = S == 1 ? C : w_in.stride[3], sr = R == 1 ? S * ss : w_in.stride[2], sk = w_in.stride[0];
     const long long lo = std::min(0LL, (R - 1) * sr) + std::min(0LL, (S - 1) * ss);
     const long long hi = std::max(0LL, (R - 1) * sr) + std::max(0LL, (S - 1) * ss) + C;
@@ -1201,12 +1208,13 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   a.chunk_bytes = chunk_bytes;
   a.chunks_per_tap = chunks_per_tap;
   a.total_chunks = static_cast<int>(total_chunks_ll);
-  a.C = static_cast<int>(Cg);
+  a.C = chunks_per_tap * chunk_elems;
   a.a_tiled = a_tiled ? 1 : 0;
   a.num_n_tiles = static_cast<int>(n_tiles);
   a.b_k0 = static_cast<int>(b_k0);
-  a.b_jump_s = static_cast<int>(b_jump_s);
+  a.b_jump_s = ragged_taps ? -chunks_per_tap * chunk_elems : static_cast<int>(b_jump_s);
   a.b_jump_r = static_cast<int>(b_jump_r);
+  a.b_tap_step = ragged_taps ? 1 : 0;
   // K-major operand descriptors. Swizzled rows of chunk_bytes: 8-row groups are 8*chunk_bytes apart
   // (SBO) and one MMA (32 B of K) stays inside a row. Unswizzled 16-byte chunks: an 8-row x 16 B core
   // matrix is 128 contiguous bytes (SBO) and the MMA's second K half is the next chunk (LBO).
@@ -1324,12 +1332,15 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     const int smem = tb200::conv_smem_bytes(bn, stages, pair_v, rows2_v, shared_bias);
 
     CUtensorMap tmap_w;
-    // repacked or dense weights: one row is the whole Kgemm axis; in-place strided taps: one row spans the taps
-    const cuuint64_t gdim[2] = {(cuuint64_t)(w_remap ? w_row_elems : Kgemm), (cuuint64_t)K};
-    const cuuint64_t gstr[1] = {(cuuint64_t)((w_remap ? w_pitch : Kgemm) * es)};
-    const cuuint32_t box[2] = {(cuuint32_t)chunk_elems, (cuuint32_t)(pair_v ? bn / 2 : bn)};
-    const cuuint32_t estr[2] = {1u, 1u};
-    CUresult r = g_encode_tiled(&tmap_w, tmap_dtype(x.dtype), 2, const_cast<void*>(w_ptr), gdim, gstr,
+    // {column, tap, output channel}. Repacked or dense weights: one row is the whole Kgemm axis, or one tap of it when
+    // the k-chunks do not divide a tap; in-place strided taps: one row spans the taps
+    const long long row_elems = w_remap ? w_row_elems : (ragged_taps ? Cg : Kgemm);
+    const long long k_pitch = w_remap ? w_pitch : Kgemm;
+    const cuuint64_t gdim[3] = {(cuuint64_t)row_elems, (cuuint64_t)(ragged_taps ? R * Sg : 1), (cuuint64_t)K};
+    const cuuint64_t gstr[2] = {(cuuint64_t)((ragged_taps ? Cg : k_pitch) * es), (cuuint64_t)(k_pitch * es)};
+    const cuuint32_t box[3] = {(cuuint32_t)chunk_elems, 1u, (cuuint32_t)(pair_v ? bn / 2 : bn)};
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    CUresult r = g_encode_tiled(&tmap_w, tmap_dtype(x.dtype), 3, const_cast<void*>(w_ptr), gdim, gstr,
                                 box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, tmap_swizzle(chunk_bytes),
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
