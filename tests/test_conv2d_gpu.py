@@ -547,6 +547,40 @@ def test_ragged_channel_counts(c_bytes, r, s, stride, dtype):
     assert np.isfinite(np.delete(got, 5, axis=1)).all()
 
 
+# --------------------------------------------------------------------------- outputs that are not 16-byte aligned rows
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("channels_last", [True, False], ids=["nhwc", "nchw"])
+@pytest.mark.parametrize("K", [1, 3, 4, 5, 7, 15, 18, 31, 33, 63, 66, 129, 258])
+def test_output_widths_in_both_memory_formats(K, channels_last, dtype):
+    """Every way the epilogue stores: whole aligned rows, rows in 4-byte and single-element accesses, pixel by pixel, and
+    four NCHW pixels at a time -- output planes of 8x8 (multiple of 4), 6x7 (even) and 5x9 (odd) pixels -- with a residual
+    in the same memory."""
+    for h, w_ in ((8, 8), (6, 7), (5, 9)):
+        x = cc.uniform((3, 64, h, w_), 22, "ow/x")
+        w = cc.kaiming((K, 64, 3, 3), 22, "ow/w")
+        b = cc.normal((K,), 22, "ow/b", 0.1)
+        res = cc.normal((3, K, h, w_), 22, "ow/res")
+        check(x, w, b, res, 1, 1, 1, "bias+residual+relu", dtype, channels_last=channels_last, out_channels_last=channels_last)
+        check(x, w, b, None, 1, 1, 1, "gelu", dtype, channels_last=channels_last, out_channels_last=channels_last)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("offset,K,pitch", [(1, 40, 64), (2, 40, 66), (1, 41, 43), (8, 64, 72)])
+def test_unaligned_output_and_residual_views(offset, K, pitch, dtype):
+    """The output and the residual are channel slices of wider NHWC buffers that start at any element."""
+    x = cc.uniform((2, 64, 7, 9), 23, "uo/x")
+    w = cc.kaiming((K, 64, 3, 3), 23, "uo/w")
+    res = cc.normal((2, K, 7, 9), 23, "uo/r")
+    big = torch.full((2, pitch + offset, 7, 9), 7.0, dtype=TORCH_DT[dtype], device="cuda").contiguous(memory_format=torch.channels_last)
+    rbig = torch.zeros_like(big)
+    rview, view = rbig[:, offset:offset + K], big[:, offset:offset + K]
+    rview.copy_(to_dev(res, dtype))
+    ops.conv2d_into(to_dev(x, dtype), to_dev(w, dtype), view, None, rview, 1, 1, epilogue=ffi.EPILOGUE_RESIDUAL_RELU)
+    want = run_oracle(x, w, None, res, 1, 1, 1, "residual+relu", dtype)
+    assert cc.rel_err(view.float().cpu().numpy(), want) <= cc.tol_for(dtype)
+    assert (big[:, :offset] == 7.0).all() and (big[:, offset + K:] == 7.0).all()
+
+
 # --------------------------------------------------------------------------- tiles split over K (opt-in schedule)
 _SPLIT_K_SCRIPT = r"""
 import sys

@@ -101,15 +101,14 @@ struct ConvKernelArgs {
   // channels-last (sc == 1) and NCHW (sw == 1) memory are written without a transpose pass.
   void* out;
   long long out_sn, out_sh, out_sw, out_sc;
-  int out_vec;            // sc == 1 and 16-byte vector stores are legal
+  int out_vec;            // kStoreRows: bytes a lane may store at once (16, 4, or one element)
+  int out_quad;           // kStoreStrided: four consecutive pixels are always 8 consecutive, aligned bytes (16-bit types)
   const void* bias;       // [K_out], fp32 or OutT
   int bias_is_f32;
   const void* residual;   // same dtype as out
   long long res_sn, res_sh, res_sw, res_sc;
-  int res_vec;
+  int res_vec;            // as out_vec, for the residual
   int act;
-  int out_tma;            // 1: out is dense row-major [M][pitch] and is written by TMA stores
-  int res_tma;            // 1: residual is dense row-major too and is TMA-loaded into the staging boxes
   // error reporting: 4 words {code, block, detail, 0}; first error wins
   uint32_t* status;
   long long wait_limit;   // cycles any single wait may take before the role gives up (args.wait_limit unless a test shortens it)
@@ -303,37 +302,56 @@ __device__ __forceinline__ void add16(float* f, const uint4& raw) {
   for (int j = 0; j < kVec; ++j) f[j] += OutTraits<OutT>::to_f(e[j]);
 }
 
-// Out-of-line path for outputs / residuals the TMA boxes cannot address (NCHW or irregular
-// strides, K_out not a multiple of the vector width): finishes one 32-column block of one pixel --
-// residual, activation, store. `f` holds accumulator + bias. Kept out of line so that the common
-// path's instruction footprint stays small.
+// How a kernel's epilogue reaches the output (and the residual). One instantiation each: code for another form inside the
+// TMA kernels cost them registers, and a spilled register here goes all the way to L2.
+enum : int {
+  kStoreTma = 0,      // dense [M][pitch] rows: staging boxes, moved by the TMA unit
+  kStoreRows = 1,     // channel-contiguous, any pixel strides: the same boxes, moved by the warp itself
+  kStoreStrided = 2,  // anything else, NCHW above all: each lane stores its own pixel's channels
+};
+
+// Strided outputs: finishes one 32-column block of one pixel per lane -- residual, activation, store. `f` holds
+// accumulator + bias, `cols` how many of the columns exist; res_px / out_px point at the pixel's first column.
+// With pixels adjacent in memory (NCHW) a warp's store of one column covers 32 consecutive elements, 64 bytes at 16 bits:
+// that is bound by the number of store instructions, so where the host found four consecutive pixels always to be 8
+// aligned bytes (args.out_quad) the lanes transpose 4 pixels x 4 columns with shuffles first and store 8 bytes each,
+// 8 instructions in place of 32. (3x3 64->128 on one 222x222 fp16 NCHW image: 60.7 us with an out-of-line, element-wise
+// store, 25.0 us with this; 1x1 256->1024 with a residual on 32 images of 14x14: 189 -> 51 us.)
 template <typename OutT>
-__device__ __noinline__ void epilogue_block_generic(const ConvKernelArgs& args, float* f, const OutT* res_px,
-                                                    OutT* out_px, int n_first, bool row_ok) {
-  constexpr int kVec = 16 / sizeof(OutT);
+__device__ __forceinline__ void store_strided32(const ConvKernelArgs& args, float (&f)[32], const OutT* res_px, OutT* out_px,
+                                                int cols, bool row_ok, int lane) {
   if (res_px != nullptr && row_ok) {
-    if (args.res_vec) {
 #pragma unroll
-      for (int c = 0; c < 32 / kVec; ++c)
-        if (n_first + c * kVec < args.K_out) add16<OutT>(f + c * kVec, __ldg(reinterpret_cast<const uint4*>(res_px) + c));
-    } else {
-#pragma unroll 4
-      for (int j = 0; j < 32; ++j)
-        if (n_first + j < args.K_out) f[j] += OutTraits<OutT>::to_f(res_px[j * args.res_sc]);
+    for (int j = 0; j < 32; ++j)
+      if (j < cols) f[j] += OutTraits<OutT>::to_f(res_px[j * args.res_sc]);
+  }
+  apply_act32<sizeof(OutT) == 2>(f, args.act);
+  if constexpr (sizeof(OutT) == 2) {
+    if (args.out_quad) {
+      uint32_t w[16];                      // word k: columns 2k (low half) and 2k + 1 of this lane's pixel
+#pragma unroll
+      for (int k = 0; k < 16; ++k) w[k] = pack2<OutT, false>(f[2 * k], f[2 * k + 1]);
+      const bool odd = (lane & 1) != 0, upper = (lane & 2) != 0;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {       // -> pixels (lane & ~1, lane | 1) of column 2k + (lane & 1)
+        const uint32_t o = __shfl_xor_sync(0xffffffffu, w[k], 1);
+        w[k] = odd ? __byte_perm(o, w[k], 0x7632) : __byte_perm(w[k], o, 0x5410);
+      }
+      OutT* quad = out_px - (lane & 3);    // the quad's first pixel
+#pragma unroll
+      for (int k = 0; k < 16; k += 2) {    // -> all four pixels of column 2 (k + (lane >> 1 & 1)) + (lane & 1)
+        const uint32_t o = __shfl_xor_sync(0xffffffffu, upper ? w[k] : w[k + 1], 2);
+        const int col = 2 * (k + (upper ? 1 : 0)) + (odd ? 1 : 0);
+        if (row_ok && col < cols)
+          *reinterpret_cast<uint2*>(quad + col * args.out_sc) = upper ? make_uint2(o, w[k + 1]) : make_uint2(w[k], o);
+      }
+      return;
     }
   }
-  apply_act32<sizeof(OutT) == 2>(*reinterpret_cast<float(*)[32]>(f), args.act);
   if (!row_ok) return;
-  if (args.out_vec) {
 #pragma unroll
-    for (int c = 0; c < 32 / kVec; ++c)
-      if (n_first + c * kVec < args.K_out) reinterpret_cast<uint4*>(out_px)[c] = pack16<OutT>(f + c * kVec);
-  } else {
-    // lanes are consecutive pixels: for NCHW memory (sw == 1) each store instruction is coalesced
-#pragma unroll 4
-    for (int j = 0; j < 32; ++j)
-      if (n_first + j < args.K_out) out_px[j * args.out_sc] = OutTraits<OutT>::from_f(f[j]);
-  }
+  for (int j = 0; j < 32; ++j)
+    if (j < cols) out_px[j * args.out_sc] = OutTraits<OutT>::from_f(f[j]);
 }
 
 // kPair: launched as clusters of two CTAs (cta_group::2). The pair owns a 256 x BN tile: each CTA loads its own
@@ -347,7 +365,8 @@ __device__ __noinline__ void epilogue_block_generic(const ConvKernelArgs& args, 
 // <-> global memory, moved by the warp itself for outputs the TMA unit cannot address as one matrix. Lane l handles
 // chunk l & 7 of rows (l >> 3) + 4 i, so each instruction covers four whole 128-byte rows. `row_base` points at the
 // first element of the group's columns in pixel 0's row; `row_off` is this lane's own pixel offset (in elements),
-// `row_ok` whether its pixel exists; `cols_left` = K_out - first column of the group. Only instantiated in the kCoop kernels.
+// `row_ok` whether its pixel exists; `cols_left` = K_out - first column of the group. Only instantiated in
+// the kStoreRows kernels.
 template <typename OutT>
 __device__ __noinline__ void coop_store_box(uint32_t stg, OutT* row_base, long long row_off, bool row_ok, int cols_left,
                                             int lane) {
@@ -382,6 +401,67 @@ __device__ __noinline__ void coop_load_box(uint32_t stg, const OutT* row_base, l
     ptx::st_shared_v4(stg + static_cast<uint32_t>(r) * 128u + ((chunk ^ (static_cast<uint32_t>(r) & 7u)) << 4), v);
   }
   __syncwarp();   // rows were written by other lanes than the ones that read them next
+}
+
+// The same for pixel rows that are not all 16-byte aligned (an odd channel count above all): the warp walks the box row by
+// row, every lane moving sizeof(Word) bytes, so an instruction still covers 64 or 128 consecutive bytes of one row.
+template <typename OutT, typename Word>
+__device__ __noinline__ void coop_store_box_narrow(uint32_t stg, OutT* row_base, long long row_off, bool row_ok, int cols_left,
+                                                   int lane) {
+  constexpr int kPer = sizeof(Word) / sizeof(OutT);       // elements per lane and instruction
+  constexpr int kSegs = 128 / (32 * sizeof(Word));        // instructions per row
+  __syncwarp();
+  const uint32_t ok_rows = __ballot_sync(0xffffffffu, row_ok);
+#pragma unroll 8
+  for (int r = 0; r < 32; ++r) {
+    const long long off = __shfl_sync(0xffffffffu, row_off, r);
+#pragma unroll
+    for (int s = 0; s < kSegs; ++s) {
+      const uint32_t byte = static_cast<uint32_t>(s * 32 + lane) * sizeof(Word);
+      const uint32_t src = stg + static_cast<uint32_t>(r) * 128u + (((byte >> 4) ^ (static_cast<uint32_t>(r) & 7u)) << 4) + (byte & 15u);
+      if ((s * 32 + lane) * kPer < cols_left && ((ok_rows >> r) & 1u))
+        reinterpret_cast<Word*>(row_base + off)[s * 32 + lane] = ptx::ld_shared_word<Word>(src);
+    }
+  }
+  __syncwarp();
+}
+
+template <typename OutT, typename Word>
+__device__ __noinline__ void coop_load_box_narrow(uint32_t stg, const OutT* row_base, long long row_off, bool row_ok,
+                                                  int cols_left, int lane) {
+  constexpr int kPer = sizeof(Word) / sizeof(OutT);
+  constexpr int kSegs = 128 / (32 * sizeof(Word));
+  const uint32_t ok_rows = __ballot_sync(0xffffffffu, row_ok);
+#pragma unroll 8
+  for (int r = 0; r < 32; ++r) {
+    const long long off = __shfl_sync(0xffffffffu, row_off, r);
+#pragma unroll
+    for (int s = 0; s < kSegs; ++s) {
+      const uint32_t byte = static_cast<uint32_t>(s * 32 + lane) * sizeof(Word);
+      Word v = Word(0);
+      if ((s * 32 + lane) * kPer < cols_left && ((ok_rows >> r) & 1u))
+        v = reinterpret_cast<const Word*>(row_base + off)[s * 32 + lane];
+      ptx::st_shared_word<Word>(
+          stg + static_cast<uint32_t>(r) * 128u + (((byte >> 4) ^ (static_cast<uint32_t>(r) & 7u)) << 4) + (byte & 15u), v);
+    }
+  }
+  __syncwarp();
+}
+
+// `vec`: bytes per access that all rows allow -- 16, 4, or one element (ConvKernelArgs::out_vec / res_vec).
+template <typename OutT>
+__device__ __forceinline__ void store_rows(int vec, uint32_t stg, OutT* row_base, long long row_off, bool row_ok, int cols_left,
+                                           int lane) {
+  if (vec == 16) coop_store_box<OutT>(stg, row_base, row_off, row_ok, cols_left, lane);
+  else if (vec == 4) coop_store_box_narrow<OutT, uint32_t>(stg, row_base, row_off, row_ok, cols_left, lane);
+  else if constexpr (sizeof(OutT) == 2) coop_store_box_narrow<OutT, uint16_t>(stg, row_base, row_off, row_ok, cols_left, lane);
+}
+template <typename OutT>
+__device__ __forceinline__ void load_rows(int vec, uint32_t stg, const OutT* row_base, long long row_off, bool row_ok,
+                                          int cols_left, int lane) {
+  if (vec == 16) coop_load_box<OutT>(stg, row_base, row_off, row_ok, cols_left, lane);
+  else if (vec == 4) coop_load_box_narrow<OutT, uint32_t>(stg, row_base, row_off, row_ok, cols_left, lane);
+  else if constexpr (sizeof(OutT) == 2) coop_load_box_narrow<OutT, uint16_t>(stg, row_base, row_off, row_ok, cols_left, lane);
 }
 
 // One unit of work of a worker: k-steps [k_begin, k_end) of tile `tile`. A whole tile has k_begin == 0 and
@@ -623,7 +703,7 @@ __device__ __noinline__ void sk_reduce_many(const ConvKernelArgs& a, uint32_t ta
 // kSplit: the launch cuts some tiles over K (ConvKernelArgs::sk_tiles > 0). A separate instantiation, so that the
 // launches that split nothing -- most of them -- carry none of the exchange code: the call to it alone costs the
 // epilogue registers, and a spilled register here goes all the way to L2.
-template <typename OutT, int BN, bool kPair, bool kRows2, bool kCoop, bool kSplit>
+template <typename OutT, int BN, bool kPair, bool kRows2, int kStore, bool kSplit>
 __global__ void __launch_bounds__(kRows2 ? kNumThreadsRows2 : kNumThreads, 1)
 conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
                           const __grid_constant__ CUtensorMap tmap_w,
@@ -687,8 +767,10 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
     fence_mbar_init();
     prefetch_tmap(&tmap_x);
     prefetch_tmap(&tmap_w);
-    if (args.out_tma) prefetch_tmap(&tmap_out);
-    if (args.res_tma) prefetch_tmap(&tmap_res);
+    if constexpr (kStore == kStoreTma) {
+      prefetch_tmap(&tmap_out);
+      if (args.residual != nullptr) prefetch_tmap(&tmap_res);
+    }
   }
   if (warp == 1) {
     if constexpr (kPair) {
@@ -1015,7 +1097,6 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
     float* bias_w = reinterpret_cast<float*>(smem_gen + bias_off) + bias_slot;
     const uint32_t bias_w_s = smem_base + bias_off + static_cast<uint32_t>(bias_slot) * 4u;
     const uint32_t stg0 = staging_base + static_cast<uint32_t>(ew) * (kStagingDepth * kStagingBoxBytes);
-    const bool res_tma = args.res_tma != 0;
     // this lane's 16-byte chunk c of its staging row lives at row*128 + ((c ^ (row & 7)) << 4): the
     // SWIZZLE_128B pattern of the out / residual tensor maps (bank-conflict free for 8-lane phases)
     const uint32_t lane_row_off = static_cast<uint32_t>(lane) * 128u;
@@ -1087,13 +1168,11 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
     long long prof_wacc = 0, prof_wres = 0, prof_ld = 0, prof_math = 0, prof_stage = 0, prof_wstore = 0;
     (void)prof_wacc; (void)prof_wres; (void)prof_ld; (void)prof_math; (void)prof_stage; (void)prof_wstore;
     TB200_PROF_T(prof_t0);
-    const bool need_coords = !args.out_tma || (res != nullptr && !res_tma);
-    // kCoop kernels serve channel-contiguous outputs whose pixels are not one dense [M][pitch] matrix (a strided
-    // view, one phase of a transposed convolution; the host launches them only then, with out_tma = 0): same staging
-    // boxes as the TMA path, but the warp moves them itself, 8 lanes per pixel and 16 bytes each, so every store /
-    // residual load instruction covers 4 whole 128-byte rows. A separate instantiation, because inside the TMA
-    // kernels this code cost 1.3 % through register spills.
-    const bool res_staged = res_tma || (kCoop && res != nullptr);
+    constexpr bool need_coords = kStore != kStoreTma;
+    // kStoreRows: same staging boxes as the TMA path, but the warp moves them itself, so every store / residual load
+    // instruction covers whole rows.
+    const bool res_tma = kStore == kStoreTma && res != nullptr;   // the host has a TMA map of any residual then
+    const bool res_staged = kStore != kStoreStrided && res != nullptr;
     // ---- exchange of partial sums, ahead of the main loop. The pieces of split tiles are the first (at most two)
     // items of a worker. For each piece this warp owns rows of: wait for its accumulator, take a ticket, then either
     // write the partial sums out and release the accumulator (bit stays 0: the main loop skips the item), or -- last
@@ -1190,7 +1269,6 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
         out_off = img * args.out_sn + ho * args.out_sh + wo * args.out_sw;
         res_off = img * args.res_sn + ho * args.res_sh + wo * args.res_sw;
       }
-      const OutT* res_row = res + res_off + static_cast<long long>(n_base) * args.res_sc;
 
       // Residual box of the tile's first live group: requested before the accumulator is waited for.
       // Box `box` was last stored from two groups ago; only the newer store may still be pending.
@@ -1272,14 +1350,14 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               tma_load_2d(stg0 + nb * kStagingBoxBytes, &tmap_res, res_bar(ew, nb), n0 + g_step * kGroupCols, m_row0);
             }
           }
-        } else if (args.out_tma) {
+        } else if constexpr (kStore == kStoreTma) {
           TB200_PROF_T(ts);
           if (lane == 0) bulk_wait_group_read<1>();   // this box's previous store (two groups ago) has been read out
           __syncwarp();
           TB200_PROF_ADD(prof_wstore, ts);
         }
-        if constexpr (kCoop) {
-          if (res != nullptr) coop_load_box<OutT>(stg, res + n0, res_off, row_ok, args.K_out - n0, lane);
+        if constexpr (kStore == kStoreRows) {
+          if (res != nullptr) load_rows<OutT>(args.res_vec, stg, res + n0, res_off, row_ok, args.K_out - n0, lane);
         }
 
         TB200_PROF_T(tm);
@@ -1295,17 +1373,13 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
             add2(f[j4 * 4 + 0], f[j4 * 4 + 1], b4.x, b4.y);
             add2(f[j4 * 4 + 2], f[j4 * 4 + 3], b4.z, b4.w);
           }
-          if (!kCoop && !args.out_tma) {
-            float fg[32];   // a copy the out-of-line path may keep in local memory; f stays in registers
-#pragma unroll
-            for (int j = 0; j < 32; ++j) fg[j] = f[j];
-            epilogue_block_generic<OutT>(
-                args, fg, res != nullptr ? res_row + static_cast<long long>(g * kGroupCols + h * 32) * args.res_sc : nullptr,
-                out + out_off + static_cast<long long>(n0 + h * 32) * args.out_sc, n0 + h * 32, row_ok);
+          if constexpr (kStore == kStoreStrided) {
+            const int n_first = n0 + h * 32;
+            store_strided32<OutT>(args, f, res != nullptr ? res + res_off + n_first * args.res_sc : nullptr,
+                                  out + out_off + n_first * args.out_sc, args.K_out - n_first, row_ok, lane);
             continue;
           }
-          // TMA output; a residual, if any, sits in this lane's row of the staging box (the host
-          // guarantees a residual is TMA-loaded whenever the output is TMA-stored)
+          // a residual, if any, sits in this lane's row of the staging box
           uint4 rchunks[kChunksPerLd];
           if (res_staged) {
 #pragma unroll
@@ -1327,7 +1401,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
         }
         TB200_PROF_ADD(prof_math, tm);
         TB200_PROF_T(tg);
-        if (args.out_tma) {
+        if constexpr (kStore == kStoreTma) {
           // the lane's pixel row goes to its swizzled 128-byte row of the box; one TMA store writes the box
 #pragma unroll
           for (int c = 0; c < 8; ++c)
@@ -1339,17 +1413,17 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
             bulk_commit_group();
           }
           box ^= 1u;
-        } else if constexpr (kCoop) {
+        } else if constexpr (kStore == kStoreRows) {
 #pragma unroll
           for (int c = 0; c < 8; ++c)
             st_shared_v4(stg + lane_row_off + ((static_cast<uint32_t>(c) ^ lane_xor) << 4), packed[c]);
-          coop_store_box<OutT>(stg, out + n0, out_off, row_ok, args.K_out - n0, lane);
+          store_rows<OutT>(args.out_vec, stg, out + n0, out_off, row_ok, args.K_out - n0, lane);
           box ^= 1u;
         }
         TB200_PROF_ADD(prof_stage, tg);
       }
     }
-    if (args.out_tma && lane == 0) bulk_wait_group0();
+    if (kStore == kStoreTma && lane == 0) bulk_wait_group0();
     if (warp == 2 && lane == 0) {
       TB200_PROF_STORE(5, prof_wacc);
       TB200_PROF_STORE(6, prof_wres);

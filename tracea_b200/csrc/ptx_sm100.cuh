@@ -247,6 +247,24 @@ __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
+// One 4-byte or 2-byte word.
+template <typename Word>
+__device__ __forceinline__ Word ld_shared_word(uint32_t addr) {
+  if constexpr (sizeof(Word) == 4) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+  } else {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+    return v;
+  }
+}
+template <typename Word>
+__device__ __forceinline__ void st_shared_word(uint32_t addr, Word v) {
+  if constexpr (sizeof(Word) == 4) asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+  else asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
+}
 __device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));

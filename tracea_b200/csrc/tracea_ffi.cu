@@ -105,9 +105,9 @@ DeviceState g_dev[kMaxDevices];
 std::atomic<long long> g_test_wait_limit{0};
 std::atomic<int> g_test_producer_stop{-1};
 // "opt-in shared memory size has been set for this kernel variant on this device":
-// [device][dtype][bn index][tiling: single CTA / CTA pair / two row blocks; x3: plain, coop epilogue, K-split].
+// [device][dtype][bn index][tiling: single CTA / CTA pair / two row blocks; x4: the three store forms, K-split].
 // Setting the attribute twice is harmless, so a relaxed flag is enough.
-std::atomic<bool> g_attr_set[kMaxDevices][3][3][9];
+std::atomic<bool> g_attr_set[kMaxDevices][3][3][12];
 std::atomic<unsigned long long> g_kernel_launches{0};   // every kernel this library has launched (conv + layout adapters)
 // the same, by kind: 0 general implicit-GEMM kernel, 1 its K-split instantiations, 2 resident-filter kernel, 3 layout adapters
 std::atomic<unsigned long long> g_launches_by_kind[5];
@@ -397,12 +397,12 @@ int pick_stages(int bn, bool pair, bool rows2, bool shared_bias) {
   return std::min(s, tb200::kMaxStages);
 }
 
-template <typename OutT, int BN, bool kPair, bool kRows2, bool kCoop, bool kSplit>
+template <typename OutT, int BN, bool kPair, bool kRows2, int kStore, bool kSplit>
 void launch_one_variant(DeviceState& st, int dt_idx, int bn_idx, const CUtensorMap& tx, const CUtensorMap& tw,
                 const CUtensorMap& to, const CUtensorMap& tr, const ConvKernelArgs& args, int grid, int smem,
                 cudaStream_t stream) {
-  auto kern = tb200::conv2d_igemm_sm100_kernel<OutT, BN, kPair, kRows2, kCoop, kSplit>;
-  constexpr int kVariant = (kPair ? 1 : (kRows2 ? 2 : 0)) + (kCoop ? 3 : (kSplit ? 6 : 0));
+  auto kern = tb200::conv2d_igemm_sm100_kernel<OutT, BN, kPair, kRows2, kStore, kSplit>;
+  constexpr int kVariant = (kPair ? 1 : (kRows2 ? 2 : 0)) + 3 * (kSplit ? 3 : kStore);
   std::atomic<bool>& attr_done = g_attr_set[st.dev][dt_idx][bn_idx][kVariant];
   if (!attr_done.load(std::memory_order_relaxed)) {
     TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
@@ -438,48 +438,56 @@ void launch_one_variant(DeviceState& st, int dt_idx, int bn_idx, const CUtensorM
   g_launches_by_kind[kSplit ? 1 : 0].fetch_add(1, std::memory_order_relaxed);
 }
 
-// The K-split kernels exist for the TMA-store / per-lane epilogues only (the host never splits a coop launch).
-template <typename OutT, int BN, bool kPair, bool kRows2, bool kCoop>
+// The K-split kernels exist for the TMA epilogue only (the host splits no other launch).
+template <typename OutT, int BN, bool kPair, bool kRows2, int kStore>
 void launch_one(DeviceState& st, int dt_idx, int bn_idx, const CUtensorMap& tx, const CUtensorMap& tw,
                 const CUtensorMap& to, const CUtensorMap& tr, const ConvKernelArgs& args, int grid, int smem,
                 cudaStream_t stream) {
-  if constexpr (!kCoop) {
+  if constexpr (kStore == tb200::kStoreTma) {
     if (args.sk_tiles > 0) {
-      launch_one_variant<OutT, BN, kPair, kRows2, false, true>(st, dt_idx, bn_idx, tx, tw, to, tr, args, grid, smem, stream);
+      launch_one_variant<OutT, BN, kPair, kRows2, kStore, true>(st, dt_idx, bn_idx, tx, tw, to, tr, args, grid, smem, stream);
       return;
     }
   }
-  launch_one_variant<OutT, BN, kPair, kRows2, kCoop, false>(st, dt_idx, bn_idx, tx, tw, to, tr, args, grid, smem, stream);
+  launch_one_variant<OutT, BN, kPair, kRows2, kStore, false>(st, dt_idx, bn_idx, tx, tw, to, tr, args, grid, smem, stream);
 }
 
-// `coop`: the kernel variant whose epilogue moves its staging boxes to a strided, channel-contiguous output itself.
-template <typename OutT, bool kCoop>
+template <typename OutT, int kStore>
 void launch_tiling(DeviceState& st, int dt_idx, int bn, bool pair, bool rows2, const CUtensorMap& tx,
                    const CUtensorMap& tw, const CUtensorMap& to, const CUtensorMap& tr, const ConvKernelArgs& args,
                    int grid, int smem, cudaStream_t stream) {
   if (rows2) {
-    if (bn == 64) launch_one<OutT, 64, false, true, kCoop>(st, dt_idx, 0, tx, tw, to, tr, args, grid, smem, stream);
-    else launch_one<OutT, 128, false, true, kCoop>(st, dt_idx, 1, tx, tw, to, tr, args, grid, smem, stream);
+    if (bn == 64) launch_one<OutT, 64, false, true, kStore>(st, dt_idx, 0, tx, tw, to, tr, args, grid, smem, stream);
+    else launch_one<OutT, 128, false, true, kStore>(st, dt_idx, 1, tx, tw, to, tr, args, grid, smem, stream);
     return;
   }
   if (pair) {
-    if (bn == 128) launch_one<OutT, 128, true, false, kCoop>(st, dt_idx, 1, tx, tw, to, tr, args, grid, smem, stream);
-    else launch_one<OutT, 256, true, false, kCoop>(st, dt_idx, 2, tx, tw, to, tr, args, grid, smem, stream);
+    if (bn == 128) launch_one<OutT, 128, true, false, kStore>(st, dt_idx, 1, tx, tw, to, tr, args, grid, smem, stream);
+    else launch_one<OutT, 256, true, false, kStore>(st, dt_idx, 2, tx, tw, to, tr, args, grid, smem, stream);
     return;
   }
   switch (bn) {
-    case 64: launch_one<OutT, 64, false, false, kCoop>(st, dt_idx, 0, tx, tw, to, tr, args, grid, smem, stream); break;
-    case 128: launch_one<OutT, 128, false, false, kCoop>(st, dt_idx, 1, tx, tw, to, tr, args, grid, smem, stream); break;
-    default: launch_one<OutT, 256, false, false, kCoop>(st, dt_idx, 2, tx, tw, to, tr, args, grid, smem, stream); break;
+    case 64: launch_one<OutT, 64, false, false, kStore>(st, dt_idx, 0, tx, tw, to, tr, args, grid, smem, stream); break;
+    case 128: launch_one<OutT, 128, false, false, kStore>(st, dt_idx, 1, tx, tw, to, tr, args, grid, smem, stream); break;
+    default: launch_one<OutT, 256, false, false, kStore>(st, dt_idx, 2, tx, tw, to, tr, args, grid, smem, stream); break;
   }
 }
 
 template <typename OutT>
-void launch_bn(DeviceState& st, int dt_idx, int bn, bool pair, bool rows2, bool coop, const CUtensorMap& tx,
+void launch_bn(DeviceState& st, int dt_idx, int bn, bool pair, bool rows2, int store, const CUtensorMap& tx,
                const CUtensorMap& tw, const CUtensorMap& to, const CUtensorMap& tr, const ConvKernelArgs& args, int grid,
                int smem, cudaStream_t stream) {
-  if (coop) launch_tiling<OutT, true>(st, dt_idx, bn, pair, rows2, tx, tw, to, tr, args, grid, smem, stream);
-  else launch_tiling<OutT, false>(st, dt_idx, bn, pair, rows2, tx, tw, to, tr, args, grid, smem, stream);
+  switch (store) {
+    case tb200::kStoreTma:
+      launch_tiling<OutT, tb200::kStoreTma>(st, dt_idx, bn, pair, rows2, tx, tw, to, tr, args, grid, smem, stream);
+      break;
+    case tb200::kStoreRows:
+      launch_tiling<OutT, tb200::kStoreRows>(st, dt_idx, bn, pair, rows2, tx, tw, to, tr, args, grid, smem, stream);
+      break;
+    default:
+      launch_tiling<OutT, tb200::kStoreStrided>(st, dt_idx, bn, pair, rows2, tx, tw, to, tr, args, grid, smem, stream);
+      break;
+  }
 }
 
 CUtensorMapDataType tmap_dtype(TraceaDType t) {
@@ -1243,52 +1251,60 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   a.out_sc = out.stride[1];
   a.out_sh = out.stride[2];
   a.out_sw = out.stride[3];
-  auto vec_legal = [&](const View4& v) {
-    return (v.stride[1] == 1) && aligned16(v.ptr) && (v.stride[0] * es) % 16 == 0 &&
-           (v.stride[2] * es) % 16 == 0 && (v.stride[3] * es) % 16 == 0 && (K % vec_elems) == 0;
+  // ---- how the epilogue reaches the output. Rows that are linear in m = (n*Ho + ho)*Wo + wo form a [M][pitch] matrix:
+  // the epilogue stages 32-pixel x 128-byte boxes in shared memory and the TMA unit moves them, if the rows are 16-byte
+  // aligned. Channel-contiguous tensors that are not (a strided view, one phase of a transposed convolution, an odd
+  // channel count) go through the same boxes, moved by the warp in the widest accesses that all rows allow. Everything
+  // else -- NCHW, or so few channels that a row is a fraction of a sector -- is stored pixel by pixel, each lane its own.
+  // (2048 x 2047 x 1024 product, bf16: two-byte rows 13.1 us, per-lane stores 68.4, 16-byte boxes on 2048 columns 11.3.
+  // Between 3 and 5 channels rows and per-lane stores cost the same.)
+  const View4* res_v = epi.residual ? residual : nullptr;
+  auto row_vec = [&](const View4& v) -> int {   // bytes per access of a channel-contiguous tensor's rows
+    auto ok = [&](long long bytes) {
+      return reinterpret_cast<uintptr_t>(v.ptr) % bytes == 0 && v.stride[0] * es % bytes == 0 &&
+             v.stride[2] * es % bytes == 0 && v.stride[3] * es % bytes == 0 && K * es % bytes == 0;
+    };
+    return ok(16) ? 16 : (ok(4) ? 4 : es);
   };
-  a.out_vec = vec_legal(out) ? 1 : 0;
-  // Output rows that are linear in m = (n*Ho + ho)*Wo + wo form a [M][pitch] matrix: the epilogue
-  // stages 32-pixel x 128-byte boxes in shared memory and the TMA unit writes them out.
-  const bool out_rows_linear = out.stride[2] == Wo * out.stride[3] && out.stride[0] == Ho * out.stride[2];
-  if (a.out_vec && out_rows_linear && knobs().no_tma_store == 0) {
+  auto rows_linear = [&](const View4& v) {
+    return v.stride[2] == Wo * v.stride[3] && v.stride[0] == Ho * v.stride[2];
+  };
+  auto encode_rows = [&](CUtensorMap* m, const View4& v, CUtensorMapL2promotion promo, const char* what) {
     const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
-    const cuuint64_t gstr[1] = {(cuuint64_t)(out.stride[3] * es)};
+    const cuuint64_t gstr[1] = {(cuuint64_t)(v.stride[3] * es)};
     const cuuint32_t box[2] = {(cuuint32_t)(128 / es), 32u};
     const cuuint32_t estr[2] = {1u, 1u};
-    CUresult r = g_encode_tiled(&tmap_out, tmap_dtype(x.dtype), 2, out.ptr, gdim, gstr, box, estr,
-                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled (out) failed with %d", (int)r);
-    a.out_tma = 1;
+    CUresult r = g_encode_tiled(m, tmap_dtype(x.dtype), 2, v.ptr, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                CU_TENSOR_MAP_SWIZZLE_128B, promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled (%s) failed with %d", what, (int)r);
+  };
+  int store = tb200::kStoreStrided;
+  if (out.stride[1] == 1 && (res_v == nullptr || res_v->stride[1] == 1)) {
+    a.out_vec = row_vec(out);
+    a.res_vec = res_v != nullptr ? row_vec(*res_v) : 0;
+    if (a.out_vec == 16 && rows_linear(out) && knobs().no_tma_store == 0 &&
+        (res_v == nullptr || (a.res_vec == 16 && rows_linear(*res_v) && knobs().no_tma_residual == 0)))
+      store = tb200::kStoreTma;
+    else if (K > 4 || a.out_vec == 16)
+      store = tb200::kStoreRows;
   }
+  if (store == tb200::kStoreTma) {
+    encode_rows(&tmap_out, out, CU_TENSOR_MAP_L2_PROMOTION_NONE, "out");
+    if (res_v != nullptr) encode_rows(&tmap_res, *res_v, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, "residual");
+  }
+  a.out_quad = store == tb200::kStoreStrided && es == 2 && out.stride[3] == 1 && out.stride[2] == Wo &&
+               (Ho * Wo) % 4 == 0 && out.stride[0] % 4 == 0 && out.stride[1] % 4 == 0 &&
+               reinterpret_cast<uintptr_t>(out.ptr) % 8 == 0;
   if (epi.bias && bias != nullptr) {
     a.bias = bias->ptr;
     a.bias_is_f32 = bias->dtype == TRACEA_DTYPE_FLOAT32 ? 1 : 0;
   }
-  if (epi.residual && residual != nullptr) {
-    a.residual = residual->ptr;
-    a.res_sn = residual->stride[0];
-    a.res_sc = residual->stride[1];
-    a.res_sh = residual->stride[2];
-    a.res_sw = residual->stride[3];
-    a.res_vec = vec_legal(*residual) ? 1 : 0;
-    // a residual with the same dense row-linear form is TMA-loaded into the epilogue's staging boxes
-    const bool res_rows_linear = residual->stride[2] == Wo * residual->stride[3] &&
-                                 residual->stride[0] == Ho * residual->stride[2];
-    if (a.out_tma && a.res_vec && res_rows_linear && knobs().no_tma_residual == 0) {
-      const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
-      const cuuint64_t gstr[1] = {(cuuint64_t)(residual->stride[3] * es)};
-      const cuuint32_t box[2] = {(cuuint32_t)(128 / es), 32u};
-      const cuuint32_t estr[2] = {1u, 1u};
-      CUresult r = g_encode_tiled(&tmap_res, tmap_dtype(x.dtype), 2, residual->ptr, gdim, gstr, box, estr,
-                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled (residual) failed with %d", (int)r);
-      a.res_tma = 1;
-    } else {
-      a.out_tma = 0;   // the kernel's TMA epilogue takes its residual through TMA or not at all
-    }
+  if (res_v != nullptr) {
+    a.residual = res_v->ptr;
+    a.res_sn = res_v->stride[0];
+    a.res_sc = res_v->stride[1];
+    a.res_sh = res_v->stride[2];
+    a.res_sw = res_v->stride[3];
   }
   a.act = epi.act;
   a.status = st.status;
@@ -1303,9 +1319,6 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     if (*p.chain == 0) { a.pdl_mode = 1; *p.chain = 1; }
     else a.pdl_mode = staged ? 0 : 2;
   }
-  // channel-contiguous output (and residual, if any) that the TMA unit cannot address as one matrix: the kernel
-  // variant whose epilogue writes its staging boxes out itself, whole 128-byte rows at a time
-  const bool coop = !a.out_tma && a.out_vec && (a.residual == nullptr || a.res_vec);
 #ifdef TB200_PROFILE
   {  // bring-up builds only: TRACEA_B200_PROF_PTR carries a device pointer to 8 counters per CTA
     const char* pp = getenv("TRACEA_B200_PROF_PTR");
@@ -1382,7 +1395,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     Scratch sk_scratch;
     const long long k_iters = total_chunks_ll;   // 128-byte chunks: one per pipeline stage
     const int split_env = knobs().split_k;
-    if (chunk_bytes == 128 && !a_tiled && !coop && split_env != 0 && arena == nullptr && k_iters >= 2 &&
+    if (chunk_bytes == 128 && !a_tiled && store == tb200::kStoreTma && split_env != 0 && arena == nullptr && k_iters >= 2 &&
         2 * workers_max * k_iters < (1LL << 30)) {
       const long long rem = tiles % workers_max;       // tiles of the last, partly filled wave (all of them if < 1 wave)
       if (rem > 0) {
@@ -1438,13 +1451,13 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     const int grid = static_cast<int>(pair_v ? 2 * workers : workers);
     switch (x.dtype) {
       case TRACEA_DTYPE_BFLOAT16:
-        launch_bn<__nv_bfloat16>(st, 0, bn, pair_v, rows2_v, coop, tmap_x, tmap_w, tmap_out, tmap_res, la, grid, smem, stream);
+        launch_bn<__nv_bfloat16>(st, 0, bn, pair_v, rows2_v, store, tmap_x, tmap_w, tmap_out, tmap_res, la, grid, smem, stream);
         break;
       case TRACEA_DTYPE_FLOAT16:
-        launch_bn<__half>(st, 1, bn, pair_v, rows2_v, coop, tmap_x, tmap_w, tmap_out, tmap_res, la, grid, smem, stream);
+        launch_bn<__half>(st, 1, bn, pair_v, rows2_v, store, tmap_x, tmap_w, tmap_out, tmap_res, la, grid, smem, stream);
         break;
       default:
-        launch_bn<float>(st, 2, bn, pair_v, rows2_v, coop, tmap_x, tmap_w, tmap_out, tmap_res, la, grid, smem, stream);
+        launch_bn<float>(st, 2, bn, pair_v, rows2_v, store, tmap_x, tmap_w, tmap_out, tmap_res, la, grid, smem, stream);
         break;
     }
   };
