@@ -106,3 +106,38 @@ def test_layer_bench_example_parses_its_arguments():
     for bad in (["gemm", "1", "2"], ["preset", "nope"], ["conv", "1", "2", "3"]):
         with pytest.raises(SystemExit):
             lb.parse(bad)
+
+
+# --------------------------------------------------------------------------- tensor front end (argument errors need no GPU)
+def test_tensor_front_end_rejects_what_it_cannot_describe():
+    import pytest
+    import torch
+    from tracea_b200 import ffi, ops
+    x, w = torch.zeros(1, 4, 4, 8), torch.zeros(8, 3, 3, 8)
+    with pytest.raises(TypeError):                                   # no such dtype in the ABI
+        ops.conv2d(x.double(), w.double())
+    with pytest.raises(TypeError):
+        ops.gemm(x[0, 0].double(), x[0, 0].t())
+    with pytest.raises(TypeError):                                   # not a tensor
+        ops.conv2d(x, w, bias=[0.0] * 8, epilogue="bias")
+    with pytest.raises(ValueError):                                  # a residual needs the output's four dimensions
+        ops.conv2d(x, w, residual=torch.zeros(8), epilogue="residual")
+    with pytest.raises(RuntimeError):                                # the filter does not fit: a negative output extent
+        ops.conv2d(x[:, :1], torch.zeros(8, 5, 5, 8))
+    with pytest.raises(ffi.TraceaError) as e:                        # errors of the library carry its status and text
+        ops.conv2d_into(torch.zeros(2, 2), w, x)
+    assert e.value.status == ffi.INVALID_PARAMS and "Expected 4D tensors" in e.value.message
+
+
+def test_every_spelling_of_an_epilogue_is_parsed_once_and_checked_every_time():
+    import pytest
+    from tracea_b200 import ffi, ops
+    b = object()
+    for _ in range(2):                                               # the second time from the cache
+        assert ops.parse_epilogue("Bias + ReLU", b) == ffi.EPILOGUE_BIAS_RELU
+        with pytest.raises(ValueError):
+            ops.parse_epilogue("Bias + ReLU", None)
+        with pytest.raises(ValueError):
+            ops.parse_epilogue("relu+bias", b)
+        with pytest.raises(ValueError):
+            ops.parse_epilogue("bias+tanh", b)

@@ -9,9 +9,12 @@ Mirrors (paths relative to the reference project's root):
   * the NCHW / OIHW call the C++ header documents (include/tracea.hpp:101-105) as ``conv2d_nchw``.
 
 torch is used for device memory and streams only. Every call goes through ``tracea_conv2d`` in
-libtracea_b200.so; nothing here computes a convolution itself.
+libtracea_b200.so; nothing here computes a convolution itself. The calls below hand their tensors to the library through
+the ``_ops_native`` module, which builds the C tensor views (csrc/py_ops.cpp); ``ffi`` is the same ABI through ctypes, for
+callers that hold raw pointers.
 """
 import ctypes
+import functools
 
 import torch
 
@@ -22,15 +25,22 @@ _DTYPES = {torch.float32: ffi.DTYPE_FLOAT32, torch.float16: ffi.DTYPE_FLOAT16,
 
 _ACTS = ("relu", "gelu", "silu")
 
+_native_module = None
 
-def parse_epilogue(epilogue, bias=None, residual=None):
-    """Epilogue string -> TraceaEpilogueKind, with the grammar and the errors of
-    src/interface/python.rs:41-87: '+'-separated, case-insensitive ops out of identity, relu, gelu,
-    silu, bias, residual; 'bias' / 'residual' without the matching tensor is a ValueError, so is an
-    unknown op. The kernel applies bias -> residual -> activation, the order the reference's graph
-    fusion produces (tests/fusion_verification.rs:110-170); other orders are rejected."""
-    if epilogue is None:
-        return ffi.EPILOGUE_IDENTITY
+
+def _native():
+    """The tensor front end of the library, loaded with it on first use (raises if either has not been built)."""
+    global _native_module
+    if _native_module is None:
+        ffi.load()
+        from . import _ops_native
+        _native_module = _ops_native
+    return _native_module
+
+
+@functools.lru_cache(maxsize=256)
+def _epilogue_ops(epilogue):
+    """The ops of an epilogue string, as a tuple; ValueError on an unknown one."""
     ops = []
     for part in epilogue.split("+"):
         op = part.strip().lower()
@@ -40,27 +50,41 @@ def parse_epilogue(epilogue, bias=None, residual=None):
             ops.append(op)
         else:
             raise ValueError("Unknown epilogue op: %s" % part)
+    return tuple(ops)
+
+
+_EPILOGUE_KINDS = {
+    (): ffi.EPILOGUE_IDENTITY,
+    ("bias",): ffi.EPILOGUE_BIAS_ADD,
+    ("relu",): ffi.EPILOGUE_RELU,
+    ("gelu",): ffi.EPILOGUE_GELU,
+    ("silu",): ffi.EPILOGUE_SILU,
+    ("bias", "relu"): ffi.EPILOGUE_BIAS_RELU,
+    ("bias", "silu"): ffi.EPILOGUE_BIAS_SILU,
+    ("residual",): ffi.EPILOGUE_RESIDUAL,
+    ("residual", "relu"): ffi.EPILOGUE_RESIDUAL_RELU,
+    ("bias", "residual", "relu"): ffi.EPILOGUE_BIAS_RESIDUAL_RELU,
+    ("bias", "residual"): ffi.EPILOGUE_BIAS_RESIDUAL,
+}
+
+
+def parse_epilogue(epilogue, bias=None, residual=None):
+    """Epilogue string -> TraceaEpilogueKind, with the grammar and the errors of
+    src/interface/python.rs:41-87: '+'-separated, case-insensitive ops out of identity, relu, gelu,
+    silu, bias, residual; 'bias' / 'residual' without the matching tensor is a ValueError, so is an
+    unknown op. The kernel applies bias -> residual -> activation, the order the reference's graph
+    fusion produces (tests/fusion_verification.rs:110-170); other orders are rejected."""
+    if epilogue is None:
+        return ffi.EPILOGUE_IDENTITY
+    ops = _epilogue_ops(epilogue)
     if "bias" in ops and bias is None:
         raise ValueError("Epilogue contains 'bias' but no bias argument provided")
     if "residual" in ops and residual is None:
         raise ValueError("Epilogue contains 'residual' but no reference provided")
-    table = {
-        (): ffi.EPILOGUE_IDENTITY,
-        ("bias",): ffi.EPILOGUE_BIAS_ADD,
-        ("relu",): ffi.EPILOGUE_RELU,
-        ("gelu",): ffi.EPILOGUE_GELU,
-        ("silu",): ffi.EPILOGUE_SILU,
-        ("bias", "relu"): ffi.EPILOGUE_BIAS_RELU,
-        ("bias", "silu"): ffi.EPILOGUE_BIAS_SILU,
-        ("residual",): ffi.EPILOGUE_RESIDUAL,
-        ("residual", "relu"): ffi.EPILOGUE_RESIDUAL_RELU,
-        ("bias", "residual", "relu"): ffi.EPILOGUE_BIAS_RESIDUAL_RELU,
-        ("bias", "residual"): ffi.EPILOGUE_BIAS_RESIDUAL,
-    }
-    kind = table.get(tuple(ops))
+    kind = _EPILOGUE_KINDS.get(ops)
     if kind is None:
         raise ValueError("Unsupported epilogue sequence %r (supported: %s)" % (
-            epilogue, ", ".join("+".join(k) or "identity" for k in table)))
+            epilogue, ", ".join("+".join(k) or "identity" for k in _EPILOGUE_KINDS)))
     return kind
 
 
@@ -82,13 +106,6 @@ def _view(t, shape=None, stride=None):
                     t.device.index if t.is_cuda else -1)
 
 
-def _nchw_view_of_nhwc(t):
-    """Logical NCHW view (shape + element strides) of a tensor whose dims are (N, H, W, C)."""
-    n, h, w, c = t.shape
-    sn, sh, sw, sc = t.stride()
-    return _view(t, (n, c, h, w), (sn, sc, sh, sw))
-
-
 def _stream_of(t):
     return torch.cuda.current_stream(t.device).cuda_stream if t.is_cuda else 0
 
@@ -98,7 +115,10 @@ def conv2d_into(x, w, out, bias=None, residual=None, stride=1, padding=0, dilati
     """out <- epilogue(conv2d(x, w)) with logical NCHW / OIHW tensors of any strides (a
     ``channels_last`` torch tensor is consumed in place). Enqueues on torch's current stream."""
     if stream is None:
-        stream = _stream_of(x)
+        sh, sw = _pair(stride)
+        ph, pw = _pair(padding)
+        dh, dw = _pair(dilation)
+        return _native().conv2d(x, w, bias, residual, out, False, int(epilogue), sh, sw, ph, pw, dh, dw, groups)
     ffi.conv2d_raw(_view(x), _view(w), _view(bias) if bias is not None else None,
                    _view(residual) if residual is not None else None, _view(out),
                    _pair(stride), _pair(padding), _pair(dilation), groups, epilogue, stream)
@@ -121,7 +141,7 @@ def conv2d_nchw(x, w, bias=None, residual=None, stride=1, padding=0, dilation=1,
         channels_last_out = x.stride(1) == 1 and x.shape[1] > 1
     fmt = torch.channels_last if channels_last_out else torch.contiguous_format
     out = torch.empty((n, k, ho, wo), dtype=x.dtype, device=x.device, memory_format=fmt)
-    return conv2d_into(x, w, out, bias, residual, stride, padding, dilation, groups, kind)
+    return _native().conv2d(x, w, bias, residual, out, False, kind, sh, sw, ph, pw, dh, dw, groups)
 
 
 def conv2d(x, w, bias=None, residual=None, epilogue=None, stride=1, padding=0, dilation=1):
@@ -140,9 +160,8 @@ def conv2d(x, w, bias=None, residual=None, epilogue=None, stride=1, padding=0, d
     h_out = (h + 2 * ph - dh * (r - 1) - 1) // sh + 1
     w_out = (w_in + 2 * pw - dw * (s - 1) - 1) // sw + 1
     o = torch.empty((n_batch, h_out, w_out, k), dtype=x.dtype, device=x.device)
-    Context().conv2d(x, w, o, n_batch, c, h, w_in, k, r, s, stride=stride, pad=padding, dilation=dilation,
-                     epilogue=epilogue, bias=bias, residual=residual)
-    return o
+    kind = parse_epilogue(epilogue, bias, residual)
+    return _native().conv2d(x, w, bias, residual, o, True, kind, sh, sw, ph, pw, dh, dw, 1)
 
 
 def gemm(x, w, bias=None, epilogue=None, residual=None):
@@ -155,9 +174,7 @@ def gemm(x, w, bias=None, epilogue=None, residual=None):
         raise ValueError(f"Inner dimension mismatch: x({x.shape[1]}) vs w({w.shape[0]})")
     kind = parse_epilogue(epilogue, bias, residual)
     out = torch.empty((x.shape[0], w.shape[1]), dtype=x.dtype, device=x.device)
-    ffi.gemm_raw(_view(x), _view(w), _view(bias) if bias is not None else None,
-                 _view(residual) if residual is not None else None, _view(out), kind, _stream_of(x))
-    return out
+    return _native().gemm(x, w, bias, residual, out, kind)
 
 
 def conv_transpose2d(x, w, bias=None, residual=None, epilogue=None, stride=1, padding=0, output_padding=0,
@@ -178,10 +195,8 @@ def conv_transpose2d(x, w, bias=None, residual=None, epilogue=None, stride=1, pa
     w_out = (w_in - 1) * sw - 2 * pw + s + ow
     kind = parse_epilogue(epilogue, bias, residual)
     o = torch.empty((n_batch, h_out, w_out, k), dtype=x.dtype, device=x.device)
-    ffi.conv_transpose2d_raw(_view(x), _view(w), _view(bias) if bias is not None else None,
-                             _view(residual) if residual is not None else None, _view(o), (sh, sw), (ph, pw),
-                             (oh, ow), _pair(dilation), 1, kind, _stream_of(x))
-    return o
+    dh, dw = _pair(dilation)
+    return _native().conv_transpose2d(x, w, bias, residual, o, kind, sh, sw, ph, pw, oh, ow, dh, dw)
 
 
 def prepack_conv2d_weight(w):
@@ -222,11 +237,10 @@ class Context:
         kind = parse_epilogue(epilogue, bias, residual)
         if tuple(x.shape) != (n, h, w_in, c) or tuple(w.shape) != (k, r, s, c):
             raise ValueError("x must be (n, h, w_in, c) and w must be (k, r, s, c)")
-        wk, wr, ws_, wc = w.stride()
-        res_view = _nchw_view_of_nhwc(residual) if residual is not None else None
-        ffi.conv2d_raw(_nchw_view_of_nhwc(x), _view(w, (k, c, r, s), (wk, wc, wr, ws_)),
-                       _view(bias) if bias is not None else None, res_view, _nchw_view_of_nhwc(o),
-                       _pair(stride), _pair(pad), _pair(dilation), 1, kind, _stream_of(x))
+        sh, sw = _pair(stride)
+        ph, pw = _pair(pad)
+        dh, dw = _pair(dilation)
+        _native().conv2d(x, w, bias, residual, o, True, kind, sh, sw, ph, pw, dh, dw, 1)
         return 0
 
     def synchronize(self):
