@@ -581,6 +581,47 @@ def test_unaligned_output_and_residual_views(offset, K, pitch, dtype):
     assert (big[:, :offset] == 7.0).all() and (big[:, offset + K:] == 7.0).all()
 
 
+# --------------------------------------------------------------------------- layout adapters
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("shape", [(2, 64, 8, 8), (1, 70, 9, 15), (3, 33, 6, 7), (2, 8, 5, 13), (4, 130, 1, 9), (5, 40, 3, 3),
+                                   (1, 257, 16, 16), (2, 64, 13, 1), (70, 24, 1, 1), (2, 1, 12, 12)])
+@pytest.mark.parametrize("form", ["nchw", "nhwc", "nhwc_odd", "window", "hwcn"])
+def test_operands_of_any_memory_format_are_copied_exactly(shape, form, dtype):
+    """A 1x1 convolution with an identity filter returns its input bit for bit, whatever memory the input and the filter come
+    in: pixels contiguous (tiles, and whole groups of channels for small images), channels contiguous at any alignment, a
+    window of a larger image, a permuted one."""
+    N, C, H, W = shape
+    t = TORCH_DT[dtype]
+    x = torch.randint(-100, 100, shape, device="cuda").to(t)
+    if form == "nchw":
+        xv = x
+    elif form == "nhwc":
+        xv = x.contiguous(memory_format=torch.channels_last)
+    elif form == "nhwc_odd":            # rows one element apart from any alignment
+        xv = torch.zeros((N, H, W, C + 3), dtype=t, device="cuda").permute(0, 3, 1, 2)[:, 1:C + 1]
+        xv.copy_(x)
+    elif form == "window":
+        xv = torch.zeros((N, C, H + 3, W + 2), dtype=t, device="cuda")[:, :, 2:H + 2, 1:W + 1]
+        xv.copy_(x)
+    else:
+        xv = torch.empty((H, W, C, N), dtype=t, device="cuda").permute(3, 2, 0, 1)
+        xv.copy_(x)
+    eye = torch.eye(C, device="cuda").to(t)
+    for w in (eye.view(C, C, 1, 1), eye.t().contiguous().t().view(C, C, 1, 1)):
+        out = ops.conv2d_nchw(xv, w, channels_last_out=True)
+        assert torch.equal(out, x)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("K,C,R,S", [(5, 40, 3, 3), (64, 70, 2, 2), (33, 130, 5, 5), (3, 64, 6, 6), (9, 64, 1, 3), (130, 16, 3, 1)])
+def test_filters_are_repacked_exactly(K, C, R, S, dtype):
+    """Prepacking writes [K][R][S][C] memory (channels padded to 16 bytes) from OIHW, KRSC and permuted filters alike."""
+    w = torch.randn((K, C, R, S), device="cuda").to(TORCH_DT[dtype])
+    for v in (w, w.contiguous(memory_format=torch.channels_last), w.permute(2, 3, 0, 1).contiguous().permute(2, 3, 0, 1)):
+        packed = ops.prepack_conv2d_weight(v)
+        assert torch.equal(packed[:, :C], w) and bool((packed[:, C:] == 0).all())
+
+
 # --------------------------------------------------------------------------- tiles split over K (opt-in schedule)
 _SPLIT_K_SCRIPT = r"""
 import sys

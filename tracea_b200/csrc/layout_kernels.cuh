@@ -1,46 +1,183 @@
 // Layout adapters for callers that hand over NCHW-contiguous activations or OIHW-contiguous
 // weights (the layouts include/tracea.hpp:101-105 documents). The conv kernel itself reads
 // channels-last memory, which is what the reference's kernel reads too (NHWC input, conv.rs:202-247).
-// Both adapters read through arbitrary element strides and write dense, channel-padded buffers.
+// The adapters read through arbitrary element strides and write dense, channel-padded buffers.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace tb200 {
 
-// x[n, c, h, w] (element strides sn, sc, sh, sw) -> dst[n][h*W + w][Cp] with channels c >= C
-// zero-filled. One CTA moves a 32 (channels) x 32 (pixels) tile through shared memory so that
-// both sides are coalesced when the source is NCHW-contiguous.
+// One copy src[n][c][p] (element strides) -> dst[n][p][Cp], channels C .. Cp-1 zero-filled: an activation tensor (p: its
+// pixels), a filter bank (n: output channels, p: taps) or a matrix. Cp * sizeof(T) is a multiple of 16 bytes and dst is
+// 16-byte aligned, except in kCopyElements.
+enum : int {
+  kCopyPlanes = 0,     // pixels contiguous (NCHW): 128-byte x 64-pixel tiles transposed through shared memory
+  kCopyTaps = 1,       // pixels contiguous, few of them, and channels right behind one another (OIHW filters): a group of
+                       // channels is one contiguous run
+  kCopyRows = 2,       // channels contiguous but rows unaligned or short: rows copied with their padding
+  kCopyElements = 3,   // anything else: 32 x 32 tiles, element by element
+};
+struct CopyJob {
+  const void* src;
+  void* dst;
+  int mode;
+  int vec;             // elements per source access (kCopyPlanes: along pixels, kCopyRows: along channels)
+  int C, Cp, P, W;     // W: pixels per row of the source (pixel p is at (p / W) * sh + (p % W) * sw)
+  long long N;
+  long long sn, sc, sh, sw;
+  long long blocks;
+};
+struct CopyJobs {
+  CopyJob job[2];
+};
+constexpr int kCopyThreads = 256;
+constexpr int kCopyMaxTaps = 32;                       // kCopyTaps: pixels per image
+template <typename T> constexpr int kCopyTileC = 128 / sizeof(T);   // channels per tile: 128 bytes
+constexpr int kCopyTileP = 64;
+template <typename T> constexpr int kCopyPitch = kCopyTileC<T> + 4 / static_cast<int>(sizeof(T));   // 33 words: an odd number
+
+template <typename T, int kVec> struct CopyVec;
+template <> struct CopyVec<uint16_t, 8> { using type = uint4; };
+template <> struct CopyVec<uint16_t, 4> { using type = uint2; };
+template <> struct CopyVec<uint16_t, 2> { using type = uint32_t; };
+template <> struct CopyVec<uint16_t, 1> { using type = uint16_t; };
+template <> struct CopyVec<uint32_t, 4> { using type = uint4; };
+template <> struct CopyVec<uint32_t, 2> { using type = uint2; };
+template <> struct CopyVec<uint32_t, 1> { using type = uint32_t; };
+
+// Planes: every thread's source accesses are issued before the first is used, consecutive lanes read consecutive pixels.
+template <typename T, int kVec>
+__device__ __forceinline__ void copy_tile_in(const CopyJob& j, T* tile, const T* src, int c0, int p0) {
+  using V = typename CopyVec<T, kVec>::type;
+  constexpr int kPerRow = kCopyTileP / kVec;
+  constexpr int kIters = kCopyTileC<T> * kPerRow / kCopyThreads;
+  V v[kIters];
+#pragma unroll
+  for (int i = 0; i < kIters; ++i) {
+    const int t = i * kCopyThreads + static_cast<int>(threadIdx.x);
+    const int c = c0 + t / kPerRow, p = p0 + t % kPerRow * kVec;
+    v[i] = V{};
+    if (c < j.C && p < j.P) v[i] = *reinterpret_cast<const V*>(src + c * j.sc + p);   // P is a multiple of kVec
+  }
+#pragma unroll
+  for (int i = 0; i < kIters; ++i) {
+    const int t = i * kCopyThreads + static_cast<int>(threadIdx.x);
+    const int c = t / kPerRow, p = t % kPerRow * kVec;
+    const T* e = reinterpret_cast<const T*>(&v[i]);
+#pragma unroll
+    for (int k = 0; k < kVec; ++k) tile[(p + k) * kCopyPitch<T> + c] = e[k];
+  }
+}
+// 16 bytes of one tile row (4-byte aligned).
 template <typename T>
-__global__ void to_channels_last_kernel(const T* __restrict__ src, T* __restrict__ dst, int C, int H,
-                                        int W, int Cp, long long sn, long long sc, long long sh,
-                                        long long sw) {
-  __shared__ T tile[32][33];
-  const int HW = H * W;
-  const int n = blockIdx.z;
-  const int p0 = blockIdx.x * 32;
-  const int c0 = blockIdx.y * 32;
-  const int tx = threadIdx.x;  // 0..31
-  const int ty = threadIdx.y;  // 0..7
-  // read: consecutive tx -> consecutive pixels (contiguous for NCHW sources)
-  const int p = p0 + tx;
-  long long poff = 0;
-  if (p < HW) {
-    const int h = p / W;
-    poff = h * sh + (p - h * W) * sw;
-  }
-  for (int i = ty; i < 32; i += 8) {
-    const int c = c0 + i;
-    T v = T(0);
-    if (p < HW && c < C) v = src[n * sn + c * sc + poff];
-    tile[i][tx] = v;
-  }
-  __syncthreads();
-  // write: consecutive tx -> consecutive channels
-  const int c = c0 + tx;
-  for (int i = ty; i < 32; i += 8) {
-    const int pp = p0 + i;
-    if (pp < HW && c < Cp) dst[(static_cast<long long>(n) * HW + pp) * Cp + c] = tile[tx][i];
+__device__ __forceinline__ uint4 tile_chunk(const T* row, int chunk) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(row) + chunk * 4;
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Layout adapters of one call -- the activations, the filter bank, or both -- as one launch: a small call's time is the
+// number of dependent launches in front of its convolution, not their bytes.
+template <typename T>
+__global__ void __launch_bounds__(kCopyThreads) copy_channels_last_kernel(const __grid_constant__ CopyJobs jobs) {
+  // the convolution behind this launch may bring up its CTAs; the sources may come from, and the scratch may still be read
+  // by, the launch in front of it
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  __shared__ __align__(16) T tile[kCopyTileP * kCopyPitch<T>];
+  constexpr int kChunk = 16 / sizeof(T);               // elements per 16 bytes
+  long long b = blockIdx.x;
+  const bool second = b >= jobs.job[0].blocks;
+  if (second) b -= jobs.job[0].blocks;
+  const CopyJob& j = jobs.job[second ? 1 : 0];
+  const T* src = static_cast<const T*>(j.src);
+  T* dst = static_cast<T*>(j.dst);
+  const int tid = static_cast<int>(threadIdx.x);
+  if (j.mode == kCopyPlanes) {
+    const int tiles_p = (j.P + kCopyTileP - 1) / kCopyTileP, tiles_c = (j.Cp + kCopyTileC<T> - 1) / kCopyTileC<T>;
+    const int tp = static_cast<int>(b % tiles_p);
+    const long long t = b / tiles_p;
+    const int c0 = static_cast<int>(t % tiles_c) * kCopyTileC<T>, p0 = tp * kCopyTileP;
+    const long long n = t / tiles_c;
+    const T* s = src + n * j.sn;
+    if (j.vec == 1) copy_tile_in<T, 1>(j, tile, s, c0, p0);
+    else if (j.vec == 2) copy_tile_in<T, 2>(j, tile, s, c0, p0);
+    else if (j.vec == 4) copy_tile_in<T, 4>(j, tile, s, c0, p0);
+    else if constexpr (sizeof(T) == 2) copy_tile_in<T, 8>(j, tile, s, c0, p0);
+    __syncthreads();
+    for (int i = tid; i < kCopyTileP * 8; i += kCopyThreads) {   // 8 lanes write one pixel's 128 bytes
+      const int p = i >> 3, c = c0 + (i & 7) * kChunk;
+      if (p0 + p < j.P && c < j.Cp)
+        *reinterpret_cast<uint4*>(dst + (n * j.P + p0 + p) * j.Cp + c) = tile_chunk(tile + p * kCopyPitch<T>, i & 7);
+    }
+  } else if (j.mode == kCopyTaps) {
+    // one block: one group of 128 bytes of channels of as many images (output channels) as fill the tile
+    const int tiles_c = (j.Cp + kCopyTileC<T> - 1) / kCopyTileC<T>;
+    const int c0 = static_cast<int>(b % tiles_c) * kCopyTileC<T>;
+    const int per = kCopyTileP / j.P;
+    const long long n0 = b / tiles_c * per;
+    const int run = min(kCopyTileC<T>, j.C - c0) * j.P;            // contiguous source elements (<= 0: padding only)
+    const int full = kCopyTileC<T> * j.P;
+#pragma unroll 4
+    for (int i = tid; i < per * full; i += kCopyThreads) {
+      const int k = i / full, e = i - k * full;
+      const int c = e / j.P, p = e - c * j.P;
+      T v = T(0);
+      if (n0 + k < j.N && e < run) v = src[(n0 + k) * j.sn + static_cast<long long>(c0) * j.P + e];
+      tile[(k * j.P + p) * kCopyPitch<T> + c] = v;
+    }
+    __syncthreads();
+    for (int i = tid; i < per * j.P * 8; i += kCopyThreads) {
+      const int r = i >> 3, c = c0 + (i & 7) * kChunk;
+      if (n0 + r / j.P < j.N && c < j.Cp)
+        *reinterpret_cast<uint4*>(dst + (n0 * j.P + r) * j.Cp + c) = tile_chunk(tile + r * kCopyPitch<T>, i & 7);
+    }
+  } else if (j.mode == kCopyRows) {
+    const int per_row = j.Cp / kChunk;
+    const long long total = j.N * j.P * per_row;
+    const long long i = b * kCopyThreads + tid;
+    if (i >= total) return;
+    const long long row = i / per_row;
+    const int c = static_cast<int>(i - row * per_row) * kChunk;
+    const long long n = row / j.P;
+    const int p = static_cast<int>(row - n * j.P), h = p / j.W;
+    const T* s = src + n * j.sn + h * j.sh + (p - h * j.W) * j.sw + c;
+    uint4 out = make_uint4(0u, 0u, 0u, 0u);
+    T* e = reinterpret_cast<T*>(&out);
+    if (c + kChunk <= j.C) {
+      if (sizeof(T) == 2 && j.vec == 2) {
+        uint32_t* w = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[k] = reinterpret_cast<const uint32_t*>(s)[k];
+      } else {
+#pragma unroll
+        for (int k = 0; k < kChunk; ++k) e[k] = s[k];
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kChunk; ++k)
+        if (c + k < j.C) e[k] = s[k];
+    }
+    *reinterpret_cast<uint4*>(dst + i * kChunk) = out;
+  } else {
+    const int tiles_p = (j.P + 31) / 32, tiles_c = (j.Cp + 31) / 32;
+    const int p0 = static_cast<int>(b % tiles_p) * 32;
+    const long long t = b / tiles_p;
+    const int c0 = static_cast<int>(t % tiles_c) * 32;
+    const long long n = t / tiles_c;
+    const int tx = tid & 31, ty = tid >> 5;
+    const int p = p0 + tx;
+    const long long poff = p < j.P ? static_cast<long long>(p / j.W) * j.sh + (p % j.W) * j.sw : 0;
+    for (int i = ty; i < 32; i += kCopyThreads / 32) {
+      const int c = c0 + i;
+      T v = T(0);
+      if (p < j.P && c < j.C) v = src[n * j.sn + c * j.sc + poff];
+      tile[i * 33 + tx] = v;
+    }
+    __syncthreads();
+    const int c = c0 + tx;
+    for (int i = ty; i < 32; i += kCopyThreads / 32)
+      if (p0 + i < j.P && c < j.Cp) dst[(n * j.P + p0 + i) * j.Cp + c] = tile[tx * 33 + i];
   }
 }
 

@@ -575,27 +575,89 @@ NoAllocState& noalloc_state(int dev) {
   return na;
 }
 
-// ------------------------------------------------------------------ weight packing
-// w[k, c, r, s] through element strides -> dst[k][r][Sd][Cp] (channels >= C and tap slots >= S zero-filled).
+// ------------------------------------------------------------------ layout adapters
+// src[n, c, h, w] through element strides -> dst[n][h * W + w][Cp], channels C .. Cp-1 zero-filled. The mode is the widest
+// access both sides allow: see CopyJob.
+tb200::CopyJob copy_job(const void* src, void* dst, int es, long long N, long long C, long long Cp, long long H, long long W,
+                        long long sn, long long sc, long long sh, long long sw) {
+  if (H * W == 1) {   // a matrix: its rows are the pixels of one image
+    W = N; sw = sn; sh = 0; N = 1; sn = 0;
+  }
+  tb200::CopyJob j;
+  memset(&j, 0, sizeof(j));
+  j.src = src; j.dst = dst;
+  j.N = N; j.C = (int)C; j.Cp = (int)Cp; j.P = (int)(H * W); j.W = (int)W;
+  j.sn = sn; j.sc = sc; j.sh = sh; j.sw = sw;
+  j.vec = 1;
+  const long long P = H * W, chunk = 16 / es;
+  const uintptr_t addr = reinterpret_cast<uintptr_t>(src);
+  const bool planar = W == 1 ? (sh == 1 || H == 1) : (sw == 1 && (H == 1 || sh == W));
+  if (Cp % chunk != 0 || !aligned16(dst)) {
+    j.mode = tb200::kCopyElements;
+  } else if (sc == 1 || C == 1) {
+    j.mode = tb200::kCopyRows;
+    if (es == 2 && C > 1 && C % 2 == 0 && addr % 4 == 0 && sn % 2 == 0 && sh % 2 == 0 && sw % 2 == 0) j.vec = 2;
+  } else if (planar && P <= tb200::kCopyMaxTaps && sc == P && N > 1) {
+    j.mode = tb200::kCopyTaps;
+  } else if (planar) {
+    j.mode = tb200::kCopyPlanes;
+    for (int v = (int)chunk; v > 1; v >>= 1)
+      if (addr % (v * es) == 0 && P % v == 0 && sc % v == 0 && (N == 1 || sn % v == 0)) { j.vec = v; break; }
+  } else {
+    j.mode = tb200::kCopyElements;
+  }
+  auto ceil_div = [](long long x, long long y) { return (x + y - 1) / y; };
+  const long long tile_c = 128 / es;
+  switch (j.mode) {
+    case tb200::kCopyPlanes: j.blocks = N * ceil_div(Cp, tile_c) * ceil_div(P, tb200::kCopyTileP); break;
+    case tb200::kCopyTaps: j.blocks = ceil_div(N, tb200::kCopyTileP / P) * ceil_div(Cp, tile_c); break;
+    case tb200::kCopyRows: j.blocks = ceil_div(N * P * (Cp / chunk), tb200::kCopyThreads); break;
+    default: j.blocks = N * ceil_div(Cp, 32) * ceil_div(P, 32); break;
+  }
+  return j;
+}
+
+// Runs up to two copies as one launch. The launch lets the kernel behind it start early and waits for the one in front
+// before it reads or writes anything.
+void launch_copies(const tb200::CopyJob* jobs, int count, int es, cudaStream_t stream) {
+  if (count == 0) return;
+  tb200::CopyJobs pack;
+  memset(&pack, 0, sizeof(pack));
+  long long blocks = 0;
+  for (int i = 0; i < count; ++i) {
+    pack.job[i] = jobs[i];
+    blocks += jobs[i].blocks;
+  }
+  if (blocks > 0x7fffffffLL) TB_FAIL(TRACEA_UNSUPPORTED_CONFIG, "layout adapter: tensor too large");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+  cfg.blockDim = dim3(tb200::kCopyThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = knobs().pdl != 0 ? 1 : 0;
+  if (es == 2) TB_CUDA(cudaLaunchKernelEx(&cfg, tb200::copy_channels_last_kernel<uint16_t>, pack));
+  else TB_CUDA(cudaLaunchKernelEx(&cfg, tb200::copy_channels_last_kernel<uint32_t>, pack));
+  TB_CUDA(cudaGetLastError());
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  g_launches_by_kind[3].fetch_add(1, std::memory_order_relaxed);
+}
+
+// w[k, c, r, s] through element strides -> dst[k][r][S][Cp] (channels >= C zero-filled).
+tb200::CopyJob weight_job(const void* src, void* dst, int es, long long K, long long C, long long R, long long S,
+                          long long Cp, const long long stride[4]) {
+  return copy_job(src, dst, es, K, C, Cp, R, S, stride[0], stride[1], stride[2], stride[3]);
+}
+
+// The same with Sd >= S tap slots per filter row, slots >= S zero (the row-band and the widened-pixel forms).
 void launch_weight_pack(const void* src, void* dst, int es, long long K, long long C, long long R, long long S,
                         long long Sd, long long Cp, const long long stride[4], cudaStream_t stream) {
   const long long total = K * R * Sd * Cp;
   const int threads = 256;
   const unsigned blocks = static_cast<unsigned>((total + threads - 1) / threads);
-  if (R == 1 && Sd == 1 && (Cp + 31) / 32 <= 65535) {
-    // a 1x1 filter is a [K][C] matrix: the tiled transpose keeps both sides coalesced when w arrives C-major
-    // (a row-major GEMM B operand)
-    dim3 grid(static_cast<unsigned>((K + 31) / 32), static_cast<unsigned>((Cp + 31) / 32), 1u);
-    dim3 block(32, 8);
-    if (es == 2)
-      tb200::to_channels_last_kernel<uint16_t><<<grid, block, 0, stream>>>(
-          static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), (int)C, 1, (int)K, (int)Cp, 0LL, stride[1], 0LL,
-          stride[0]);
-    else
-      tb200::to_channels_last_kernel<uint32_t><<<grid, block, 0, stream>>>(
-          static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), (int)C, 1, (int)K, (int)Cp, 0LL, stride[1], 0LL,
-          stride[0]);
-  } else if (es == 2) {
+  if (es == 2) {
     tb200::pack_weights_krsc_kernel<uint16_t><<<blocks, threads, 0, stream>>>(
         static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), total, (int)C, (int)R, (int)S, (int)Sd, (int)Cp,
         stride[0], stride[1], stride[2], stride[3]);
@@ -608,7 +670,6 @@ void launch_weight_pack(const void* src, void* dst, int es, long long K, long lo
   g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
   g_launches_by_kind[3].fetch_add(1, std::memory_order_relaxed);
 }
-
 
 // ------------------------------------------------------------------ the device path
 // The conv geometry the kernel runs: the public parameters plus a separate padding behind the last row /
@@ -1047,29 +1108,16 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     x.stride[1] = 1;
     x.stride[2] = Wpitch * Cp;
     x.stride[3] = Cp;
-  } else if (!x_direct || knobs().force_staging) {
-    void* x_stage = staging(x_scratch, static_cast<size_t>(N * H * W * Cp) * es, "the channels-last copy of x");
-    dim3 grid(static_cast<unsigned>((H * W + 31) / 32), static_cast<unsigned>((Cp + 31) / 32),
-              static_cast<unsigned>(N));
-    if (grid.y > 65535u || grid.z > 65535u)
-      TB_FAIL(TRACEA_UNSUPPORTED_CONFIG, "layout adapter: N or C too large");
-    dim3 block(32, 8);
-    if (es == 2)
-      tb200::to_channels_last_kernel<uint16_t><<<grid, block, 0, stream>>>(
-          static_cast<const uint16_t*>(x.ptr), static_cast<uint16_t*>(x_stage), (int)C, (int)H,
-          (int)W, (int)Cp, x.stride[0], x.stride[1], x.stride[2], x.stride[3]);
-    else
-      tb200::to_channels_last_kernel<uint32_t><<<grid, block, 0, stream>>>(
-          static_cast<const uint32_t*>(x.ptr), static_cast<uint32_t*>(x_stage), (int)C, (int)H,
-          (int)W, (int)Cp, x.stride[0], x.stride[1], x.stride[2], x.stride[3]);
-    TB_CUDA(cudaGetLastError());
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-    g_launches_by_kind[3].fetch_add(1, std::memory_order_relaxed);
-    x.ptr = x_stage;
-    x.stride[0] = H * W * Cp;
+  }
+  const bool stage_x = !window && (!x_direct || knobs().force_staging);
+  // Rows of a staged operand start on 32-byte boundaries: the TMA unit fetches whole 32-byte sectors, and rows 16 bytes off
+  // cost it nearly twice the time (3x3 C->128 on 32 images of 28x28: C = 104 25.1 us, C = 112 13.9).
+  const long long Cs = Cp * es > 16 ? (Cp * es + 31) / 32 * 32 / es : Cp;
+  if (stage_x) {   // its address is filled in below, where the weights' form is known too
+    x.stride[0] = H * W * Cs;
     x.stride[1] = 1;
-    x.stride[2] = W * Cp;
-    x.stride[3] = Cp;
+    x.stride[2] = W * Cs;
+    x.stride[3] = Cs;
   }
 
   // ---- k-chunking: how many bytes of one pixel's channels one copy brings in (see pick_chunk_bytes)
@@ -1094,7 +1142,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   // filters of a transposed convolution). The loader then starts at column b_k0 and adds b_jump_s / b_jump_r to its
   // column at every tap / filter-row boundary. Anything else is repacked into scratch.
   const void* w_ptr = w_in.ptr;
-  Scratch w_scratch;
+  Scratch op_scratch;
   long long w_row_elems = R * S * C, w_pitch = R * S * C, b_k0 = 0, b_jump_s = 0, b_jump_r = 0;
   const bool w_dense = C == Cp && (w_in.stride[1] == 1) && w_in.stride[3] == C &&
                        w_in.stride[2] == S * C && w_in.stride[0] == R * S * C && aligned16(w_in.ptr);
@@ -1116,11 +1164,28 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
       b_jump_r = sr - S * ss;
     }
   }
-  const long long Sd = window ? 8 : S;   // tap slots per filter row in the packed weights
-  if (!w_direct || window) {
-    void* w_stage = staging(w_scratch, static_cast<size_t>(K * R * Sd * Cp) * es, "the repacked weights");
-    launch_weight_pack(w_in.ptr, w_stage, es, K, C, R, S, Sd, Cp, w_in.stride, stream);
-    w_ptr = w_stage;
+  const bool stage_w = !w_direct || window;
+  {
+    // one block of scratch and one launch for both operands
+    const long long Sd = window ? 8 : S;   // tap slots per filter row in the packed weights
+    const size_t x_bytes = stage_x ? (static_cast<size_t>(N * H * W * Cs) * es + 255) / 256 * 256 : 0;
+    const size_t w_bytes = stage_w ? static_cast<size_t>(K * R * Sd * (window ? Cp : Cs)) * es : 0;
+    tb200::CopyJob jobs[2];
+    int count = 0;
+    if (stage_x || stage_w) {
+      char* base = static_cast<char*>(staging(op_scratch, x_bytes + w_bytes, "the channels-last copies of x and w"));
+      if (stage_x) {
+        x.ptr = base;
+        jobs[count++] = copy_job(x_in.ptr, x.ptr, es, N, C, Cs, H, W, x_in.stride[0], x_in.stride[1], x_in.stride[2],
+                                 x_in.stride[3]);
+      }
+      if (stage_w) {
+        w_ptr = base + x_bytes;
+        if (window) launch_weight_pack(w_in.ptr, base + x_bytes, es, K, C, R, S, Sd, Cp, w_in.stride, stream);
+        else jobs[count++] = weight_job(w_in.ptr, base + x_bytes, es, K, C, R, S, Cs, w_in.stride);
+      }
+    }
+    launch_copies(jobs, count, es, stream);
   }
 
   const long long Kgemm = R * Sg * Cg;
@@ -1348,9 +1413,10 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     // {column, tap, output channel}. Repacked or dense weights: one row is the whole Kgemm axis, or one tap of it when
     // the k-chunks do not divide a tap; in-place strided taps: one row spans the taps
     const long long row_elems = w_remap ? w_row_elems : (ragged_taps ? Cg : Kgemm);
-    const long long k_pitch = w_remap ? w_pitch : Kgemm;
+    const long long tap_pitch = stage_w && !window ? Cs : Cg;
+    const long long k_pitch = w_remap ? w_pitch : R * Sg * tap_pitch;
     const cuuint64_t gdim[3] = {(cuuint64_t)row_elems, (cuuint64_t)(ragged_taps ? R * Sg : 1), (cuuint64_t)K};
-    const cuuint64_t gstr[2] = {(cuuint64_t)((ragged_taps ? Cg : k_pitch) * es), (cuuint64_t)(k_pitch * es)};
+    const cuuint64_t gstr[2] = {(cuuint64_t)((ragged_taps ? tap_pitch : k_pitch) * es), (cuuint64_t)(k_pitch * es)};
     const cuuint32_t box[3] = {(cuuint32_t)chunk_elems, 1u, (cuuint32_t)(pair_v ? bn / 2 : bn)};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     CUresult r = g_encode_tiled(&tmap_w, tmap_dtype(x.dtype), 3, const_cast<void*>(w_ptr), gdim, gstr,
@@ -1995,7 +2061,8 @@ void conv2d_prepack_checked(const TraceaTensorView& wv, void* dst, uint64_t dst_
   if (dst_bytes < need) TB_FAIL(TRACEA_INVALID_PARAMS, "dst holds %llu bytes, the packed weights need %llu",
                                 (unsigned long long)dst_bytes, need);
   DeviceGuard guard(w.device);
-  launch_weight_pack(w.ptr, dst, es, K, C, R, S, S, Cp, w.stride, static_cast<cudaStream_t>(stream));
+  const tb200::CopyJob job = weight_job(w.ptr, dst, es, K, C, R, S, Cp, w.stride);
+  launch_copies(&job, 1, es, static_cast<cudaStream_t>(stream));
   packed_shape[0] = (uint64_t)K; packed_shape[1] = (uint64_t)Cp; packed_shape[2] = (uint64_t)R; packed_shape[3] = (uint64_t)S;
   packed_stride[0] = R * S * Cp; packed_stride[1] = 1; packed_stride[2] = S * Cp; packed_stride[3] = Cp;
 }
@@ -2016,7 +2083,8 @@ void gemm_prepack_b_checked(const TraceaTensorView& bv, void* dst, uint64_t dst_
                                 (unsigned long long)dst_bytes, need);
   DeviceGuard guard(bv.device_id);
   const long long stride[4] = {b.stride[1], b.stride[0], 0, 0};   // filter bank [N, K, 1, 1]
-  launch_weight_pack(bv.ptr, dst, es, N, K, 1, 1, 1, K, stride, static_cast<cudaStream_t>(stream));
+  const tb200::CopyJob job = weight_job(bv.ptr, dst, es, N, K, 1, 1, K, stride);
+  launch_copies(&job, 1, es, static_cast<cudaStream_t>(stream));
   packed_stride[0] = 1;
   packed_stride[1] = K;
 }
