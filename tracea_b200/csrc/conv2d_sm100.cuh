@@ -719,7 +719,8 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
   constexpr uint32_t kBBytes = kBRows * kStageKBytes;
   constexpr uint32_t kStageBytes = kABytes + kBBytes;
   constexpr int kTileM = (kPair || kRows2) ? 2 * kBlockM : kBlockM;   // output pixels per tile
-  const uint32_t cta_rank = kPair ? cluster_ctarank() : 0u;
+  // (shuffles: the same value in every lane, provably -- the MMA warp's control flow has to be uniform)
+  const uint32_t cta_rank = kPair ? __shfl_sync(0xffffffffu, cluster_ctarank(), 0) : 0u;
   const bool leader = cta_rank == 0u;
   // tiles are dealt to CTAs (or CTA pairs) round robin
   const int worker = kPair ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
@@ -748,7 +749,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
   volatile uint32_t* tmem_slot_p = reinterpret_cast<volatile uint32_t*>(smem_gen + bar_off + 8u * kNumBars);
   volatile uint32_t* abort_p = tmem_slot_p + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -983,25 +984,29 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
     }
   } else if (warp == 1 || (kRows2 && warp == 10)) {
     // ------------------------------------------------------------ MMA issuer
-    // One thread. Descriptor low words are precomputed per k-slice; per stage they only move by the
-    // stage pitch, so an MMA costs two adds and one instruction here (the tensor pipe needs a new
-    // 128 x BN x 32-byte MMA every BN/2 cycles).
-    // kRows2 (BN <= 128): one thread cannot issue that fast -- measured about 90 cycles per MMA in this loop against
-    // the 64 an N = 128 MMA takes -- so the tile's two 128-row blocks have an issuer each (warps 1 and 10): separate
-    // accumulators, the same stages; a stage is released, and a tile handed over, when both have committed.
-    if (lane == 0 && leader) {
+    // The whole warp walks the loop in uniform control flow and one lane issues: descriptor words then live in uniform
+    // registers and an MMA costs a couple of instructions here. Descriptor low words are precomputed per k-slice; per
+    // stage they only move by the stage pitch.
+    // As a single-thread loop the same code cost one image through the 53-layer stack 6 %, the bottleneck block 1.2 %.
+    // kRows2 (BN <= 128): the tile's two 128-row blocks have an issuer each (warps 1 and 10): separate accumulators, the
+    // same stages; a stage is released, and a tile handed over, when both have committed.
+    if (leader) {
+      const uint32_t issue = elect_one_lane();
       const uint32_t blk = (kRows2 && warp == 10) ? 1u : 0u;
       constexpr bool kTf32 = OutTraits<OutT>::kTf32;
       const uint32_t desc_hi = ((args.a_sbo >> 4) & 0x3FFFu) | (1u << 14) | ((args.swizzle_mode & 7u) << 29);
       uint32_t a_k[4], b_k[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        a_k[k] = ((smem_base + args.a_mma_off[k] + blk * kABlockBytes) >> 4) | (((args.a_lbo >> 4) & 0x3FFFu) << 16);
-        b_k[k] = ((smem_base + kABytes + args.b_mma_off[k]) >> 4) | (((args.b_lbo >> 4) & 0x3FFFu) << 16);
+        a_k[k] = __shfl_sync(0xffffffffu, ((smem_base + args.a_mma_off[k] + blk * kABlockBytes) >> 4) |
+                                              (((args.a_lbo >> 4) & 0x3FFFu) << 16), 0);
+        b_k[k] = __shfl_sync(0xffffffffu, ((smem_base + kABytes + args.b_mma_off[k]) >> 4) |
+                                              (((args.b_lbo >> 4) & 0x3FFFu) << 16), 0);
       }
       constexpr uint32_t kStageUnits = kStageBytes >> 4;
       const uint32_t ring_units = ring_bytes >> 4;
       const uint32_t idesc = args.idesc;
+      const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
       uint32_t s_off = 0;                          // current stage's offset in 16-byte units
       uint32_t full_addr = full_bar0, empty_addr = empty_bar0;
       uint32_t phase = 0;
@@ -1010,7 +1015,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
       long long prof_wfull = 0, prof_wtmem = 0;
       (void)prof_wfull; (void)prof_wtmem;
       TB200_PROF_T(prof_t0);
-      bool stage_ready = mbar_test_wait(full_addr, phase);
+      bool stage_ready = __all_sync(0xffffffffu, mbar_test_wait(full_addr, phase));
       WorkIter witer;
       witer.template init<kSplit>(args, worker, k_iters);
       WorkItem item;
@@ -1018,19 +1023,19 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
         const int buf = local_tile & 1;
         const uint32_t use = static_cast<uint32_t>(local_tile >> 1);
         TB200_PROF_T(tw0);
-        if (!mbar_wait_bounded(tempty_bar(buf), (use & 1u) ^ 1u, abort_p, args.wait_limit)) {
-          report_error(args, abort_p, kErrMmaWaitTmem, (uint32_t)local_tile);
+        if (!mbar_wait_bounded_uniform(tempty_bar(buf), (use & 1u) ^ 1u, abort_p, args.wait_limit)) {
+          if (issue) report_error(args, abort_p, kErrMmaWaitTmem, (uint32_t)local_tile);
           ok = false;
           break;
         }
         TB200_PROF_ADD(prof_wtmem, tw0);
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf) * kAccCols + blk * BN;
+        const uint32_t d_tmem = tmem_u + static_cast<uint32_t>(buf) * kAccCols + blk * BN;
         for (int it = item.k_begin; it < item.k_end; ++it) {
           const bool first = it == item.k_begin;   // the piece's first MMA overwrites the accumulator
           TB200_PROF_T(tw1);
-          if (!stage_ready && !mbar_wait_bounded(full_addr, phase, abort_p, args.wait_limit)) {
-            report_error(args, abort_p, kErrMmaWaitFull, (uint32_t)it);
+          if (!stage_ready && !mbar_wait_bounded_uniform(full_addr, phase, abort_p, args.wait_limit)) {
+            if (issue) report_error(args, abort_p, kErrMmaWaitFull, (uint32_t)it);
             ok = false;
             break;
           }
@@ -1045,31 +1050,32 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               next_ready = mma_stage4_probe_pair<kTf32, false>(d_tmem, a_k[0] + s_off, a_k[1] + s_off, a_k[2] + s_off,
                                                                a_k[3] + s_off, b_k[0] + s_off, b_k[1] + s_off,
                                                                b_k[2] + s_off, b_k[3] + s_off, desc_hi, idesc,
-                                                               empty_addr, nfull, nphase);
+                                                               empty_addr, nfull, nphase, issue);
             else
               next_ready = mma_stage4_probe_pair<kTf32, true>(d_tmem, a_k[0] + s_off, a_k[1] + s_off, a_k[2] + s_off,
                                                               a_k[3] + s_off, b_k[0] + s_off, b_k[1] + s_off,
                                                               b_k[2] + s_off, b_k[3] + s_off, desc_hi, idesc,
-                                                              empty_addr, nfull, nphase);
+                                                              empty_addr, nfull, nphase, issue);
           } else {
             if (first)
               next_ready = mma_stage4_probe<kTf32, false>(d_tmem, a_k[0] + s_off, a_k[1] + s_off, a_k[2] + s_off,
                                                           a_k[3] + s_off, b_k[0] + s_off, b_k[1] + s_off, b_k[2] + s_off,
-                                                          b_k[3] + s_off, desc_hi, idesc, empty_addr, nfull, nphase);
+                                                          b_k[3] + s_off, desc_hi, idesc, empty_addr, nfull, nphase, issue);
             else
               next_ready = mma_stage4_probe<kTf32, true>(d_tmem, a_k[0] + s_off, a_k[1] + s_off, a_k[2] + s_off,
                                                          a_k[3] + s_off, b_k[0] + s_off, b_k[1] + s_off, b_k[2] + s_off,
-                                                         b_k[3] + s_off, desc_hi, idesc, empty_addr, nfull, nphase);
+                                                         b_k[3] + s_off, desc_hi, idesc, empty_addr, nfull, nphase, issue);
           }
           s_off = n_off; full_addr = nfull; empty_addr = nempty; phase = nphase;
-          stage_ready = next_ready;
+          stage_ready = __all_sync(0xffffffffu, next_ready);
         }
-        if (ok) {                                 // accumulator complete (in both CTAs of a pair)
+        if (ok && issue) {                        // accumulator complete (in both CTAs of a pair)
           if constexpr (kPair) mma_commit_pair(tfull_bar(buf));
           else mma_commit(tfull_bar(buf));
         }
+        __syncwarp();
       }
-      if (blk == 0u) {
+      if (issue && blk == 0u) {
         TB200_PROF_STORE(2, prof_wfull);
         TB200_PROF_STORE(3, prof_wtmem);
         TB200_PROF_STORE(4, clock64() - prof_t0);

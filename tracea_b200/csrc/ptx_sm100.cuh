@@ -315,39 +315,43 @@ __device__ __forceinline__ void tc_fence_after() {
 // the four MMAs of this stage, commit them to this stage's empty barrier, and only then read the
 // probe's predicate -- so the probe's latency is spent under the MMA issue instead of stalling the
 // in-order thread in front of it. Returns whether the next stage was already full.
+// Executed by the whole (converged) MMA warp with the same operands in every lane; the MMAs and the commit are predicated on
+// `issue`, 1 in one lane. In uniform control flow the operand arithmetic stays in uniform registers, where the MMA reads its
+// descriptors from.
 template <bool kTf32, bool kFirstAccumulates>
 __device__ __forceinline__ bool mma_stage4_probe(uint32_t tmem_d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                  uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3,
                                                  uint32_t desc_hi, uint32_t idesc, uint32_t empty_bar,
-                                                 uint32_t next_full_bar, uint32_t next_parity) {
+                                                 uint32_t next_full_bar, uint32_t next_parity, uint32_t issue) {
   uint32_t ready;
 #define TB200_MMA_STAGE(KIND)                                                                   \
   asm volatile(                                                                                  \
       "{\n"                                                                                      \
-      ".reg .pred pn, p0, p1;\n"                                                                 \
+      ".reg .pred pn, p0, p1, q;\n"                                                                 \
       ".reg .b64 da, db;\n"                                                                      \
       "mbarrier.test_wait.parity.shared::cta.b64 pn, [%13], %14;\n"                              \
       "setp.ne.b32 p0, %15, 0;\n"                                                                \
-      "setp.eq.b32 p1, 0, 0;\n"                                                                  \
+      "setp.eq.b32 p1, 0, 0;\n"                                                                 \
+      "setp.ne.b32 q, %16, 0;\n"                                                                \
       "mov.b64 da, {%2, %10};\n"                                                                 \
       "mov.b64 db, {%6, %10};\n"                                                                 \
-      "tcgen05.mma.cta_group::1.kind::" KIND " [%1], da, db, %11, p0;\n"                         \
+      "@q tcgen05.mma.cta_group::1.kind::" KIND " [%1], da, db, %11, p0;\n"                         \
       "mov.b64 da, {%3, %10};\n"                                                                 \
       "mov.b64 db, {%7, %10};\n"                                                                 \
-      "tcgen05.mma.cta_group::1.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
+      "@q tcgen05.mma.cta_group::1.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
       "mov.b64 da, {%4, %10};\n"                                                                 \
       "mov.b64 db, {%8, %10};\n"                                                                 \
-      "tcgen05.mma.cta_group::1.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
+      "@q tcgen05.mma.cta_group::1.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
       "mov.b64 da, {%5, %10};\n"                                                                 \
       "mov.b64 db, {%9, %10};\n"                                                                 \
-      "tcgen05.mma.cta_group::1.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%12];\n"           \
+      "@q tcgen05.mma.cta_group::1.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%12];\n"           \
       "selp.u32 %0, 1, 0, pn;\n"                                                                 \
       "}\n"                                                                                      \
       : "=r"(ready)                                                                              \
       : "r"(tmem_d), "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(b2), "r"(b3),     \
         "r"(desc_hi), "r"(idesc), "r"(empty_bar), "r"(next_full_bar), "r"(next_parity),          \
-        "n"(kFirstAccumulates ? 1 : 0)                                                           \
+        "n"(kFirstAccumulates ? 1 : 0), "r"(issue)                                                           \
       : "memory")
   if constexpr (kTf32) {
     TB200_MMA_STAGE("tf32");
@@ -365,37 +369,38 @@ template <bool kTf32, bool kFirstAccumulates>
 __device__ __forceinline__ bool mma_stage4_probe_pair(uint32_t tmem_d, uint32_t a0, uint32_t a1, uint32_t a2,
                                                       uint32_t a3, uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3,
                                                       uint32_t desc_hi, uint32_t idesc, uint32_t empty_bar,
-                                                      uint32_t next_full_bar, uint32_t next_parity) {
+                                                      uint32_t next_full_bar, uint32_t next_parity, uint32_t issue) {
   uint32_t ready;
 #define TB200_MMA_STAGE2(KIND)                                                                  \
   asm volatile(                                                                                  \
       "{\n"                                                                                      \
-      ".reg .pred pn, p0, p1;\n"                                                                 \
+      ".reg .pred pn, p0, p1, q;\n"                                                                 \
       ".reg .b64 da, db;\n"                                                                      \
       ".reg .b16 msk;\n"                                                                         \
       "mov.b16 msk, 3;\n"                                                                        \
       "mbarrier.test_wait.parity.shared::cta.b64 pn, [%13], %14;\n"                              \
       "setp.ne.b32 p0, %15, 0;\n"                                                                \
-      "setp.eq.b32 p1, 0, 0;\n"                                                                  \
+      "setp.eq.b32 p1, 0, 0;\n"                                                                 \
+      "setp.ne.b32 q, %16, 0;\n"                                                                \
       "mov.b64 da, {%2, %10};\n"                                                                 \
       "mov.b64 db, {%6, %10};\n"                                                                 \
-      "tcgen05.mma.cta_group::2.kind::" KIND " [%1], da, db, %11, p0;\n"                         \
+      "@q tcgen05.mma.cta_group::2.kind::" KIND " [%1], da, db, %11, p0;\n"                         \
       "mov.b64 da, {%3, %10};\n"                                                                 \
       "mov.b64 db, {%7, %10};\n"                                                                 \
-      "tcgen05.mma.cta_group::2.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
+      "@q tcgen05.mma.cta_group::2.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
       "mov.b64 da, {%4, %10};\n"                                                                 \
       "mov.b64 db, {%8, %10};\n"                                                                 \
-      "tcgen05.mma.cta_group::2.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
+      "@q tcgen05.mma.cta_group::2.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
       "mov.b64 da, {%5, %10};\n"                                                                 \
       "mov.b64 db, {%9, %10};\n"                                                                 \
-      "tcgen05.mma.cta_group::2.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%12], msk;\n" \
+      "@q tcgen05.mma.cta_group::2.kind::" KIND " [%1], da, db, %11, p1;\n"                         \
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%12], msk;\n" \
       "selp.u32 %0, 1, 0, pn;\n"                                                                 \
       "}\n"                                                                                      \
       : "=r"(ready)                                                                              \
       : "r"(tmem_d), "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(b2), "r"(b3),     \
         "r"(desc_hi), "r"(idesc), "r"(empty_bar), "r"(next_full_bar), "r"(next_parity),          \
-        "n"(kFirstAccumulates ? 1 : 0)                                                           \
+        "n"(kFirstAccumulates ? 1 : 0), "r"(issue)                                                           \
       : "memory")
   if constexpr (kTf32) {
     TB200_MMA_STAGE2("tf32");
