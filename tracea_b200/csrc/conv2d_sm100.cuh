@@ -731,7 +731,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
 
   TB200_PROF_NOW(12);
   extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t smem_base = __shfl_sync(0xffffffffu, (smem_u32(smem_raw) + 1023u) & ~1023u, 0);
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const int num_stages = args.num_stages;
   const uint32_t ring_bytes = static_cast<uint32_t>(num_stages) * kStageBytes;
@@ -818,14 +818,16 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
     nt = n0 + rem - mt * width;
   };
   const uint32_t full_bar0 = bar_base, empty_bar0 = bar_base + 8u * kMaxStages;
-  const uint32_t full_leader0 = kPair ? mapa_cluster(full_bar0, 0u) : full_bar0;   // leader's full barriers
+  const uint32_t full_leader0 = kPair ? __shfl_sync(0xffffffffu, mapa_cluster(full_bar0, 0u), 0) : full_bar0;   // leader's full barriers
   const uint32_t ring_end = smem_base + ring_bytes;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    // One thread; the loop body is kept to a handful of instructions per stage, because at
-    // 256 cycles of tensor work per stage (BN = 128) the issuing thread itself can become the limit.
-    if (lane == 0) {
+    // The whole warp walks the loop in uniform control flow and one lane issues. As a loop of one thread, with every operand
+    // moved to a uniform register in front of each copy, a stage took ~500 cycles to issue -- with its slots free: this
+    // thread, not the memory system or the tensor pipe, was what bounded every tiling.
+    {
+      const uint32_t issue = elect_one_lane();
       uint32_t stage_addr = smem_base;             // A buffer of the current stage
       uint32_t full_addr = full_bar0, empty_addr = empty_bar0;
       uint32_t phase = 0;
@@ -838,7 +840,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
       long long prof_wait = 0;
       (void)prof_wait;
       TB200_PROF_T(prof_t0);
-      bool slot_free = mbar_test_wait(empty_addr, phase ^ 1u);
+      bool slot_free = __all_sync(0xffffffffu, mbar_test_wait(empty_addr, phase ^ 1u));
       WorkIter witer;
       witer.template init<kSplit>(args, worker, k_iters);
       WorkItem item;
@@ -883,8 +885,8 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               break;
             }
             TB200_PROF_T(tw);
-            if (!slot_free && !mbar_wait_bounded(empty_addr, phase ^ 1u, abort_p, args.wait_limit)) {
-              report_error(args, abort_p, kErrProducerWait, (uint32_t)it);
+            if (!slot_free && !mbar_wait_bounded_uniform(empty_addr, phase ^ 1u, abort_p, args.wait_limit)) {
+              if (issue) report_error(args, abort_p, kErrProducerWait, (uint32_t)it);
               ok = false;
               break;
             }
@@ -898,16 +900,16 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               next_free = tma_stage_probe_pair(stage_addr, stage_addr + kABytes, full_addr,
                                                full_leader0 + (full_addr - full_bar0), leader ? 2u * kStageBytes : 0u,
                                                &tmap_x, c_coord, w_start, h_start, img0, (uint16_t)off_w,
-                                               (uint16_t)off_h, &tmap_w, k_coord, tap_coord, n_coord, nempty, nphase ^ 1u);
+                                               (uint16_t)off_h, &tmap_w, k_coord, tap_coord, n_coord, nempty, nphase ^ 1u, issue);
             } else if constexpr (kRows2) {
               next_free = tma_stage_probe_rows2(stage_addr, stage_addr + kABlockBytes, stage_addr + kABytes, full_addr,
                                                 kStageBytes, &tmap_x, c_coord, w_start, h_start, img0, w_start1,
                                                 h_start1, img1, (uint16_t)off_w, (uint16_t)off_h, &tmap_w, k_coord,
-                                                tap_coord, n_coord, nempty, nphase ^ 1u);
+                                                tap_coord, n_coord, nempty, nphase ^ 1u, issue);
             } else {
               next_free = tma_stage_probe(stage_addr, stage_addr + kABytes, full_addr, kStageBytes, &tmap_x, c_coord,
                                           w_start, h_start, img0, (uint16_t)off_w, (uint16_t)off_h, &tmap_w, k_coord,
-                                          tap_coord, n_coord, nempty, nphase ^ 1u);
+                                          tap_coord, n_coord, nempty, nphase ^ 1u, issue);
             }
             k_coord += args.chunk_elems;
             c_coord += args.chunk_elems;
@@ -920,18 +922,18 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
             }
             ++issued;
             stage_addr = nstage; full_addr = nfull; empty_addr = nempty; phase = nphase;
-            slot_free = next_free;
+            slot_free = __all_sync(0xffffffffu, next_free);
           }
         } else {
           // narrow k-chunks (several per stage): whole tiles only, the host never splits these over K
           int chunk = 0, tap_r = 0, tap_s = 0, cc = 0, b_col = 0, tap_coord = 0;
           for (int it = 0; it < k_iters; ++it) {
-            if (!mbar_wait_bounded(empty_addr, phase ^ 1u, abort_p, args.wait_limit)) {
-              report_error(args, abort_p, kErrProducerWait, (uint32_t)it);
+            if (!mbar_wait_bounded_uniform(empty_addr, phase ^ 1u, abort_p, args.wait_limit)) {
+              if (issue) report_error(args, abort_p, kErrProducerWait, (uint32_t)it);
               ok = false;
               break;
             }
-            mbar_arrive_expect_tx(full_addr, kStageBytes);
+            mbar_arrive_expect_tx_if(issue, full_addr, kStageBytes);
             const uint32_t a_dst = stage_addr;
             const uint32_t b_dst = a_dst + kABytes;
             for (int j = 0; j < chunks_per_stage; ++j, ++chunk) {
@@ -941,13 +943,13 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               // (the last tap's row ends at or before column args.C, a single contiguous row at total_chunks chunks)
               const int k_coord = pad_chunk ? args.total_chunks * args.chunk_elems : b_col;
               if (args.a_tiled) {
-                tma_load_2d(a_dst + j * a_chunk_bytes, &tmap_x, full_addr, c_coord, m0);
+                tma_load_2d_if(issue, a_dst + j * a_chunk_bytes, &tmap_x, full_addr, c_coord, m0);
               } else {
-                tma_load_im2col_4d(a_dst + j * a_chunk_bytes, &tmap_x, full_addr, c_coord,
+                tma_load_im2col_4d_if(issue, a_dst + j * a_chunk_bytes, &tmap_x, full_addr, c_coord,
                                    w_start, h_start, img0, (uint16_t)(tap_s * args.dil_w),
                                    (uint16_t)(tap_r * args.dil_h));
               }
-              tma_load_3d(b_dst + j * b_chunk_bytes, &tmap_w, full_addr, k_coord, tap_coord, n_coord);
+              tma_load_3d_if(issue, b_dst + j * b_chunk_bytes, &tmap_w, full_addr, k_coord, tap_coord, n_coord);
               if (!pad_chunk) {
                 b_col += args.chunk_elems;
                 if (++cc == args.chunks_per_tap) {
@@ -965,14 +967,16 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
           slot_free = false;   // this path waits in full every time
         }
       }
-      TB200_PROF_STORE(0, prof_wait);
-      TB200_PROF_STORE(1, clock64() - prof_t0);
+      if (issue) {
+        TB200_PROF_STORE(0, prof_wait);
+        TB200_PROF_STORE(1, clock64() - prof_t0);
+      }
       // Never leave with copies in flight into this CTA's shared memory: wait (bounded) until the
       // MMA side has released every stage that was filled.
       if (ok) {
         const int pending = issued < num_stages ? issued : num_stages;
         for (int i = 0; i < pending; ++i) {
-          if (!mbar_wait_bounded(empty_addr, phase ^ 1u, abort_p, args.wait_limit)) break;
+          if (!mbar_wait_bounded_uniform(empty_addr, phase ^ 1u, abort_p, args.wait_limit)) break;
           stage_addr += kStageBytes; empty_addr += 8u;
           if (stage_addr == ring_end) { stage_addr = smem_base; empty_addr = empty_bar0; phase ^= 1u; }
         }

@@ -201,6 +201,49 @@ __device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const void* tma
       : "memory");
 }
 
+// The same loads, executed by a whole converged warp with the same operands in every lane and predicated on `issue`, 1 in one
+// lane: see tma_stage_probe.
+__device__ __forceinline__ void mbar_arrive_expect_tx_if(uint32_t issue, uint32_t bar, uint32_t bytes) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %2, 0;\n"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
+      "}\n" ::"r"(bar), "r"(bytes), "r"(issue)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_if(uint32_t issue, uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %5, 0;\n"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
+      "}\n" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(issue)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_if(uint32_t issue, uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1,
+                                               int c2) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %6, 0;\n"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
+      "}\n" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(issue)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_im2col_4d_if(uint32_t issue, uint32_t dst, const void* tmap, uint32_t bar, int c, int w,
+                                                      int h, int n, uint16_t off_w, uint16_t off_h) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %9, 0;\n"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};\n"
+      "}\n" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w),
+      "h"(off_h), "r"(issue)
+      : "memory");
+}
+
 // Same im2col box, but only pulled into L2 (no shared-memory destination, no barrier): used to run the
 // HBM fetch of the activations several k-steps ahead of the shared-memory ring.
 __device__ __forceinline__ void tma_prefetch_im2col_4d(const void* tmap, int c, int w, int h, int n, uint16_t off_w,
@@ -429,51 +472,55 @@ __device__ __forceinline__ bool tma_stage_probe_pair(uint32_t a_dst, uint32_t b_
                                                      uint32_t full_bar_leader, uint32_t expect_bytes,
                                                      const void* tmap_x, int c, int w, int h, int n, uint16_t off_w,
                                                      uint16_t off_h, const void* tmap_w, int k0, int tap, int n0,
-                                                     uint32_t next_empty_bar, uint32_t next_parity) {
+                                                     uint32_t next_empty_bar, uint32_t next_parity, uint32_t issue) {
   uint32_t free_next;
   asm volatile(
       "{\n"
-      ".reg .pred pn, pl;\n"
+      ".reg .pred pn, pl, q;\n"
       "mbarrier.test_wait.parity.shared::cta.b64 pn, [%17], %18;\n"
-      "setp.ne.b32 pl, %4, 0;\n"
+      "setp.ne.b32 q, %19, 0;\n"
+      "setp.ne.and.b32 pl, %4, 0, q;\n"
       "@pl mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %4;\n"
-      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+      "@q cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
       " [%1], [%6, {%7, %8, %9, %10}], [%5], {%11, %12};\n"
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%2], [%13, {%14, %15, %16}], [%5];\n"
       "selp.u32 %0, 1, 0, pn;\n"
       "}\n"
       : "=r"(free_next)
       : "r"(a_dst), "r"(b_dst), "r"(full_bar_local), "r"(expect_bytes), "r"(full_bar_leader),
         "l"(reinterpret_cast<uint64_t>(tmap_x)), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h),
-        "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(tap), "r"(n0), "r"(next_empty_bar), "r"(next_parity)
+        "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(tap), "r"(n0), "r"(next_empty_bar), "r"(next_parity),
+        "r"(issue)
       : "memory");
   return free_next != 0;
 }
 
 // One pipeline stage of the TMA producer as a single block, same idea: probe the NEXT slot's empty
 // barrier first, then arm this slot's full barrier and issue the im2col copy of A and the tiled copy
-// of B, then read the probe.
+// of B, then read the probe. Like the MMAs' stage (and for the same reason) executed by a whole converged warp with the same
+// operands in every lane, the copies predicated on `issue`.
 __device__ __forceinline__ bool tma_stage_probe(uint32_t a_dst, uint32_t b_dst, uint32_t full_bar, uint32_t stage_bytes,
                                                 const void* tmap_x, int c, int w, int h, int n, uint16_t off_w,
                                                 uint16_t off_h, const void* tmap_w, int k0, int tap, int n0,
-                                                uint32_t next_empty_bar, uint32_t next_parity) {
+                                                uint32_t next_empty_bar, uint32_t next_parity, uint32_t issue) {
   uint32_t free_next;
   asm volatile(
       "{\n"
-      ".reg .pred pn;\n"
+      ".reg .pred pn, q;\n"
       "mbarrier.test_wait.parity.shared::cta.b64 pn, [%16], %17;\n"
-      "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %4;\n"
-      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+      "setp.ne.b32 q, %18, 0;\n"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %4;\n"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
       " [%1], [%5, {%6, %7, %8, %9}], [%3], {%10, %11};\n"
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%2], [%12, {%13, %14, %15}], [%3];\n"
       "selp.u32 %0, 1, 0, pn;\n"
       "}\n"
       : "=r"(free_next)
       : "r"(a_dst), "r"(b_dst), "r"(full_bar), "r"(stage_bytes), "l"(reinterpret_cast<uint64_t>(tmap_x)), "r"(c),
         "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h), "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(tap),
-        "r"(n0), "r"(next_empty_bar), "r"(next_parity)
+        "r"(n0), "r"(next_empty_bar), "r"(next_parity), "r"(issue)
       : "memory");
   return free_next != 0;
 }
@@ -484,25 +531,28 @@ __device__ __forceinline__ bool tma_stage_probe_rows2(uint32_t a0_dst, uint32_t 
                                                       uint32_t full_bar, uint32_t stage_bytes, const void* tmap_x,
                                                       int c, int w0, int h0, int n0i, int w1, int h1, int n1i,
                                                       uint16_t off_w, uint16_t off_h, const void* tmap_w, int k0, int tap,
-                                                      int ncol, uint32_t next_empty_bar, uint32_t next_parity) {
+                                                      int ncol, uint32_t next_empty_bar, uint32_t next_parity,
+                                                      uint32_t issue) {
   uint32_t free_next;
   asm volatile(
       "{\n"
-      ".reg .pred pn;\n"
+      ".reg .pred pn, q;\n"
       "mbarrier.test_wait.parity.shared::cta.b64 pn, [%20], %21;\n"
-      "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n"
-      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+      "setp.ne.b32 q, %22, 0;\n"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%4], %5;\n"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
       " [%1], [%6, {%7, %8, %9, %10}], [%4], {%14, %15};\n"
-      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
       " [%2], [%6, {%7, %11, %12, %13}], [%4], {%14, %15};\n"
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%3], [%16, {%17, %18, %19}], [%4];\n"
       "selp.u32 %0, 1, 0, pn;\n"
       "}\n"
       : "=r"(free_next)
       : "r"(a0_dst), "r"(a1_dst), "r"(b_dst), "r"(full_bar), "r"(stage_bytes), "l"(reinterpret_cast<uint64_t>(tmap_x)),
         "r"(c), "r"(w0), "r"(h0), "r"(n0i), "r"(w1), "r"(h1), "r"(n1i), "h"(off_w), "h"(off_h),
-        "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(tap), "r"(ncol), "r"(next_empty_bar), "r"(next_parity)
+        "l"(reinterpret_cast<uint64_t>(tmap_w)), "r"(k0), "r"(tap), "r"(ncol), "r"(next_empty_bar), "r"(next_parity),
+        "r"(issue)
       : "memory");
   return free_next != 0;
 }
