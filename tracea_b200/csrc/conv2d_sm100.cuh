@@ -103,6 +103,9 @@ struct ConvKernelArgs {
   long long out_sn, out_sh, out_sw, out_sc;
   int out_vec;            // kStoreRows: bytes a lane may store at once (16, 4, or one element)
   int out_quad;           // kStoreStrided: four consecutive pixels are always 8 consecutive, aligned bytes (16-bit types)
+  // small-tile kernel: output and residual are channel-contiguous; A's / B's map is {column in chunk, row, chunk} and one
+  // copy brings in two k-steps; the weights are the caller's, worth an early prefetch
+  int out_rows, a_steps2, b_steps2, b_prefetch;
   const void* bias;       // [K_out], fp32 or OutT
   int bias_is_f32;
   const void* residual;   // same dtype as out

@@ -254,6 +254,14 @@ __device__ __forceinline__ void tma_prefetch_im2col_4d(const void* tmap, int c, 
                : "memory");
 }
 
+// A tiled 3-D box, likewise only pulled into L2.
+__device__ __forceinline__ void tma_prefetch_3d(const void* tmap, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
+               :
+               : "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+
 // Tiled 2-D store shared -> global (bulk-group completion). Rows / columns outside the tensor are
 // clipped by the TMA unit, which is what handles the M and K_out tails.
 __device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t src, int c0, int c1) {
@@ -403,6 +411,43 @@ __device__ __forceinline__ bool mma_stage4_probe(uint32_t tmem_d, uint32_t a0, u
   }
 #undef TB200_MMA_STAGE
   return ready != 0;
+}
+
+// The four MMAs of one 128-byte k-step on their own (whole-warp code, see mma_stage4_probe).
+template <bool kTf32, bool kFirstAccumulates>
+__device__ __forceinline__ void mma_step4(uint32_t tmem_d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                          uint32_t b1, uint32_t b2, uint32_t b3, uint32_t desc_hi, uint32_t idesc,
+                                          uint32_t issue) {
+#define TB200_MMA_STEP(KIND)                                                                    \
+  asm volatile(                                                                                  \
+      "{\n"                                                                                      \
+      ".reg .pred p0, p1, q;\n"                                                                  \
+      ".reg .b64 da, db;\n"                                                                      \
+      "setp.ne.b32 p0, %11, 0;\n"                                                                \
+      "setp.eq.b32 p1, 0, 0;\n"                                                                  \
+      "setp.ne.b32 q, %12, 0;\n"                                                                 \
+      "mov.b64 da, {%1, %9};\n"                                                                  \
+      "mov.b64 db, {%5, %9};\n"                                                                  \
+      "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], da, db, %10, p0;\n"                      \
+      "mov.b64 da, {%2, %9};\n"                                                                  \
+      "mov.b64 db, {%6, %9};\n"                                                                  \
+      "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], da, db, %10, p1;\n"                      \
+      "mov.b64 da, {%3, %9};\n"                                                                  \
+      "mov.b64 db, {%7, %9};\n"                                                                  \
+      "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], da, db, %10, p1;\n"                      \
+      "mov.b64 da, {%4, %9};\n"                                                                  \
+      "mov.b64 db, {%8, %9};\n"                                                                  \
+      "@q tcgen05.mma.cta_group::1.kind::" KIND " [%0], da, db, %10, p1;\n"                      \
+      "}\n" ::"r"(tmem_d),                                                                       \
+      "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(b2), "r"(b3), "r"(desc_hi),      \
+      "r"(idesc), "n"(kFirstAccumulates ? 1 : 0), "r"(issue)                                     \
+      : "memory")
+  if constexpr (kTf32) {
+    TB200_MMA_STEP("tf32");
+  } else {
+    TB200_MMA_STEP("f16");
+  }
+#undef TB200_MMA_STEP
 }
 
 // The same stage for a CTA pair: issued by the leader CTA only; each MMA spans both SMs (M = 256: 128 rows of

@@ -24,6 +24,7 @@
 
 #include "../../include/tracea_b200.h"
 #include "conv2d_sm100.cuh"
+#include "conv2d_small_sm100.cuh"
 #include "conv2d_window_sm100.cuh"
 #include "conv2d_rowband_sm100.cuh"
 #include "layout_kernels.cuh"
@@ -471,6 +472,35 @@ void launch_tiling(DeviceState& st, int dt_idx, int bn, bool pair, bool rows2, c
     case 128: launch_one<OutT, 128, false, false, kStore>(st, dt_idx, 1, tx, tw, to, tr, args, grid, smem, stream); break;
     default: launch_one<OutT, 256, false, false, kStore>(st, dt_idx, 2, tx, tw, to, tr, args, grid, smem, stream); break;
   }
+}
+
+std::atomic<bool> g_small_attr_set[kMaxDevices][3][2];
+
+template <typename OutT, int BN>
+void launch_small(DeviceState& st, int dt_idx, const CUtensorMap& tx, const CUtensorMap& tw, const ConvKernelArgs& args,
+                  int grid, cudaStream_t stream) {
+  auto kern = tb200::conv2d_small_sm100_kernel<OutT, BN>;
+  const int smem = tb200::small_smem_bytes(BN, args.num_stages);
+  std::atomic<bool>& attr_done = g_small_attr_set[st.dev][dt_idx][BN / 64];
+  if (!attr_done.load(std::memory_order_relaxed)) {
+    TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 tb200::small_smem_bytes(BN, tb200::small_stages(BN))));
+    attr_done.store(true, std::memory_order_relaxed);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(tb200::kSmallThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = knobs().pdl != 0 ? 1 : 0;
+  TB_CUDA(cudaLaunchKernelEx(&cfg, kern, tx, tw, args));
+  TB_CUDA(cudaGetLastError());
+  g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+  g_launches_by_kind[0].fetch_add(1, std::memory_order_relaxed);
 }
 
 template <typename OutT>
@@ -1221,6 +1251,38 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   const bool rows2 = !pair && chunk_bytes == 128 && bn <= 128 && rows2_env != 0 &&
                      (rows2_env == 1 || (total_chunks_ll >= 7 && 8 * waves_256 < 5 * waves_128));
 
+  // ---- problems of up to one wave: the small-tile kernel (conv2d_small_sm100.cuh). Where two k-steps come in one copy per
+  // operand -- 1x1 convolutions and products over whole 128-byte chunks -- a k-step takes it about half the general kernel's
+  // time (2048 -> 512 channels on one 7x7 image 8.3 -> 5.1 us, 64 x 1000 x 2048 8.7 -> 5.3); with im2col copies a step costs
+  // more than the general kernel's, and the microsecond that its launch is shorter by pays for about 30 of them (3x3, one
+  // image: 64 channels 5.1 -> 4.5, 128 channels 6.5 -> 6.1, but 256 channels 9.3 -> 9.6). More than one tile per SM gains
+  // nothing (1x1 64->64 at 4 images: 196 tiles, 3.65 -> 3.88). Costs in cycles.
+  const bool whole_chunks = chunk_bytes == 128 && row_bytes % 128 == 0;
+  const bool plain_a = whole_chunks && !window && R == 1 && S == 1 && p.stride_h == 1 && p.stride_w == 1 &&
+                       p.padding_h == 0 && p.padding_w == 0 && p.pad_h_hi == 0 && p.pad_w_hi == 0 &&
+                       x.stride[2] == W * x.stride[3] && x.stride[0] == H * x.stride[2];
+  int small_bn = 0;
+  if (chunk_bytes == 128 && forced_bn == 0 && pair_env == -1 && rows2_env == -1 && knobs().split_k == 0 &&
+      knobs().tiled_a == 0) {
+    const long long k_steps = total_chunks_ll;
+    const long long pair_waves = ((m_tiles_128 + 1) / 2 * n_tiles + st.num_sms / 2 - 1) / std::max(1, st.num_sms / 2);
+    const long long general = pair ? pair_waves * 512 : (rows2 ? waves_256 * (bn == 128 ? 640 : 480)
+                                                              : waves_128 * (bn == 256 ? 512 : (bn == 128 ? 400 : 300)));
+    long long best = general * k_steps + 1900;
+    const long long m_tiles_64 = (M + tb200::kSmallM - 1) / tb200::kSmallM;
+    for (int b = 64; b >= 32; b >>= 1) {
+      if (m_tiles_64 * ((K + b - 1) / b) > st.num_sms) continue;
+      const long long cost = k_steps * (plain_a ? (b == 32 ? 130 : 160) : (b == 32 ? 360 : 410));
+      if (cost < best) {
+        best = cost;
+        small_bn = b;
+      }
+    }
+  }
+  const bool b_steps2 = small_bn != 0 && whole_chunks && !w_remap;
+  const bool a_steps2 = small_bn != 0 && plain_a;
+  const int a_rows = small_bn != 0 ? tb200::kSmallM : tb200::kBlockM;
+
   // ---- tensor maps shared by every launch of this call
   CUtensorMap tmap_x, tmap_out, tmap_res;
   memset(&tmap_out, 0, sizeof(tmap_out));
@@ -1231,7 +1293,16 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
                        p.stride_w == 1 && p.padding_h == 0 && p.padding_w == 0 && p.pad_h_hi == 0 && p.pad_w_hi == 0 &&
                        x.stride[3] == Cp &&
                        x.stride[2] == W * Cp && x.stride[0] == H * W * Cp;
-  if (a_tiled) {
+  if (a_steps2) {   // {column in chunk, pixel, chunk}
+    const cuuint64_t gdim[3] = {(cuuint64_t)chunk_elems, (cuuint64_t)M, (cuuint64_t)chunks_per_tap};
+    const cuuint64_t gstr[2] = {(cuuint64_t)(x.stride[3] * es), 128};
+    const cuuint32_t box[3] = {(cuuint32_t)chunk_elems, (cuuint32_t)a_rows, 2u};
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    CUresult r = g_encode_tiled(&tmap_x, tmap_dtype(x.dtype), 3, x.ptr, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled (A chunks) failed with %d", (int)r);
+  } else if (a_tiled) {
     const cuuint64_t gdim[2] = {(cuuint64_t)Cp, (cuuint64_t)M};
     const cuuint64_t gstr[1] = {(cuuint64_t)(Cp * es)};
     const cuuint32_t box[2] = {(cuuint32_t)chunk_elems, (cuuint32_t)tb200::kBlockM};
@@ -1252,7 +1323,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
                           (int)p.pad_h_hi - (int)((R - 1) * p.dilation_h)};
     const cuuint32_t estr[4] = {1u, p.stride_w, p.stride_h, 1u};
     CUresult r = g_encode_im2col(&tmap_x, tmap_dtype(x.dtype), 4, x.ptr, gdim, gstr, lower, upper,
-                                 (cuuint32_t)chunk_elems, (cuuint32_t)tb200::kBlockM, estr,
+                                 (cuuint32_t)chunk_elems, (cuuint32_t)a_rows, estr,
                                  CU_TENSOR_MAP_INTERLEAVE_NONE, tmap_swizzle(chunk_bytes),
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1291,7 +1362,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   // K-major operand descriptors. Swizzled rows of chunk_bytes: 8-row groups are 8*chunk_bytes apart
   // (SBO) and one MMA (32 B of K) stays inside a row. Unswizzled 16-byte chunks: an 8-row x 16 B core
   // matrix is 128 contiguous bytes (SBO) and the MMA's second K half is the next chunk (LBO).
-  const uint32_t a_chunk = tb200::kBlockM * chunk_bytes, b_chunk = bn * chunk_bytes;
+  const uint32_t a_chunk = a_rows * chunk_bytes, b_chunk = (small_bn != 0 ? small_bn : bn) * chunk_bytes;
   if (chunk_bytes >= 32) {
     a.swizzle_mode = chunk_bytes == 128 ? 2u : (chunk_bytes == 64 ? 4u : 6u);
     a.a_sbo = a.b_sbo = 8u * chunk_bytes;
@@ -1353,7 +1424,8 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     else if (K > 4 || a.out_vec == 16)
       store = tb200::kStoreRows;
   }
-  if (store == tb200::kStoreTma) {
+  a.out_rows = store != tb200::kStoreStrided;
+  if (store == tb200::kStoreTma && small_bn == 0) {
     encode_rows(&tmap_out, out, CU_TENSOR_MAP_L2_PROMOTION_NONE, "out");
     if (res_v != nullptr) encode_rows(&tmap_res, *res_v, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, "residual");
   }
@@ -1392,6 +1464,34 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
 #endif
   const uint32_t fmt = x.dtype == TRACEA_DTYPE_FLOAT16 ? 0u : (x.dtype == TRACEA_DTYPE_BFLOAT16 ? 1u : 2u);
 
+  auto encode_w = [&](CUtensorMap* m, int box_rows) {
+    if (b_steps2) {   // {column in chunk, output channel, chunk of Kgemm}
+      const cuuint64_t gdim[3] = {(cuuint64_t)chunk_elems, (cuuint64_t)K, (cuuint64_t)total_chunks_ll};
+      const cuuint64_t gstr[2] = {(cuuint64_t)(Kgemm * es), 128};
+      const cuuint32_t box[3] = {(cuuint32_t)chunk_elems, (cuuint32_t)box_rows, 2u};
+      const cuuint32_t estr[3] = {1u, 1u, 1u};
+      CUresult r = g_encode_tiled(m, tmap_dtype(x.dtype), 3, const_cast<void*>(w_ptr), gdim, gstr, box, estr,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      if (r != CUDA_SUCCESS) TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled (B chunks) failed with %d", (int)r);
+      return;
+    }
+    // {column, tap, output channel}. Repacked or dense weights: one row is the whole Kgemm axis, or one tap of it when
+    // the k-chunks do not divide a tap; in-place strided taps: one row spans the taps
+    const long long row_elems = w_remap ? w_row_elems : (ragged_taps ? Cg : Kgemm);
+    const long long tap_pitch = stage_w && !window ? Cs : Cg;
+    const long long k_pitch = w_remap ? w_pitch : R * Sg * tap_pitch;
+    const cuuint64_t gdim[3] = {(cuuint64_t)row_elems, (cuuint64_t)(ragged_taps ? R * Sg : 1), (cuuint64_t)K};
+    const cuuint64_t gstr[2] = {(cuuint64_t)((ragged_taps ? tap_pitch : k_pitch) * es), (cuuint64_t)(k_pitch * es)};
+    const cuuint32_t box[3] = {(cuuint32_t)chunk_elems, 1u, (cuuint32_t)box_rows};
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    CUresult r = g_encode_tiled(m, tmap_dtype(x.dtype), 3, const_cast<void*>(w_ptr), gdim, gstr,
+                                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, tmap_swizzle(chunk_bytes),
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+      TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled failed with %d (Kgemm=%lld K=%lld bn=%d)", (int)r,
+              Kgemm, K, box_rows);
+  };
   // ---- one launch over output pixels [row_begin, row_end) with the given tiling. (Splitting a partly filled last
   // wave off into a second launch with 128-row tiles was measured and is slower: a CTA pair's 256-row tile costs
   // each SM exactly what a 128-row tile costs it, so the tail does not get shorter, and the launch boundary adds
@@ -1410,21 +1510,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     const int smem = tb200::conv_smem_bytes(bn, stages, pair_v, rows2_v, shared_bias);
 
     CUtensorMap tmap_w;
-    // {column, tap, output channel}. Repacked or dense weights: one row is the whole Kgemm axis, or one tap of it when
-    // the k-chunks do not divide a tap; in-place strided taps: one row spans the taps
-    const long long row_elems = w_remap ? w_row_elems : (ragged_taps ? Cg : Kgemm);
-    const long long tap_pitch = stage_w && !window ? Cs : Cg;
-    const long long k_pitch = w_remap ? w_pitch : R * Sg * tap_pitch;
-    const cuuint64_t gdim[3] = {(cuuint64_t)row_elems, (cuuint64_t)(ragged_taps ? R * Sg : 1), (cuuint64_t)K};
-    const cuuint64_t gstr[2] = {(cuuint64_t)((ragged_taps ? tap_pitch : k_pitch) * es), (cuuint64_t)(k_pitch * es)};
-    const cuuint32_t box[3] = {(cuuint32_t)chunk_elems, 1u, (cuuint32_t)(pair_v ? bn / 2 : bn)};
-    const cuuint32_t estr[3] = {1u, 1u, 1u};
-    CUresult r = g_encode_tiled(&tmap_w, tmap_dtype(x.dtype), 3, const_cast<void*>(w_ptr), gdim, gstr,
-                                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, tmap_swizzle(chunk_bytes),
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS)
-      TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled failed with %d (Kgemm=%lld K=%lld bn=%d)", (int)r,
-              Kgemm, K, bn);
+    encode_w(&tmap_w, pair_v ? bn / 2 : bn);
 
     ConvKernelArgs la = a;
     la.m_begin = static_cast<int>(row_begin);
@@ -1527,6 +1613,31 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
         break;
     }
   };
+  if (small_bn != 0) {
+    const long long tiles_n = (K + small_bn - 1) / small_bn;
+    const long long tiles = (M + tb200::kSmallM - 1) / tb200::kSmallM * tiles_n;
+    CUtensorMap tmap_w;
+    encode_w(&tmap_w, small_bn);
+    a.M = static_cast<int>(M);
+    a.num_n_tiles = static_cast<int>(tiles_n);
+    const long long stages_needed = (total_chunks_ll + 1) / 2;   // two 128-byte k-steps each
+    a.num_stages = static_cast<int>(std::min<long long>(tb200::small_stages(small_bn), stages_needed));
+    a.idesc = tb200::ptx::make_idesc(fmt, tb200::kSmallM, small_bn);
+    a.a_steps2 = a_steps2 ? 1 : 0;
+    a.b_steps2 = b_steps2 ? 1 : 0;
+    a.b_prefetch = b_steps2 && !stage_w ? 1 : 0;
+    const int dt_idx = x.dtype == TRACEA_DTYPE_BFLOAT16 ? 0 : (x.dtype == TRACEA_DTYPE_FLOAT16 ? 1 : 2);
+    const int grid = static_cast<int>(tiles);
+    auto go = [&](auto tag) {
+      using T = decltype(tag);
+      if (small_bn == 32) launch_small<T, 32>(st, dt_idx, tmap_x, tmap_w, a, grid, stream);
+      else launch_small<T, 64>(st, dt_idx, tmap_x, tmap_w, a, grid, stream);
+    };
+    if (dt_idx == 0) go(__nv_bfloat16{});
+    else if (dt_idx == 1) go(__half{});
+    else go(0.0f);
+    return;
+  }
   launch_rows(pair, rows2, 0, M);
 }
 
