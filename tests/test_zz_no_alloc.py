@@ -71,6 +71,17 @@ def test_noalloc_entry_matches_tracea_conv2d_and_the_oracle_on_two_calls_in_a_ro
     assert ffi.load().tracea_b200_device_status(0) == 0
 
 
+@pytest.mark.parametrize("C,hw", [(24, (512, 512)), (40, (400, 500)), (40, (250, 300))])
+def test_noalloc_entry_takes_every_copy_that_fits_its_scratch_without_row_padding(C, hw):
+    """48- and 80-byte rows are padded to 64 and 96 bytes where there is room: 12.6 MB of copies that would be 16.8, 16.0 that
+    would be 19.2 (both over the 16 MiB there are), and 6.0 that may be 7.2."""
+    x = torch.randn((1, C) + hw, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((8, C, 1, 1), device="cuda") * 0.1).to(torch.bfloat16)
+    outs = [_call(e, x, w, None, None, torch.empty((1, 8) + hw, dtype=torch.bfloat16, device="cuda"), 1, 0,
+                  ffi.EPILOGUE_IDENTITY) for e in ("tracea_conv2d", "tracea_conv2d_noalloc")]
+    assert torch.equal(outs[0], outs[1])
+
+
 def test_noalloc_entry_takes_no_memory_from_the_device_or_the_pool():
     """Steady state (the kernels of this shape have run once, so the driver has loaded them): across a call
     the device's free memory does not move and the library's scratch pool hands nothing out."""

@@ -1142,7 +1142,9 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   const bool stage_x = !window && (!x_direct || knobs().force_staging);
   // Rows of a staged operand start on 32-byte boundaries: the TMA unit fetches whole 32-byte sectors, and rows 16 bytes off
   // cost it nearly twice the time (3x3 C->128 on 32 images of 28x28: C = 104 25.1 us, C = 112 13.9).
-  const long long Cs = Cp * es > 16 ? (Cp * es + 31) / 32 * 32 / es : Cp;
+  long long Cs = Cp * es > 16 ? (Cp * es + 31) / 32 * 32 / es : Cp;
+  // (the built-in scratch of the no-alloc entry is small: there the padding is left out when only that makes the copies fit)
+  if (arena != nullptr && arena->used + (N * H * W + K * R * S) * Cs * es + 1024 > static_cast<long long>(arena->capacity)) Cs = Cp;
   if (stage_x) {   // its address is filled in below, where the weights' form is known too
     x.stride[0] = H * W * Cs;
     x.stride[1] = 1;
