@@ -7,6 +7,8 @@ The oracle is fed the inputs already rounded to the storage type, accumulates in
 to the storage type once at the end, like the kernel's single rounding after the epilogue.
 """
 import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -66,6 +68,15 @@ def check(x, w, b, res, stride, padding, dilation, epi, dtype, **kw):
     err = cc.rel_err(got, want)
     assert err <= cc.tol_for(dtype), "rel err %.3g" % err
     return got, want
+
+
+def run_child(script, ok, **env):
+    """Runs `script` (argv[1]: the repository's root) in a process of its own with more environment: the library reads its
+    knobs once per process."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", script, root], env=dict(os.environ, **env), capture_output=True, text=True,
+                         timeout=600)
+    assert res.returncode == 0 and ok in res.stdout, res.stdout[-2000:] + res.stderr[-2000:]
 
 
 # --------------------------------------------------------------------------- golden fixtures
@@ -545,6 +556,29 @@ def test_ragged_channel_counts(c_bytes, r, s, stride, dtype):
     # padding pixels are zeros: 0 * inf is NaN where the tap lies outside the image, inf where it does not
     assert np.isposinf(got[:, 5][reached]).all() and np.isnan(got[:, 5][~reached]).all()
     assert np.isfinite(np.delete(got, 5, axis=1)).all()
+
+
+_FORCED_CHUNK_SCRIPT = r"""
+import sys
+sys.path.insert(0, sys.argv[1]); sys.path.insert(0, sys.argv[1] + "/tests")
+import convcases as cc
+import test_conv2d_gpu as t
+for dtype, es in (("bf16", 2), ("f32", 4)):
+    for c_bytes in (48, 80, 96, 208):      # copied taps are padded to 64, 96, 96 and 224 bytes
+        C = c_bytes // es
+        x = cc.uniform((2, C, 9, 11), 24, "fc/x", 0.1, 1.0)
+        w, b = cc.kaiming((72, C, 3, 3), 24, "fc/w"), cc.normal((72,), 24, "fc/b", 0.1)
+        for channels_last in (True, False):    # filters read in place, filters repacked
+            t.check(x, w, b, None, 1, 1, 1, "bias+relu", dtype, channels_last=channels_last, out_channels_last=True)
+print("forced chunk ok")
+"""
+
+
+@pytest.mark.parametrize("chunk", [16, 32, 64, 128])
+def test_every_forced_k_chunk_width_gives_the_same_convolution(chunk):
+    """TRACEA_B200_FORCE_CHUNK (read once per process, hence the child) with channel counts whose rows it divides and does not
+    divide, from filters that are read in place and from filters that are repacked with padded taps."""
+    run_child(_FORCED_CHUNK_SCRIPT, "forced chunk ok", TRACEA_B200_FORCE_CHUNK=str(chunk))
 
 
 # --------------------------------------------------------------------------- outputs that are not 16-byte aligned rows

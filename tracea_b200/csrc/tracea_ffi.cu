@@ -1162,9 +1162,12 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   if (forced_chunk == 16 || forced_chunk == 32 || forced_chunk == 64 || forced_chunk == 128) chunk_bytes = forced_chunk;
   const int chunk_elems = chunk_bytes / es;
   const int chunks_per_tap = static_cast<int>((Cg + chunk_elems - 1) / chunk_elems);
-  // the last chunk of a tap is partly past the channels: fine for the activations (the TMA unit fills channels >= C with
-  // zeros), but the weights then need a map with one row per tap, unless there is only one tap
-  const bool ragged_taps = row_bytes % chunk_bytes != 0 && R * Sg > 1;
+  const bool w_dense = C == Cp && (w_in.stride[1] == 1) && w_in.stride[3] == C &&
+                       w_in.stride[2] == S * C && w_in.stride[0] == R * S * C && aligned16(w_in.ptr);
+  // Where the last chunk of a tap is partly past the channels, the TMA unit fills the activations' channels >= C with zeros,
+  // but the weights need a map with one row per tap, unless there is only one tap. So do weights that are repacked with
+  // padded taps, whatever the chunk (chunks that divide an unpadded tap then only come from TRACEA_B200_FORCE_CHUNK).
+  const bool ragged_taps = (row_bytes % chunk_bytes != 0 || (!w_dense && !window && Cs != Cp)) && R * Sg > 1;
   const long long total_chunks_ll = R * Sg * chunks_per_tap;
   if (total_chunks_ll > 0x7fffffffLL / 128) TB_FAIL(TRACEA_UNSUPPORTED_CONFIG, "R*S*C too large");
 
@@ -1176,8 +1179,6 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   const void* w_ptr = w_in.ptr;
   Scratch op_scratch;
   long long w_row_elems = R * S * C, w_pitch = R * S * C, b_k0 = 0, b_jump_s = 0, b_jump_r = 0;
-  const bool w_dense = C == Cp && (w_in.stride[1] == 1) && w_in.stride[3] == C &&
-                       w_in.stride[2] == S * C && w_in.stride[0] == R * S * C && aligned16(w_in.ptr);
   bool w_direct = w_dense, w_remap = false;
   if (!w_dense && !window && C == Cp && w_in.stride[1] == 1 && chunk_bytes == 128 && !ragged_taps) {
     const long long ss = S == 1 ? C : w_in.stride[3], sr = R == 1 ? S * ss : w_in.stride[2], sk = w_in.stride[0];
