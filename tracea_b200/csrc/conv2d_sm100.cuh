@@ -101,16 +101,17 @@ struct ConvKernelArgs {
   // channels-last (sc == 1) and NCHW (sw == 1) memory are written without a transpose pass.
   void* out;
   long long out_sn, out_sh, out_sw, out_sc;
-  int out_vec;            // kStoreRows: bytes a lane may store at once (16, 4, or one element)
-  int out_quad;           // kStoreStrided: four consecutive pixels are always 8 consecutive, aligned bytes (16-bit types)
-  // small-tile kernel: output and residual are channel-contiguous; A's / B's map is {column in chunk, row, chunk} and one
-  // copy brings in two k-steps; the weights are the caller's, worth an early prefetch
-  int out_rows, a_steps2, b_steps2, b_prefetch;
+  int out_vec;            // kStoreRows, kStoreMixed: bytes a lane may store at once (16, 4, or one element)
+  int out_quad;           // kStoreStrided, kStoreMixed: four consecutive pixels are always 8 consecutive, aligned bytes (16-bit types)
+  int out_rows;           // kStoreMixed: the output is channel-contiguous; small-tile kernel: and so is the residual
+  // small-tile kernel: A's / B's map is {column in chunk, row, chunk} and one copy brings in two k-steps; the weights are the
+  // caller's, worth an early prefetch
+  int a_steps2, b_steps2, b_prefetch;
   const void* bias;       // [K_out], fp32 or OutT
   int bias_is_f32;
   const void* residual;   // same dtype as out
   long long res_sn, res_sh, res_sw, res_sc;
-  int res_vec;            // as out_vec, for the residual
+  int res_vec;            // as out_vec, for the residual; 0: its channels are not contiguous
   int act;
   // error reporting: 4 words {code, block, detail, 0}; first error wins
   uint32_t* status;
@@ -311,6 +312,9 @@ enum : int {
   kStoreTma = 0,      // dense [M][pitch] rows: staging boxes, moved by the TMA unit
   kStoreRows = 1,     // channel-contiguous, any pixel strides: the same boxes, moved by the warp itself
   kStoreStrided = 2,  // anything else, NCHW above all: each lane stores its own pixel's channels
+  kStoreMixed = 3,    // output and residual in different memory formats: the residual comes in through the boxes, the output
+                      // leaves by rows or by lanes (args.out_rows)
+  kNumStores = 4,
 };
 
 // Strided outputs: finishes one 32-column block of one pixel per lane -- residual, activation, store. `f` holds
@@ -369,7 +373,7 @@ __device__ __forceinline__ void store_strided32(const ConvKernelArgs& args, floa
 // chunk l & 7 of rows (l >> 3) + 4 i, so each instruction covers four whole 128-byte rows. `row_base` points at the
 // first element of the group's columns in pixel 0's row; `row_off` is this lane's own pixel offset (in elements),
 // `row_ok` whether its pixel exists; `cols_left` = K_out - first column of the group. Only instantiated in
-// the kStoreRows kernels.
+// the kStoreRows and kStoreMixed kernels.
 template <typename OutT>
 __device__ __noinline__ void coop_store_box(uint32_t stg, OutT* row_base, long long row_off, bool row_ok, int cols_left,
                                             int lane) {
@@ -449,6 +453,22 @@ __device__ __noinline__ void coop_load_box_narrow(uint32_t stg, const OutT* row_
     }
   }
   __syncwarp();
+}
+
+// A residual whose channels are not contiguous (an NCHW one beside a channels-last output): each lane fills its own row of the
+// box from its own pixel, so that an instruction reads one channel of 32 pixels. `px`: the group's first column of the pixel.
+template <typename OutT>
+__device__ __noinline__ void strided_load_box(uint32_t stg, const OutT* px, long long sc, bool row_ok, int cols_left, int lane) {
+  constexpr int kVec = 16 / sizeof(OutT);
+#pragma unroll 4
+  for (int c = 0; c < 8; ++c) {
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    OutT* e = reinterpret_cast<OutT*>(&v);
+#pragma unroll
+    for (int j = 0; j < kVec; ++j)
+      if (row_ok && c * kVec + j < cols_left) e[j] = px[(c * kVec + j) * sc];
+    ptx::st_shared_v4(stg + static_cast<uint32_t>(lane) * 128u + ((static_cast<uint32_t>(c) ^ (static_cast<uint32_t>(lane) & 7u)) << 4), v);
+  }
 }
 
 // `vec`: bytes per access that all rows allow -- 16, 4, or one element (ConvKernelArgs::out_vec / res_vec).
@@ -1371,6 +1391,10 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
         }
         if constexpr (kStore == kStoreRows) {
           if (res != nullptr) load_rows<OutT>(args.res_vec, stg, res + n0, res_off, row_ok, args.K_out - n0, lane);
+        } else if constexpr (kStore == kStoreMixed) {
+          __syncwarp();   // every lane has read the group before this one out of the box
+          if (args.res_vec != 0) load_rows<OutT>(args.res_vec, stg, res + n0, res_off, row_ok, args.K_out - n0, lane);
+          else strided_load_box<OutT>(stg, res + res_off + n0 * args.res_sc, args.res_sc, row_ok, args.K_out - n0, lane);
         }
 
         TB200_PROF_T(tm);
@@ -1401,6 +1425,15 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               rchunks[c] = ld_shared_v4(stg + lane_row_off + ((cc ^ lane_xor) << 4));
             }
           }
+          if constexpr (kStore == kStoreMixed) {
+            if (!args.out_rows) {
+              const int n_first = n0 + h * 32;
+#pragma unroll
+              for (int c = 0; c < kChunksPerLd; ++c) add16<OutT>(f + c * kVec, rchunks[c]);
+              store_strided32<OutT>(args, f, nullptr, out + out_off + n_first * args.out_sc, args.K_out - n_first, row_ok, lane);
+              continue;
+            }
+          }
           if (args.act == kActRelu) {
             finish32<OutT, true>(f, rchunks, res_staged, packed + h * kChunksPerLd);
           } else {
@@ -1426,7 +1459,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
             bulk_commit_group();
           }
           box ^= 1u;
-        } else if constexpr (kStore == kStoreRows) {
+        } else if (kStore == kStoreRows || (kStore == kStoreMixed && args.out_rows)) {
 #pragma unroll
           for (int c = 0; c < 8; ++c)
             st_shared_v4(stg + lane_row_off + ((static_cast<uint32_t>(c) ^ lane_xor) << 4), packed[c]);

@@ -106,9 +106,9 @@ DeviceState g_dev[kMaxDevices];
 std::atomic<long long> g_test_wait_limit{0};
 std::atomic<int> g_test_producer_stop{-1};
 // "opt-in shared memory size has been set for this kernel variant on this device":
-// [device][dtype][bn index][tiling: single CTA / CTA pair / two row blocks; x4: the three store forms, K-split].
+// [device][dtype][bn index][tiling: single CTA / CTA pair / two row blocks; x5: the store forms, K-split].
 // Setting the attribute twice is harmless, so a relaxed flag is enough.
-std::atomic<bool> g_attr_set[kMaxDevices][3][3][12];
+std::atomic<bool> g_attr_set[kMaxDevices][3][3][3 * (tb200::kNumStores + 1)];
 std::atomic<unsigned long long> g_kernel_launches{0};   // every kernel this library has launched (conv + layout adapters)
 // the same, by kind: 0 general implicit-GEMM kernel, 1 its K-split instantiations, 2 resident-filter kernel, 3 layout adapters
 std::atomic<unsigned long long> g_launches_by_kind[5];
@@ -403,7 +403,7 @@ void launch_one_variant(DeviceState& st, int dt_idx, int bn_idx, const CUtensorM
                 const CUtensorMap& to, const CUtensorMap& tr, const ConvKernelArgs& args, int grid, int smem,
                 cudaStream_t stream) {
   auto kern = tb200::conv2d_igemm_sm100_kernel<OutT, BN, kPair, kRows2, kStore, kSplit>;
-  constexpr int kVariant = (kPair ? 1 : (kRows2 ? 2 : 0)) + 3 * (kSplit ? 3 : kStore);
+  constexpr int kVariant = (kPair ? 1 : (kRows2 ? 2 : 0)) + 3 * (kSplit ? tb200::kNumStores : kStore);
   std::atomic<bool>& attr_done = g_attr_set[st.dev][dt_idx][bn_idx][kVariant];
   if (!attr_done.load(std::memory_order_relaxed)) {
     TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
@@ -513,6 +513,9 @@ void launch_bn(DeviceState& st, int dt_idx, int bn, bool pair, bool rows2, int s
       break;
     case tb200::kStoreRows:
       launch_tiling<OutT, tb200::kStoreRows>(st, dt_idx, bn, pair, rows2, tx, tw, to, tr, args, grid, smem, stream);
+      break;
+    case tb200::kStoreMixed:
+      launch_tiling<OutT, tb200::kStoreMixed>(st, dt_idx, bn, pair, rows2, tx, tw, to, tr, args, grid, smem, stream);
       break;
     default:
       launch_tiling<OutT, tb200::kStoreStrided>(st, dt_idx, bn, pair, rows2, tx, tw, to, tr, args, grid, smem, stream);
@@ -1397,6 +1400,10 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   // else -- NCHW, or so few channels that a row is a fraction of a sector -- is stored pixel by pixel, each lane its own.
   // (2048 x 2047 x 1024 product, bf16: two-byte rows 13.1 us, per-lane stores 68.4, 16-byte boxes on 2048 columns 11.3.
   // Between 3 and 5 channels rows and per-lane stores cost the same.)
+  // A residual in another memory format than the output has a form of its own, so that neither side's accesses are narrowed to
+  // what the other allows (3x3 256->256 on 64 images of 14x14, bf16: channels-last output with an NCHW residual 63.4 us pixel
+  // by pixel, 24.9 so; NCHW output with a channels-last residual 35.6, 22.1; NCHW residuals beside the other forms cost
+  // those 3 % in registers. Single-element rows gain nothing: 50 -> 41 channels 9.0 either way.)
   const View4* res_v = epi.residual ? residual : nullptr;
   auto row_vec = [&](const View4& v) -> int {   // bytes per access of a channel-contiguous tensor's rows
     auto ok = [&](long long bytes) {
@@ -1418,9 +1425,9 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     if (r != CUDA_SUCCESS) TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled (%s) failed with %d", what, (int)r);
   };
   int store = tb200::kStoreStrided;
-  if (out.stride[1] == 1 && (res_v == nullptr || res_v->stride[1] == 1)) {
+  a.res_vec = res_v != nullptr && res_v->stride[1] == 1 ? row_vec(*res_v) : 0;
+  if (out.stride[1] == 1) {
     a.out_vec = row_vec(out);
-    a.res_vec = res_v != nullptr ? row_vec(*res_v) : 0;
     if (a.out_vec == 16 && rows_linear(out) && knobs().no_tma_store == 0 &&
         (res_v == nullptr || (a.res_vec == 16 && rows_linear(*res_v) && knobs().no_tma_residual == 0)))
       store = tb200::kStoreTma;
@@ -1428,11 +1435,13 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
       store = tb200::kStoreRows;
   }
   a.out_rows = store != tb200::kStoreStrided;
+  if (res_v != nullptr && (store == tb200::kStoreRows ? a.res_vec == 0 : (out.stride[1] != 1 && a.res_vec >= 4)))
+    store = tb200::kStoreMixed;
   if (store == tb200::kStoreTma && small_bn == 0) {
     encode_rows(&tmap_out, out, CU_TENSOR_MAP_L2_PROMOTION_NONE, "out");
     if (res_v != nullptr) encode_rows(&tmap_res, *res_v, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, "residual");
   }
-  a.out_quad = store == tb200::kStoreStrided && es == 2 && out.stride[3] == 1 && out.stride[2] == Wo &&
+  a.out_quad = !a.out_rows && es == 2 && out.stride[3] == 1 && out.stride[2] == Wo &&
                (Ho * Wo) % 4 == 0 && out.stride[0] % 4 == 0 && out.stride[1] % 4 == 0 &&
                reinterpret_cast<uintptr_t>(out.ptr) % 8 == 0;
   if (epi.bias && bias != nullptr) {
@@ -1622,6 +1631,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     CUtensorMap tmap_w;
     encode_w(&tmap_w, small_bn);
     a.M = static_cast<int>(M);
+    if (store == tb200::kStoreMixed) a.out_rows = 0;   // that kernel's row form takes a residual in rows only
     a.num_n_tiles = static_cast<int>(tiles_n);
     const long long stages_needed = (total_chunks_ll + 1) / 2;   // two 128-byte k-steps each
     a.num_stages = static_cast<int>(std::min<long long>(tb200::small_stages(small_bn), stages_needed));
