@@ -724,31 +724,39 @@ def test_filters_are_repacked_exactly(K, C, R, S, dtype):
 
 # --------------------------------------------------------------------------- tiles split over K (opt-in schedule)
 _SPLIT_K_SCRIPT = r"""
-import sys
+import os, sys
 import numpy as np, torch
 sys.path.insert(0, sys.argv[1]); sys.path.insert(0, sys.argv[1] + "/tests")
 import convcases as cc
 from oracle import oracle
 from tracea_b200 import ffi, ops
-cl = lambda t: t.contiguous(memory_format=torch.channels_last)
-dev = lambda a: cl(torch.from_numpy(np.ascontiguousarray(a)).to(torch.bfloat16).cuda())
-# N, C, H, K, R, pad, epilogue: more than one wave with a partial last wave (two pieces per split tile, CTA pairs and
+dev = lambda a, fmt=torch.channels_last: torch.from_numpy(np.ascontiguousarray(a)).to(torch.bfloat16).cuda().contiguous(memory_format=fmt)
+# N, C, H, K, R, pad, epilogue [, form]: more than one wave with a partial last wave (two pieces per split tile, CTA pairs and
 # single CTAs), and fewer tiles than SMs (three and more pieces per tile, two-row-block tiles)
 CASES = [(256, 256, 14, 256, 3, 1, "bias+relu"), (200, 1024, 14, 256, 1, 0, "bias+residual+relu"),
          (64, 512, 7, 512, 3, 1, "bias+relu"), (16, 2048, 7, 512, 1, 0, "bias+silu"), (40, 512, 14, 128, 3, 1, "relu"),
          (150, 256, 14, 1024, 1, 0, "bias+residual+relu"), (3, 64, 56, 64, 3, 1, "bias+relu"),
-         (8, 256, 56, 64, 3, 1, "bias+residual+relu")]   # two-row-block tiles cut in two or three: both groups finish a tile
-for N, C, H, K, R, pad, epi in CASES:
+         (8, 256, 56, 64, 3, 1, "bias+residual+relu"),   # two-row-block tiles cut in two or three: both groups finish a tile
+         # outputs that the TMA unit does not store: NCHW, rows of odd length, formats that differ
+         (200, 1024, 14, 256, 1, 0, "bias+residual+relu", "nchw"), (64, 512, 7, 512, 3, 1, "bias+relu", "nchw"),
+         (40, 512, 14, 128, 3, 1, "relu", "nchw"), (64, 512, 7, 509, 3, 1, "bias+residual+relu", "nhwc"),
+         (64, 512, 7, 512, 3, 1, "bias+residual+relu", "mixed")]
+for N, C, H, K, R, pad, epi, *form in CASES:
+    out_last, res_fmt = form != ["nchw"], torch.channels_last if form in ([], ["nhwc"]) else torch.contiguous_format
     x = np.abs(cc.normal((N, C, H, H), 3, "sk/x")); w = cc.kaiming((K, C, R, R), 3, "sk/w")
     b = cc.normal((K,), 3, "sk/b", 0.05); r = cc.normal((N, K, H, H), 3, "sk/r")
     ub, ur = "bias" in epi, "residual" in epi
     act = next((o for o in epi.split("+") if o in ("relu", "silu")), "none")
     outs = []
+    before = ffi.launch_count_of(ffi.KERNEL_SPLIT_K)
     for rep in range(2):   # twice: the second launch finds the counters the first one left behind
-        got = ops.conv2d_nchw(dev(x), dev(w), torch.from_numpy(b).cuda() if ub else None, dev(r) if ur else None,
-                              1, pad, 1, 1, epi)
+        got = ops.conv2d_nchw(dev(x), dev(w), torch.from_numpy(b).cuda() if ub else None, dev(r, res_fmt) if ur else None,
+                              1, pad, 1, 1, epi, channels_last_out=out_last)
         torch.cuda.synchronize()
         outs.append(got)
+    # level 1 leaves tiles whole where cutting them would save fewer than four k-steps (eight within one wave)
+    split = 2 if os.environ["TRACEA_B200_SPLIT_K"] == "2" or C * R * R >= 1024 else 0
+    assert ffi.launch_count_of(ffi.KERNEL_SPLIT_K) == before + split, ("split launches", N, C, H, K, R, form)
     assert torch.equal(outs[0], outs[1]), "not reproducible"
     want = oracle.conv2d_gemm(cc.channels_last(cc.round_to(x, "bf16")), cc.round_to(w, "bf16"), b if ub else None,
                               cc.channels_last(cc.round_to(r, "bf16")) if ur else None, 1, pad, 1, act)
@@ -759,18 +767,13 @@ print("split-k ok")
 """
 
 
-def test_tiles_split_over_k_match_the_oracle_and_repeat_bit_for_bit():
-    """The K-split schedule is off by default (TRACEA_B200_SPLIT_K=1 turns it on, read once per process), so it is
+@pytest.mark.parametrize("level", ["1", "2"])
+def test_tiles_split_over_k_match_the_oracle_and_repeat_bit_for_bit(level):
+    """The K-split schedule is off by default (TRACEA_B200_SPLIT_K=1 or 2 turns it on, read once per process), so it is
     exercised in a child process: ResNet-sized layers whose last wave is partly filled or that have fewer tiles
     than SMs, against the oracle, each launched twice with identical bits (the pieces are summed in piece order
-    whichever of them finishes last)."""
-    import subprocess
-    import sys
-    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    env = dict(os.environ, TRACEA_B200_SPLIT_K="1")
-    res = subprocess.run([sys.executable, "-c", _SPLIT_K_SCRIPT, root], env=env, capture_output=True, text=True,
-                         timeout=600)
-    assert res.returncode == 0 and "split-k ok" in res.stdout, res.stdout[-2000:] + res.stderr[-2000:]
+    whichever of them finishes last). The launch counter shows which layers were cut."""
+    run_child(_SPLIT_K_SCRIPT, "split-k ok", TRACEA_B200_SPLIT_K=level)
 
 
 # --------------------------------------------------------------------------- resident-filter kernel (stride-1 small filters, C = 64)

@@ -106,9 +106,9 @@ DeviceState g_dev[kMaxDevices];
 std::atomic<long long> g_test_wait_limit{0};
 std::atomic<int> g_test_producer_stop{-1};
 // "opt-in shared memory size has been set for this kernel variant on this device":
-// [device][dtype][bn index][tiling: single CTA / CTA pair / two row blocks; x5: the store forms, K-split].
+// [device][dtype][bn index][tiling: single CTA / CTA pair / two row blocks; x6: the store forms, K-split by TMA and by lanes].
 // Setting the attribute twice is harmless, so a relaxed flag is enough.
-std::atomic<bool> g_attr_set[kMaxDevices][3][3][3 * (tb200::kNumStores + 1)];
+std::atomic<bool> g_attr_set[kMaxDevices][3][3][3 * (tb200::kNumStores + 2)];
 std::atomic<unsigned long long> g_kernel_launches{0};   // every kernel this library has launched (conv + layout adapters)
 // the same, by kind: 0 general implicit-GEMM kernel, 1 its K-split instantiations, 2 resident-filter kernel, 3 layout adapters
 std::atomic<unsigned long long> g_launches_by_kind[5];
@@ -403,7 +403,7 @@ void launch_one_variant(DeviceState& st, int dt_idx, int bn_idx, const CUtensorM
                 const CUtensorMap& to, const CUtensorMap& tr, const ConvKernelArgs& args, int grid, int smem,
                 cudaStream_t stream) {
   auto kern = tb200::conv2d_igemm_sm100_kernel<OutT, BN, kPair, kRows2, kStore, kSplit>;
-  constexpr int kVariant = (kPair ? 1 : (kRows2 ? 2 : 0)) + 3 * (kSplit ? tb200::kNumStores : kStore);
+  constexpr int kVariant = (kPair ? 1 : (kRows2 ? 2 : 0)) + 3 * (kSplit ? tb200::kNumStores + (kStore == tb200::kStoreTma ? 0 : 1) : kStore);
   std::atomic<bool>& attr_done = g_attr_set[st.dev][dt_idx][bn_idx][kVariant];
   if (!attr_done.load(std::memory_order_relaxed)) {
     TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
@@ -439,12 +439,12 @@ void launch_one_variant(DeviceState& st, int dt_idx, int bn_idx, const CUtensorM
   g_launches_by_kind[kSplit ? 1 : 0].fetch_add(1, std::memory_order_relaxed);
 }
 
-// The K-split kernels exist for the TMA epilogue only (the host splits no other launch).
+// The K-split kernels exist for the TMA epilogue and for per-lane stores (the host splits no other launch).
 template <typename OutT, int BN, bool kPair, bool kRows2, int kStore>
 void launch_one(DeviceState& st, int dt_idx, int bn_idx, const CUtensorMap& tx, const CUtensorMap& tw,
                 const CUtensorMap& to, const CUtensorMap& tr, const ConvKernelArgs& args, int grid, int smem,
                 cudaStream_t stream) {
-  if constexpr (kStore == tb200::kStoreTma) {
+  if constexpr (kStore == tb200::kStoreTma || kStore == tb200::kStoreStrided) {
     if (args.sk_tiles > 0) {
       launch_one_variant<OutT, BN, kPair, kRows2, kStore, true>(st, dt_idx, bn_idx, tx, tw, to, tr, args, grid, smem, stream);
       return;
@@ -1434,8 +1434,12 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     else if (K > 4 || a.out_vec == 16)
       store = tb200::kStoreRows;
   }
+  // with the K-split option on, narrow rows and mixed formats go by lanes too: there are no K-split kernels for more forms
+  const bool split_on = knobs().split_k != 0;
+  if (split_on && store == tb200::kStoreRows && (a.out_vec != 16 || (res_v != nullptr && a.res_vec != 16)))
+    store = tb200::kStoreStrided;
   a.out_rows = store != tb200::kStoreStrided;
-  if (res_v != nullptr && (store == tb200::kStoreRows ? a.res_vec == 0 : (out.stride[1] != 1 && a.res_vec >= 4)))
+  if (res_v != nullptr && !split_on && (store == tb200::kStoreRows ? a.res_vec == 0 : (out.stride[1] != 1 && a.res_vec >= 4)))
     store = tb200::kStoreMixed;
   if (store == tb200::kStoreTma && small_bn == 0) {
     encode_rows(&tmap_out, out, CU_TENSOR_MAP_L2_PROMOTION_NONE, "out");
@@ -1559,7 +1563,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     Scratch sk_scratch;
     const long long k_iters = total_chunks_ll;   // 128-byte chunks: one per pipeline stage
     const int split_env = knobs().split_k;
-    if (chunk_bytes == 128 && !a_tiled && store == tb200::kStoreTma && split_env != 0 && arena == nullptr && k_iters >= 2 &&
+    if (chunk_bytes == 128 && !a_tiled && (store == tb200::kStoreTma || store == tb200::kStoreStrided) && split_env != 0 && arena == nullptr && k_iters >= 2 &&
         2 * workers_max * k_iters < (1LL << 30)) {
       const long long rem = tiles % workers_max;       // tiles of the last, partly filled wave (all of them if < 1 wave)
       if (rem > 0) {
