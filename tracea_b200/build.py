@@ -1,10 +1,13 @@
-"""Ahead-of-time build of libtracea_b200.so (nvcc, sm_100a only) and of its tensor front end for Python, _ops_native.so
-(host compiler, against torch's headers). Cross-compiles without a GPU.
+"""Ahead-of-time build of libtracea_b200.so (nvcc, sm_100a only) and of its tensor front end for Python, the extension module
+_ops_native (host compiler, against torch's headers). Cross-compiles without a GPU. The library needs nothing of Python or
+torch: without torch, or with ``--library-only``, it is all that is built.
 
 This replaces the reference's run-time path NVRTC -> PTX -> cuModuleLoadData
 (src/runtime/manager/kernel.rs:123-327): there is no code generation at run time here.
 """
+import importlib.util
 import os
+import runpy
 import subprocess
 import sys
 import sysconfig
@@ -21,7 +24,10 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-shared", "-cudart", "static",
 ]
 
-NATIVE = os.path.join(HERE, "_ops_native.so")
+# The front end fits one interpreter and one build of torch: the first is in its name, the second in the stamp beside it.
+NATIVE = os.path.join(HERE, "_ops_native" + sysconfig.get_config_var("EXT_SUFFIX"))
+NATIVE_STAMP = os.path.join(HERE, "_ops_native.stamp")
+UNTAGGED_NATIVE = os.path.join(HERE, "_ops_native.so")   # a name that every interpreter would import
 NATIVE_SOURCES = [os.path.join(CSRC, "py_ops.cpp")]
 NATIVE_HEADERS = [os.path.join(HERE, "..", "include", "tracea_b200.h")]
 
@@ -33,8 +39,28 @@ def _stale(target, sources):
     return any(os.path.getmtime(p) > t for p in sources)
 
 
+def _torch_build():
+    """What the front end has to fit, as the text of its stamp: the interpreter's suffix, torch's version and the commit it
+    was built from. None without torch. (Read from torch/version.py: importing torch takes seconds.)"""
+    spec = importlib.util.find_spec("torch")
+    if spec is None or not spec.submodule_search_locations:
+        return None
+    version = runpy.run_path(os.path.join(spec.submodule_search_locations[0], "version.py"))
+    return "%s torch %s %s\n" % (sysconfig.get_config_var("EXT_SUFFIX"), version["__version__"], version["git_version"])
+
+
+def _native_stale():
+    fits = _torch_build()
+    if fits is None:
+        return False
+    if os.path.exists(UNTAGGED_NATIVE) or not os.path.exists(NATIVE_STAMP):
+        return True
+    with open(NATIVE_STAMP) as f:
+        return f.read() != fits or _stale(NATIVE, NATIVE_SOURCES + NATIVE_HEADERS)
+
+
 def needs_build():
-    return _stale(LIB, SOURCES + HEADERS) or _stale(NATIVE, NATIVE_SOURCES + NATIVE_HEADERS)
+    return _stale(LIB, SOURCES + HEADERS) or _native_stale()
 
 
 def _run(cmd, what):
@@ -55,19 +81,24 @@ def _build_native():
           "-isystem", os.path.join(cuda, "include")] + NATIVE_SOURCES +
          ["-o", NATIVE, "-L" + HERE, "-l:" + os.path.basename(LIB), "-L" + os.path.join(root, "lib"),
           "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"], "c++")
+    with open(NATIVE_STAMP, "w") as f:
+        f.write(_torch_build())
+    if os.path.exists(UNTAGGED_NATIVE):
+        os.remove(UNTAGGED_NATIVE)
 
 
-def build(force=False, verbose=False):
-    """Compile what is missing or older than its sources, in-tree."""
+def build(force=False, verbose=False, library_only=False):
+    """Compile what is missing, older than its sources or made for another interpreter or torch, in-tree. The library alone if
+    asked to, or where there is no torch."""
     if force or _stale(LIB, SOURCES + HEADERS):
         nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
         res = _run([nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB] + SOURCES, "nvcc")
         if verbose:
             sys.stderr.write(res.stderr)
-    if force or _stale(NATIVE, NATIVE_SOURCES + NATIVE_HEADERS):
+    if not library_only and _torch_build() is not None and (force or _native_stale()):
         _build_native()
     return LIB
 
 
 if __name__ == "__main__":
-    print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build(force="--force" in sys.argv, verbose="-v" in sys.argv, library_only="--library-only" in sys.argv))

@@ -9,6 +9,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include "../../include/tracea_b200.h"
 
@@ -221,4 +222,11 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_ops_native", nullptr, -1, kMetho
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__ops_native() { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__ops_native() {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) < 0) {   // what it was compiled against
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

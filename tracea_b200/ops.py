@@ -29,11 +29,15 @@ _native_module = None
 
 
 def _native():
-    """The tensor front end of the library, loaded with it on first use (raises if either has not been built)."""
+    """The tensor front end of the library, loaded with it on first use (raises if either has not been built, or the front end
+    for another torch)."""
     global _native_module
     if _native_module is None:
         ffi.load()
         from . import _ops_native
+        if _ops_native.torch_version != torch.__version__.split("+")[0]:
+            raise ImportError("_ops_native was built for torch %s, this is torch %s: build it again with `python -m "
+                              "tracea_b200.build`" % (_ops_native.torch_version, torch.__version__))
         _native_module = _ops_native
     return _native_module
 
