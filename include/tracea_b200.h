@@ -269,13 +269,14 @@ void tracea_b200_test_hooks(int64_t wait_limit_cycles, int32_t producer_stop_aft
 int32_t tracea_b200_pool_stats(int32_t device_id, uint64_t stats[4], int32_t reset_high);
 
 /* Number of GPU kernels this library has launched in this process so far (conv kernels and layout adapters;
- * a call may launch more than one: a layout adapter per staged operand, one conv launch per phase of a transposed
- * convolution). Benchmarks read it before and after a timed region. No counterpart in the reference. */
+ * a call may launch more than one: a layout adapter for the operands that have to be copied, one conv launch per phase of
+ * a transposed convolution). Benchmarks read it before and after a timed region. No counterpart in the reference. */
 uint64_t tracea_b200_launch_count(void);
 
 /* The same count for one kind of kernel: 0 the general implicit-GEMM conv kernel, 1 its instantiations that cut tiles
  * over K, 2 the resident-filter kernel (stride-1 small filters over 64-channel activations), 3 layout adapters,
- * 4 the row-band kernel (few-channel 16-bit images such as the RGB stem).
+ * 4 the row-band kernel (few-channel 16-bit images such as the RGB stem), 5 the small-tile kernel (problems of up to one
+ * wave of 64-row tiles).
  * Lets tests and benchmarks see which path a call took. 0 for any other `kind`. No counterpart in the reference. */
 uint64_t tracea_b200_launch_count_of(int32_t kind);
 

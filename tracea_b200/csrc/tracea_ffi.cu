@@ -110,8 +110,10 @@ std::atomic<int> g_test_producer_stop{-1};
 // Setting the attribute twice is harmless, so a relaxed flag is enough.
 std::atomic<bool> g_attr_set[kMaxDevices][3][3][3 * (tb200::kNumStores + 2)];
 std::atomic<unsigned long long> g_kernel_launches{0};   // every kernel this library has launched (conv + layout adapters)
-// the same, by kind: 0 general implicit-GEMM kernel, 1 its K-split instantiations, 2 resident-filter kernel, 3 layout adapters
-std::atomic<unsigned long long> g_launches_by_kind[5];
+// the same, by kind: 0 general implicit-GEMM kernel, 1 its K-split instantiations, 2 resident-filter kernel, 3 layout adapters,
+// 4 row-band kernel, 5 small-tile kernel
+constexpr int kLaunchKinds = 6;
+std::atomic<unsigned long long> g_launches_by_kind[kLaunchKinds];
 EncodeTiledFn g_encode_tiled = nullptr;
 EncodeIm2colFn g_encode_im2col = nullptr;
 
@@ -500,7 +502,7 @@ void launch_small(DeviceState& st, int dt_idx, const CUtensorMap& tx, const CUte
   TB_CUDA(cudaLaunchKernelEx(&cfg, kern, tx, tw, args));
   TB_CUDA(cudaGetLastError());
   g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-  g_launches_by_kind[0].fetch_add(1, std::memory_order_relaxed);
+  g_launches_by_kind[5].fetch_add(1, std::memory_order_relaxed);
 }
 
 template <typename OutT>
@@ -2382,7 +2384,7 @@ void tracea_b200_test_hooks(int64_t wait_limit_cycles, int32_t producer_stop_aft
 uint64_t tracea_b200_launch_count(void) { return g_kernel_launches.load(std::memory_order_relaxed); }
 
 uint64_t tracea_b200_launch_count_of(int32_t kind) {
-  if (kind < 0 || kind >= 5) return 0;
+  if (kind < 0 || kind >= kLaunchKinds) return 0;
   return g_launches_by_kind[kind].load(std::memory_order_relaxed);
 }
 
