@@ -1,7 +1,7 @@
 """The kernels' failure path, exercised without faulting, trapping or hanging anything: every wait inside them is
 bounded, and a wait that runs out makes its role record a code, the CTA unwind through its normal teardown (copies
 drained, TMEM freed) and the kernel return. The library's test hooks shorten the limit of a wait and make the TMA
-producer go silent after two pipeline stages, so the MMA issuer's wait for the third stage runs out.
+producer go silent after a few pipeline stages, so the MMA issuer's wait for the next one runs out.
 
 The reference has nothing to compare with: its kernels wait without limit (src/backend/cuda/primitives.rs:70-121).
 """
@@ -23,7 +23,11 @@ CASES = {
     "cta_pair": (8, 256, 14, 256, 3, 1, ffi.KERNEL_GENERAL, 1),           # 256 x 256 tiles over two SMs (cluster of 2)
     "resident_filter": (64, 64, 56, 64, 3, 1, ffi.KERNEL_RESIDENT_FILTER, 1),   # every CTA pair gets three windows or more
     "row_band": (48, 3, (56, 224), 64, 7, 3, ffi.KERNEL_ROW_BAND, 2),     # RGB stem rows: every CTA gets four bands or more
+    "small_matrix": (1, 512, 14, 256, 1, 0, ffi.KERNEL_SMALL_TILE, 1),    # four stages of two k-steps, both operands in one copy
+    "small_im2col": (1, 64, 28, 128, 3, 1, ffi.KERNEL_SMALL_TILE, 1),     # five stages, the last half empty
+    "small_refilled": (1, 2048, 7, 512, 1, 0, ffi.KERNEL_SMALL_TILE, 1),  # 16 stages
 }
+STOP_AFTER = {"small_refilled": 6}   # stages the producer fills (2 otherwise): more than the small-tile kernel's ring of four
 
 
 def _tensors(name):
@@ -51,7 +55,7 @@ def test_a_wait_that_runs_out_is_reported_and_the_device_stays_usable(name):
     assert lib.tracea_b200_device_status(0) == 0
     before = ffi.launch_count_of(CASES[name][6])
     try:
-        lib.tracea_b200_test_hooks(400000, 2)                # ~0.2 ms per wait; producers stop after two stages
+        lib.tracea_b200_test_hooks(400000, STOP_AFTER.get(name, 2))   # ~0.2 ms per wait; producers stop after that many stages
         ops.conv2d_nchw(tx, tw, tb, None, stride, pad, 1, 1, "bias+relu")   # the launch itself succeeds: the call is asynchronous
         torch.cuda.synchronize()                             # and the kernel ends by itself
     finally:
