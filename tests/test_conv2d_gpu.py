@@ -722,6 +722,59 @@ def test_filters_are_repacked_exactly(K, C, R, S, dtype):
         assert torch.equal(packed[:, :C], w) and bool((packed[:, C:] == 0).all())
 
 
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("N,C,H,K,R", [(1, 64, 28, 64, 3), (1, 20, 31, 50, 5), (40, 72, 14, 130, 3)])
+def test_calls_with_layout_adapters_are_captured_and_replayed(N, C, H, K, R, dtype):
+    """NCHW operands: the adapter's programmatic launch sits between a pool allocation and the convolution. Captured with three
+    convolutions in a row (each reads the scratch of the one before it, freed and taken again), replayed on new inputs."""
+    rnd = lambda *s: torch.randn(s, device="cuda").to(TORCH_DT[dtype])
+    x, w, b = rnd(N, C, H, H), rnd(K, C, R, R) * (C * R * R) ** -0.5, rnd(K).float()
+    call = lambda: [ops.conv2d_nchw(v, w, b, None, 1, R // 2, 1, 1, "bias+silu") for v in (x, x.flip(0), x.neg())]
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    before = ffi.launch_count_of(ffi.KERNEL_LAYOUT)
+    with torch.cuda.graph(graph):
+        outs = call()
+    assert ffi.launch_count_of(ffi.KERNEL_LAYOUT) == before + 3
+    for _ in range(3):
+        x.copy_(rnd(N, C, H, H))
+        w.copy_(rnd(K, C, R, R) * (C * R * R) ** -0.5)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(got, want) for got, want in zip(outs, call()))
+    assert ffi.load().tracea_b200_device_status(0) == 0
+
+
+_EVERY_TILING_SCRIPT = r"""
+import sys
+sys.path.insert(0, sys.argv[1]); sys.path.insert(0, sys.argv[1] + "/tests")
+import test_conv2d_gpu as t
+for dtype in ("bf16", "f32"):
+    for K in (1, 5, 18, 31, 66, 129, 258):
+        for channels_last in (True, False):
+            t.test_output_widths_in_both_memory_formats(K, channels_last, dtype)
+        t.test_output_and_residual_in_different_memory_formats(3, 6, 8, K, dtype)
+    for view in ((1, 40, 64), (2, 40, 66), (1, 41, 43), (8, 64, 72)):
+        t.test_unaligned_output_and_residual_views(*view, dtype)
+    for c_bytes in (80, 144, 272):
+        t.test_ragged_channel_counts(c_bytes, 3, 3, 1, dtype)
+        t.test_ragged_channel_counts(c_bytes, 2, 3, 2, dtype)
+assert t.ffi.launch_count_of(t.ffi.KERNEL_GENERAL) > 200 and t.ffi.launch_count_of(t.ffi.KERNEL_SMALL_TILE) == 0
+print("tilings ok")
+"""
+
+
+@pytest.mark.parametrize("knobs", [{"FORCE_BN": "64", "ROWS2": "0"}, {"FORCE_BN": "64", "ROWS2": "1"},
+                                   {"FORCE_BN": "128", "ROWS2": "0"}, {"FORCE_BN": "128", "ROWS2": "1"},
+                                   {"FORCE_BN": "256", "PAIR": "0"}, {"FORCE_BN": "256", "PAIR": "1"}],
+                         ids=lambda k: "-".join(k[0].lower() + v for k, v in k.items()))
+def test_odd_widths_in_every_tiling_of_the_general_kernel(knobs):
+    """Small layers take the small-tile kernel: in a child process that forces the general kernel's tilings, the forms of output
+    and the channel counts of the tests above reach each of them."""
+    run_child(_EVERY_TILING_SCRIPT, "tilings ok", **{"TRACEA_B200_" + k: v for k, v in knobs.items()})
+
+
 # --------------------------------------------------------------------------- tiles split over K (opt-in schedule)
 _SPLIT_K_SCRIPT = r"""
 import os, sys
