@@ -177,32 +177,9 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint
       : "memory");
 }
 
-// Tiled 3-D load: coordinates {c0 (innermost), c1, c2}.
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5}], [%2];"
-      :
-      : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-
-// im2col-mode 4-D load over an NHWC tensor: coordinates {c, w, h, n} give the first base pixel
-// (already including the negative padding corner), {off_w, off_h} the filter-tap offset.
-__device__ __forceinline__ void tma_load_im2col_4d(uint32_t dst, const void* tmap, uint32_t bar,
-                                                   int c, int w, int h, int n, uint16_t off_w,
-                                                   uint16_t off_h) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
-      :
-      : "r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n),
-        "h"(off_w), "h"(off_h)
-      : "memory");
-}
-
-// The same loads, executed by a whole converged warp with the same operands in every lane and predicated on `issue`, 1 in one
-// lane: see tma_stage_probe.
+// Loads for a whole converged warp with the same operands in every lane, predicated on `issue`, 1 in one lane: see
+// tma_stage_probe. Tiled loads take coordinates innermost first. The im2col load reads an NHWC tensor: coordinates
+// {c, w, h, n} give the first base pixel (already including the negative padding corner), {off_w, off_h} the filter-tap offset.
 __device__ __forceinline__ void mbar_arrive_expect_tx_if(uint32_t issue, uint32_t bar, uint32_t bytes) {
   asm volatile(
       "{\n"
@@ -244,17 +221,7 @@ __device__ __forceinline__ void tma_load_im2col_4d_if(uint32_t issue, uint32_t d
       : "memory");
 }
 
-// Same im2col box, but only pulled into L2 (no shared-memory destination, no barrier): used to run the
-// HBM fetch of the activations several k-steps ahead of the shared-memory ring.
-__device__ __forceinline__ void tma_prefetch_im2col_4d(const void* tmap, int c, int w, int h, int n, uint16_t off_w,
-                                                       uint16_t off_h) {
-  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.im2col [%0, {%1, %2, %3, %4}], {%5, %6};"
-               :
-               : "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h)
-               : "memory");
-}
-
-// A tiled 3-D box, likewise only pulled into L2.
+// A tiled 3-D box, only pulled into L2 (no shared-memory destination, no barrier).
 __device__ __forceinline__ void tma_prefetch_3d(const void* tmap, int c0, int c1, int c2) {
   asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
                :

@@ -363,7 +363,8 @@ const Knobs& knobs() {
 // than derived: the tensor pipe alone would give 512 / 256 / 192 cycles (BN/2 per MMA, 48 at BN = 64 where the
 // shared-memory operand reads bind), but the narrower tiles pull (128 + BN) * 128 bytes per step through L2 -> SM
 // paths that deliver ~70 B/cycle/SM when every SM loads, so a BN = 128 step costs ~400 and a BN = 64 step ~300.
-// The widest tile wins ties: it re-reads A least.
+// The widest tile wins ties: it re-reads A least. (Measured while one thread each issued the copies and the MMAs, at 420-505
+// cycles a stage; a stage issues in 290-320 now, and the costs have not been measured again.)
 int pick_bn(long long m_tiles, int k_out, int num_sms) {
   const int bns[3] = {256, 128, 64};
   const int step_cost[3] = {512, 400, 300};
@@ -1250,9 +1251,9 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   const bool pair = pair_ok && (pair_env == 1 || (pair_env != 0 && total_chunks_ll >= 8));
   // Two row blocks per CTA for narrow outputs (bn <= 128): twice the tensor work per barrier probe and per tile.
   const int rows2_env = knobs().rows2;
-  // A 256-row tile costs an SM about 1.6x what a 128-row tile costs it (measured; the narrow tile is bound by the
-  // shared-memory fill rate, which B's reuse across two row blocks relieves): taken when it shortens the launch,
-  // wave quantisation included.
+  // A 256-row tile costs an SM about 1.6x what a 128-row tile costs it (measured with the issue loops that pick_bn's costs
+  // are from; the narrow tile was bound by the shared-memory fill rate, which B's reuse across two row blocks relieves):
+  // taken when it shortens the launch, wave quantisation included.
   const long long n_tiles = (K + bn - 1) / bn;
   const long long waves_128 = (m_tiles_128 * n_tiles + st.num_sms - 1) / st.num_sms;
   const long long waves_256 = ((m_tiles_128 + 1) / 2 * n_tiles + st.num_sms - 1) / st.num_sms;
