@@ -1262,10 +1262,11 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
 
   // ---- problems of up to one wave: the small-tile kernel (conv2d_small_sm100.cuh). Where two k-steps come in one copy per
   // operand -- 1x1 convolutions and products over whole 128-byte chunks -- a k-step takes it about half the general kernel's
-  // time (2048 -> 512 channels on one 7x7 image 8.3 -> 5.1 us, 64 x 1000 x 2048 8.7 -> 5.3); with im2col copies a step costs
-  // more than the general kernel's, and the microsecond that its launch is shorter by pays for about 30 of them (3x3, one
-  // image: 64 channels 5.1 -> 4.5, 128 channels 6.5 -> 6.1, but 256 channels 9.3 -> 9.6). More than one tile per SM gains
-  // nothing (1x1 64->64 at 4 images: 196 tiles, 3.65 -> 3.88). Costs in cycles.
+  // time (2048 -> 512 channels on one 7x7 image 8.5 -> 5.2 us, 64 x 1000 x 2048 8.7 -> 5.3); with im2col copies its step is
+  // put above the general kernel's, so that the microsecond that its launch is shorter by pays for about 30 of them. (3x3, one
+  // image: 64 channels 5.3 -> 3.8, 128 channels 6.7 -> 4.7, 192 channels, 27 steps, 8.0 -> 5.6: the 360 and 410 below, from an
+  // earlier build in which 256 channels lost, 9.3 -> 9.6, look too high and have not been measured again.) More than one tile
+  // per SM gains nothing (1x1 64->64 at 4 images: 196 tiles, 3.65 -> 3.88). Costs in cycles.
   const bool whole_chunks = chunk_bytes == 128 && row_bytes % 128 == 0;
   const bool plain_a = whole_chunks && !window && R == 1 && S == 1 && p.stride_h == 1 && p.stride_w == 1 &&
                        p.padding_h == 0 && p.padding_w == 0 && p.pad_h_hi == 0 && p.pad_w_hi == 0 &&
