@@ -1,0 +1,52 @@
+"""Edges of the forms a call can take inside the library that are chosen by a rule on its sizes, against the CPU oracle (or, for
+matrix products, float64), with the launch counters that show which kernel ran."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+import torch
+
+import convcases as cc
+from oracle import oracle
+from tracea_b200 import ffi, ops
+
+pytestmark = pytest.mark.gpu
+
+TORCH_DT = {"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}
+
+
+def conv(case, dtype):
+    """Runs one case (N, C, H, W, K, R, stride, pad, epilogue, channels-last) and returns (output, oracle's output)."""
+    N, C, H, W, K, R, stride, pad, epi, last = case
+    x, w = cc.normal((N, C, H, W), 57, "forms/x"), cc.kaiming((K, C, R, R), 57, "forms/w")
+    ho, wo = oracle.out_shape(x.shape, w.shape, stride, pad, 1)[2:]
+    b = cc.normal((K,), 57, "forms/b", 0.1) if "bias" in epi else None
+    r = cc.normal((N, K, ho, wo), 57, "forms/r") if "residual" in epi else None
+    dev = lambda a: torch.from_numpy(a).to(TORCH_DT[dtype]).cuda().contiguous(
+        memory_format=torch.channels_last if last else torch.contiguous_format)
+    got = ops.conv2d_nchw(dev(x), dev(w), torch.from_numpy(b).cuda() if b is not None else None,
+                          dev(r) if r is not None else None, stride, pad, 1, 1, epi, channels_last_out=last)
+    act = next((o for o in epi.split("+") if o in ("relu", "silu", "gelu")), "none")
+    want = oracle.conv2d_gemm(cc.channels_last(cc.round_to(x, dtype)), cc.round_to(w, dtype), b,
+                              cc.channels_last(cc.round_to(r, dtype)) if r is not None else None, stride, pad, 1, act)
+    return got, cc.round_to(np.ascontiguousarray(want), dtype)
+
+
+def check(case, dtype):
+    got, want = conv(case, dtype)
+    err = cc.rel_err(got.float().cpu().numpy(), want)
+    assert err <= cc.tol_for(dtype), (case, dtype, err)
+    return got
+
+
+# Staging boxes per epilogue warp: two below 8 k-steps and with a residual, one from 8 on, none for NCHW. The bias: resident up to
+# 512 columns (whole tiles counted), by column group above. More tiles than SMs, so that every buffer comes round again.
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("steps", [7, 8, 9])
+@pytest.mark.parametrize("K,epi,last", [(264, "bias+relu", True), (512, "bias+residual+relu", True), (520, "bias+silu", True),
+                                        (1000, "bias+residual", True), (600, "bias", False), (72, "bias+gelu", True)])
+def test_staging_depth_and_bias_forms(dtype, steps, K, epi, last):
+    C = steps * (32 if dtype == "f32" else 64)
+    check((4, C, 73, 67, K, 1, 1, 0, epi.replace("bias+gelu", "gelu"), last), dtype)

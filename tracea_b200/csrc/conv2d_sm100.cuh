@@ -51,6 +51,7 @@ enum : uint32_t {
   kErrEpilogueWait = 4,   // epilogue: accumulator never became ready
   kErrResidualWait = 5,   // epilogue: a residual box never landed
   kErrSplitWait = 6,      // epilogue: the partial sums of a tile split over K never all arrived
+  kErrSmemAlign = 7,      // the CTA's shared memory does not start on a 1024-byte boundary
 };
 
 enum : int { kActNone = 0, kActRelu = 1, kActGelu = 2, kActSilu = 3 };
@@ -82,7 +83,9 @@ struct ConvKernelArgs {
   int panel_width;  // column tiles per panel of the tile order (>= 1; num_n_tiles = one panel = row-major order)
   int panel_tiles;  // num_m_tiles * panel_width
   int num_stages;
-  int shared_bias;  // 1: one bias copy per CTA (num_n_tiles == 1) instead of one per epilogue warp
+  int shared_bias;  // floats from one column tile's bias to the next in the CTA's one copy, -1: a tile's copy per epilogue warp
+  int bias_bytes;
+  int staging_depth;  // staging boxes per epilogue warp: 2, 1 or (no box needed) 0
   // Work schedule. Tiles [0, dp_tiles) are dealt whole to the workers (CTAs, or CTA pairs) round robin. The k-steps
   // of the remaining sk_tiles tiles -- the partly filled last wave of a large layer, or every tile of a layer with
   // fewer tiles than SMs -- are laid end to end and cut into equal shares for the first sk_workers workers, so a
@@ -187,21 +190,25 @@ __device__ __forceinline__ void report_error(const ConvKernelArgs& a, volatile u
 
 // Shared memory map (offsets from a 1024-byte aligned base):
 //   [0, stages * stage_bytes)        operand ring: per stage A (128 rows x 128 B) then B (BN rows x 128 B)
-//   + kStagingBytes                  per epilogue warp 2 alternating 4 KB boxes (32 pixels x 128 B): the residual
+//   + 8 * staging_depth * 4 KB       per epilogue warp up to 2 alternating boxes (32 pixels x 128 B): the residual
 //                                    is TMA-loaded into a box, combined in place, and the box is TMA-stored
-//   + 8 * BN * 4                     per-epilogue-warp copy of the tile's bias, as fp32 (one BN * 4 copy for the
-//                                    whole CTA when the output is a single tile wide: the bias never changes)
-//   + 256                            mbarriers, TMEM base slot, abort flag
+//   + bias_bytes                     the bias as fp32: one copy for the whole CTA where all columns fit kSharedBiasColumns or
+//                                    there is none, else a copy of its tile's columns per epilogue warp
+//   + kBarrierBytes                  mbarriers, TMEM base slot, abort flag
+// What the ring does not get costs time: under load a copy takes about as long to arrive as four or five stages last.
 constexpr int kStagingBoxBytes = 32 * 128;
-constexpr int kStagingDepth = 2;
+constexpr int kStagingDepth = 2;      // at most
 constexpr int kNumEpilogueWarps = 8;
-constexpr int kStagingBytes = kNumEpilogueWarps * kStagingDepth * kStagingBoxBytes;
+constexpr int kSharedBiasColumns = 512;
+constexpr int kBarrierBytes = 512;
+__host__ __device__ constexpr int conv_bias_bytes(int bn, int n_tiles, bool has_bias) {
+  return (!has_bias ? bn : (n_tiles * bn <= kSharedBiasColumns ? n_tiles * bn : kNumEpilogueWarps * bn)) * 4;
+}
 // `pair`: two CTAs on neighbouring SMs work on one 256-row tile and each holds only half of B's rows.
 // `rows2`: one CTA owns a 256-row tile (two 128-row blocks of A per stage against one B).
-__host__ __device__ constexpr int conv_smem_bytes(int bn, int stages, bool pair = false, bool rows2 = false,
-                                                  bool shared_bias = false) {
-  return stages * ((rows2 ? 2 : 1) * kBlockM * kStageKBytes + (pair ? bn / 2 : bn) * kStageKBytes) + kStagingBytes +
-         (shared_bias ? 1 : kNumEpilogueWarps) * bn * 4 + 512 + 1024;
+__host__ __device__ constexpr int conv_smem_bytes(int bn, int stages, bool pair, bool rows2, int staging_depth, int bias_bytes) {
+  return stages * ((rows2 ? 2 : 1) * kBlockM * kStageKBytes + (pair ? bn / 2 : bn) * kStageKBytes) +
+         kNumEpilogueWarps * staging_depth * kStagingBoxBytes + bias_bytes + kBarrierBytes;
 }
 
 // (a, b) += (c, d) as one packed fp32x2 add.
@@ -738,14 +745,18 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
   static_assert(BN == 64 || BN == 128 || BN == 256, "BN");
 
   TB200_PROF_NOW(12);
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = __shfl_sync(0xffffffffu, (smem_u32(smem_raw) + 1023u) & ~1023u, 0);
-  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t smem_base = __shfl_sync(0xffffffffu, smem_u32(smem_raw), 0);
+  if ((smem_base & 1023u) != 0u) {   // the swizzled operand layout depends on it, and the host left no room to round up
+    if (threadIdx.x == 0 && args.status != nullptr) atomicCAS(args.status, 0u, static_cast<uint32_t>(kErrSmemAlign));
+    return;
+  }
+  uint8_t* smem_gen = smem_raw;
   const int num_stages = args.num_stages;
   const uint32_t ring_bytes = static_cast<uint32_t>(num_stages) * kStageBytes;
   const uint32_t staging_base = smem_base + ring_bytes;
-  const uint32_t bias_off = ring_bytes + kStagingBytes;
-  const uint32_t bar_off = bias_off + (args.shared_bias ? 1u : static_cast<uint32_t>(kNumEpilogueWarps)) * BN * 4u;
+  const uint32_t bias_off = ring_bytes + static_cast<uint32_t>(kNumEpilogueWarps * args.staging_depth) * kStagingBoxBytes;
+  const uint32_t bar_off = bias_off + static_cast<uint32_t>(args.bias_bytes);
   const uint32_t bar_base = smem_base + bar_off;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (kMaxStages + s); };
@@ -1111,10 +1122,10 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
     constexpr int kLdPerGroup = kGroupCols / 32;
     constexpr int kChunksPerLd = 32 / kVec;        // 16-byte chunks produced per 32-column TMEM load
     // with a shared copy every warp writes the same values to the same words before it reads them
-    const int bias_slot = args.shared_bias ? 0 : ew * BN;
-    float* bias_w = reinterpret_cast<float*>(smem_gen + bias_off) + bias_slot;
-    const uint32_t bias_w_s = smem_base + bias_off + static_cast<uint32_t>(bias_slot) * 4u;
-    const uint32_t stg0 = staging_base + static_cast<uint32_t>(ew) * (kStagingDepth * kStagingBoxBytes);
+    float* bias_w = reinterpret_cast<float*>(smem_gen + bias_off) + (args.shared_bias >= 0 ? 0 : ew * BN);
+    uint32_t bias_w_s = smem_base + bias_off + (args.shared_bias >= 0 ? 0u : static_cast<uint32_t>(ew) * BN * 4u);
+    const uint32_t stg0 = staging_base + static_cast<uint32_t>(ew * args.staging_depth) * kStagingBoxBytes;
+    const uint32_t box_flip = args.staging_depth == 2 ? 1u : 0u;
     // this lane's 16-byte chunk c of its staging row lives at row*128 + ((c ^ (row & 7)) << 4): the
     // SWIZZLE_128B pattern of the out / residual tensor maps (bank-conflict free for 8-lane phases)
     const uint32_t lane_row_off = static_cast<uint32_t>(lane) * 128u;
@@ -1268,6 +1279,9 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
       // this warp's fp32 copy of the tile's bias (zeros when there is none / past K_out); the values
       // were fetched into registers during the previous tile, and the next tile's are fetched now
       if (n_tile != bias_tile) {
+        const int move = args.shared_bias > 0 ? (n_tile - max(bias_tile, 0)) * args.shared_bias : 0;   // to the tile's own columns
+        bias_w += move;
+        bias_w_s += static_cast<uint32_t>(move) * 4u;
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < kBiasPerLane; ++j) bias_w[j * 32 + lane] = bias_next[j];
@@ -1370,7 +1384,10 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
           }
         } else if constexpr (kStore == kStoreTma) {
           TB200_PROF_T(ts);
-          if (lane == 0) bulk_wait_group_read<1>();   // this box's previous store (two groups ago) has been read out
+          if (lane == 0) {   // this box's previous store (one or two groups ago) has been read out
+            if (box_flip != 0u) bulk_wait_group_read<1>();
+            else bulk_wait_group_read<0>();
+          }
           __syncwarp();
           TB200_PROF_ADD(prof_wstore, ts);
         }
@@ -1443,13 +1460,13 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
             tma_store_2d(&tmap_out, stg, n0, m_row0);
             bulk_commit_group();
           }
-          box ^= 1u;
+          box ^= box_flip;
         } else if (kStore == kStoreRows || (kStore == kStoreMixed && args.out_rows)) {
 #pragma unroll
           for (int c = 0; c < 8; ++c)
             st_shared_v4(stg + lane_row_off + ((static_cast<uint32_t>(c) ^ lane_xor) << 4), packed[c]);
           store_rows<OutT>(args.out_vec, stg, out + n0, out_off, row_ok, args.K_out - n0, lane);
-          box ^= 1u;
+          box ^= box_flip;
         }
         TB200_PROF_ADD(prof_stage, tg);
       }

@@ -394,9 +394,9 @@ int pick_chunk_bytes(long long row_bytes) {
   return chunk;
 }
 
-int pick_stages(int bn, bool pair, bool rows2, bool shared_bias) {
-  const int stage_bytes = tb200::conv_smem_bytes(bn, 1, pair, rows2) - tb200::conv_smem_bytes(bn, 0, pair, rows2);
-  const int fixed = tb200::conv_smem_bytes(bn, 0, pair, rows2, shared_bias);
+int pick_stages(int bn, bool pair, bool rows2, int staging_depth, int bias_bytes) {
+  const int fixed = tb200::conv_smem_bytes(bn, 0, pair, rows2, staging_depth, bias_bytes);
+  const int stage_bytes = tb200::conv_smem_bytes(bn, 1, pair, rows2, staging_depth, bias_bytes) - fixed;
   int s = (232448 - fixed) / stage_bytes;  // 227 KB opt-in limit per CTA
   return std::min(s, tb200::kMaxStages);
 }
@@ -1516,18 +1516,30 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   // wave off into a second launch with 128-row tiles was measured and is slower: a CTA pair's 256-row tile costs
   // each SM exactly what a 128-row tile costs it, so the tail does not get shorter, and the launch boundary adds
   // ~10 us.)
+  const long long k_steps = (total_chunks_ll * chunk_bytes + 127) / 128;   // pipeline stages a tile takes
   auto launch_rows = [&](bool pair_v, bool rows2_v, long long row_begin, long long row_end) {
     const long long rows = row_end - row_begin;
     const long long tile_rows = (pair_v || rows2_v) ? 2 * tb200::kBlockM : tb200::kBlockM;
     const long long m_tiles = (rows + tile_rows - 1) / tile_rows;
     if (m_tiles * n_tiles > 0x7fffffffLL) TB_FAIL(TRACEA_UNSUPPORTED_CONFIG, "too many tiles");
-    // an output one tile wide never changes its bias: one copy per CTA instead of one per epilogue warp leaves
-    // room for a fifth stage of the CTA-pair tiling
-    const bool shared_bias = n_tiles == 1;
-    int stages = pick_stages(bn, pair_v, rows2_v, shared_bias);
+    const int bias_bytes = tb200::conv_bias_bytes(bn, static_cast<int>(n_tiles), a.bias != nullptr);
+    // Staging boxes per epilogue warp: none for per-lane stores; two where a residual arrives in one while the other is being
+    // stored, and where the epilogue sets the pace -- few k-steps between two tiles, or an activation that takes its time (3x3/2
+    // 128->256 + SiLU 110.0 -> 110.9 us with one); otherwise one, if that buys stages (pair tiling 5 and 6 where there were 4 and
+    // 5: 1x1 1024->512 at 512 images 100 -> 84 us, 2048->512 50.2 -> 46.5, 8192^3 851 -> 826; 53-layer stack at one image 306.6
+    // -> 299.8).
+    int depth = store == tb200::kStoreStrided ? 0 : 2;
+    int stages = pick_stages(bn, pair_v, rows2_v, depth, bias_bytes);
+    if (depth == 2 && res_v == nullptr && k_steps >= 8 && (epi.act == tb200::kActNone || epi.act == tb200::kActRelu)) {
+      const int more = pick_stages(bn, pair_v, rows2_v, 1, bias_bytes);
+      if (more > stages) {
+        depth = 1;
+        stages = more;
+      }
+    }
     const int forced_stages = knobs().force_stages;
     if (forced_stages >= 2 && forced_stages <= stages) stages = forced_stages;
-    const int smem = tb200::conv_smem_bytes(bn, stages, pair_v, rows2_v, shared_bias);
+    const int smem = tb200::conv_smem_bytes(bn, stages, pair_v, rows2_v, depth, bias_bytes);
 
     CUtensorMap tmap_w;
     encode_w(&tmap_w, pair_v ? bn / 2 : bn);
@@ -1544,7 +1556,9 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     la.panel_width = static_cast<int>(panel);
     la.panel_tiles = static_cast<int>(m_tiles * panel);
     la.num_stages = stages;
-    la.shared_bias = shared_bias ? 1 : 0;
+    la.shared_bias = a.bias == nullptr ? 0 : (n_tiles * bn <= tb200::kSharedBiasColumns ? bn : -1);
+    la.bias_bytes = bias_bytes;
+    la.staging_depth = depth;
     la.idesc = tb200::ptx::make_idesc(fmt, pair_v ? 2 * tb200::kBlockM : tb200::kBlockM, bn);
     const long long tiles = m_tiles * n_tiles;
     const long long workers_max = pair_v ? st.num_sms / 2 : st.num_sms;   // CTAs, or CTA pairs
