@@ -166,7 +166,8 @@ typedef struct {
  * Rank-2 views, strides in elements (NULL = row-major). It runs as the 1x1 convolution it is: `a` rows are the
  * pixels, `b` columns the output channels. The zero-copy form is a with stride[1] == 1 and b with stride[0] == 1
  * and stride[1] == K (memory [N][K], e.g. a transposed view of a Linear layer's weight, or the buffer
- * tracea_gemm_prepack_b wrote); a row-major b is transposed into scratch on every call. bias: rank-1, length N;
+ * tracea_gemm_prepack_b wrote); a row-major b of 16-bit elements whose rows start on 16-byte boundaries
+ * is read in place too, any other row-major b is transposed into scratch on every call. bias: rank-1, length N;
  * residual: [M,N], dtype of c. Dtypes as tracea_conv2d (fp32 runs as TF32; the reference's entry took fp16 only).
  * rank != 2 or a shape mismatch -> INVALID_PARAMS. */
 TraceaStatus tracea_gemm(TraceaTensorView a, TraceaTensorView b, const TraceaTensorView *bias,

@@ -50,3 +50,25 @@ def check(case, dtype):
 def test_staging_depth_and_bias_forms(dtype, steps, K, epi, last):
     C = steps * (32 if dtype == "f32" else 64)
     check((4, C, 73, 67, K, 1, 1, 0, epi.replace("bias+gelu", "gelu"), last), dtype)
+
+
+# Row-major B of 16-bit elements, read in place 64 columns at a time: columns and rows of K at the edges of those blocks, all
+# tilings (rows up to one small tile, one wave, many). The sums are added in the order of a K-major B: the same bits.
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("M", [1, 65, 3000, 20000])
+def test_row_major_b_is_read_in_place(dtype, M):
+    for N, K in ((8, 64), (64, 40), (72, 72), (136, 200), (264, 520), (1000, 776), (640, 1024)):
+        a = torch.from_numpy(cc.normal((M, K), 58, "mn/a")).to(TORCH_DT[dtype]).cuda()
+        b = torch.from_numpy(cc.normal((K, N), 58, "mn/b", K ** -0.5)).to(TORCH_DT[dtype]).cuda()
+        before = ffi.launch_count_of(ffi.KERNEL_LAYOUT)
+        got = ops.gemm(a, b)
+        assert ffi.launch_count_of(ffi.KERNEL_LAYOUT) == before, (M, N, K)
+        want = a.double() @ b.double()
+        assert float((got.double() - want).abs().max() / want.abs().max()) <= cc.TOL_16BIT, (M, N, K)
+        assert torch.equal(got, ops.gemm(a, b.t().contiguous().t())), (M, N, K)
+    wide = torch.from_numpy(cc.normal((96, 136), 58, "mn/w")).to(TORCH_DT[dtype]).cuda()
+    a = torch.from_numpy(cc.normal((M, 96), 58, "mn/a2")).to(TORCH_DT[dtype]).cuda()
+    part = wide[:, 8:128]            # columns of a wider matrix
+    assert torch.equal(ops.gemm(a, part), ops.gemm(a, part.t().contiguous().t()))
+    odd = wide[:, 1:100]             # no 16-byte rows: repacked as ever
+    assert torch.equal(ops.gemm(a, odd), ops.gemm(a, odd.t().contiguous().t()))

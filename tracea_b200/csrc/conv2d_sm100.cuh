@@ -78,6 +78,9 @@ struct ConvKernelArgs {
   // tap ends in zeros instead of in the next tap's weights; taps at any stride of the row, from column b_k0 with jumps
   // (only used with 128-byte chunks, one chunk per stage).
   int b_k0, b_jump_s, b_jump_r, b_tap_step;
+  // > 0: B is a row-major [K][N] matrix of 16-bit elements, read in place by a map {column n, row k, 1} whose copies bring 64
+  // columns x 64 rows of K each (the MMA takes such a B with N contiguous): this many copies a stage. One tap, 128-byte k-chunks.
+  int b_n_groups;
   // tiling / pipeline
   int num_m_tiles, num_n_tiles;
   int panel_width;  // column tiles per panel of the tile order (>= 1; num_n_tiles = one panel = row-major order)
@@ -733,6 +736,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
   constexpr uint32_t kBRows = kPair ? BN / 2 : BN;       // rows of B this CTA keeps in shared memory
   constexpr uint32_t kBBytes = kBRows * kStageKBytes;
   constexpr uint32_t kStageBytes = kABytes + kBBytes;
+  constexpr uint32_t kNGroupBytes = 64u * kStageKBytes;   // row-major B: 64 rows of K x 64 columns
   constexpr int kTileM = (kPair || kRows2) ? 2 * kBlockM : kBlockM;   // output pixels per tile
   // (shuffles: the same value in every lane, provably -- the MMA warp's control flow has to be uniform)
   const uint32_t cta_rank = kPair ? __shfl_sync(0xffffffffu, cluster_ctarank(), 0) : 0u;
@@ -852,7 +856,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
       uint32_t phase = 0;
       const uint32_t a_chunk_bytes = kBlockM * args.chunk_bytes;
       const uint32_t b_chunk_bytes = BN * args.chunk_bytes;
-      const bool one_chunk = (chunks_per_stage == 1) && !args.a_tiled;
+      const bool one_chunk = (chunks_per_stage == 1) && !args.a_tiled && args.b_n_groups == 0;
       bool ok = true;
       int issued = 0;
       int m_tile = 0, n_tile = 0;
@@ -939,6 +943,50 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
               tap_coord += args.b_tap_step;
               if (++tap_s == args.S) { tap_s = 0; off_w = 0; off_h += args.dil_h; k_coord += args.b_jump_r; }
             }
+            ++issued;
+            stage_addr = nstage; full_addr = nfull; empty_addr = nempty; phase = nphase;
+            slot_free = __all_sync(0xffffffffu, next_free);
+          }
+        } else if (args.b_n_groups > 0) {
+          // row-major B, one tap: as above, with a copy of B for every 64 columns. All but the last are issued ahead of the
+          // block that arms the full barrier: bytes may arrive on it before, its phase cannot end without that arrival.
+          const int last = args.b_n_groups - 1;
+          int k_coord = item.k_begin * args.chunk_elems;
+          for (int it = item.k_begin; it < item.k_end; ++it) {
+            if (issued == args.test_producer_stop) {
+              stopped = true;
+              break;
+            }
+            if (!slot_free && !mbar_wait_bounded_uniform(empty_addr, phase ^ 1u, abort_p, args.wait_limit)) {
+              if (issue) report_error(args, abort_p, kErrProducerWait, (uint32_t)it);
+              ok = false;
+              break;
+            }
+            uint32_t nstage = stage_addr + kStageBytes, nfull = full_addr + 8u, nempty = empty_addr + 8u, nphase = phase;
+            if (nstage == ring_end) { nstage = smem_base; nfull = full_bar0; nempty = empty_bar0; nphase ^= 1u; }
+            const uint32_t full_leader = full_leader0 + (full_addr - full_bar0);
+            uint32_t b_dst = stage_addr + kABytes;
+            int n_group = n_coord;
+            for (int g = 0; g < last; ++g) {
+              if constexpr (kPair) tma_load_3d_pair_if(issue, b_dst, &tmap_w, full_leader, n_group, k_coord, 0);
+              else tma_load_3d_if(issue, b_dst, &tmap_w, full_addr, n_group, k_coord, 0);
+              b_dst += kNGroupBytes;
+              n_group += 64;
+            }
+            bool next_free;
+            if constexpr (kPair) {
+              next_free = tma_stage_probe_pair(stage_addr, b_dst, full_addr, full_leader, leader ? 2u * kStageBytes : 0u,
+                                               &tmap_x, k_coord, w_start, h_start, img0, 0, 0, &tmap_w, n_group, k_coord, 0,
+                                               nempty, nphase ^ 1u, issue);
+            } else if constexpr (kRows2) {
+              next_free = tma_stage_probe_rows2(stage_addr, stage_addr + kABlockBytes, b_dst, full_addr, kStageBytes, &tmap_x,
+                                                k_coord, w_start, h_start, img0, w_start1, h_start1, img1, 0, 0, &tmap_w,
+                                                n_group, k_coord, 0, nempty, nphase ^ 1u, issue);
+            } else {
+              next_free = tma_stage_probe(stage_addr, b_dst, full_addr, kStageBytes, &tmap_x, k_coord, w_start, h_start, img0,
+                                          0, 0, &tmap_w, n_group, k_coord, 0, nempty, nphase ^ 1u, issue);
+            }
+            k_coord += args.chunk_elems;
             ++issued;
             stage_addr = nstage; full_addr = nfull; empty_addr = nempty; phase = nphase;
             slot_free = __all_sync(0xffffffffu, next_free);

@@ -70,7 +70,10 @@ conv2d_small_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gr
     prefetch_tmap(&tmap_x);
     prefetch_tmap(&tmap_w);
     // a hint only: whatever an earlier kernel still writes there is read after griddep_wait below
-    for (int i = 0; i < min(k_stages, num_stages) && args.b_prefetch; ++i) tma_prefetch_3d(&tmap_w, 0, n_base, 2 * i);
+    for (int i = 0; i < min(k_stages, num_stages) && args.b_prefetch; ++i) {
+      if (args.b_n_groups > 0) tma_prefetch_3d(&tmap_w, n_base, 2 * i * args.chunk_elems, 0);
+      else tma_prefetch_3d(&tmap_w, 0, n_base, 2 * i);
+    }
   }
   if (warp == 1) {
     tmem_alloc<BN>(tmem_slot);
@@ -98,6 +101,10 @@ conv2d_small_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gr
     const int h_start = (t - img0 * args.Ho) * args.stride_h - args.pad_h;
     int c_coord = 0, k_coord = args.b_k0, tap_coord = 0, tap_s = 0;
     uint32_t off_w = 0, off_h = 0;
+    // B two k-steps at a time: {0, n, chunk} of an [N][K] matrix, or {n, k, 0} of a row-major [K][N] one
+    const bool n_major = args.b_n_groups > 0;
+    const int b_c0 = n_major ? n_base : 0, b_d1 = n_major ? 2 * args.chunk_elems : 0, b_d2 = n_major ? 0 : 2;
+    int b_c1 = n_major ? 0 : n_base, b_c2 = 0;
     int stage = 0, issued = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -115,7 +122,11 @@ conv2d_small_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gr
       mbar_arrive_expect_tx_if(issue, full, (args.a_steps2 ? 2u : steps) * kAStep + (args.b_steps2 ? 2u : steps) * kBStep);
       // both k-steps in one copy; past the last one it reads zeros
       if (args.a_steps2) tma_load_3d_if(issue, a_dst, &tmap_x, full, 0, m0, 2 * it);
-      if (args.b_steps2) tma_load_3d_if(issue, b_dst, &tmap_w, full, 0, n_base, 2 * it);
+      if (args.b_steps2) {
+        tma_load_3d_if(issue, b_dst, &tmap_w, full, b_c0, b_c1, b_c2);
+        b_c1 += b_d1;
+        b_c2 += b_d2;
+      }
       if (!args.a_steps2 || !args.b_steps2) {
         for (uint32_t u = 0; u < steps; ++u) {
           if (!args.a_steps2)

@@ -208,6 +208,18 @@ __device__ __forceinline__ void tma_load_3d_if(uint32_t issue, uint32_t dst, con
       "}\n" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(issue)
       : "memory");
 }
+// The same from either CTA of a pair, signalling the leader's barrier (a shared::cluster address).
+__device__ __forceinline__ void tma_load_3d_pair_if(uint32_t issue, uint32_t dst, const void* tmap, uint32_t bar, int c0, int c1,
+                                                    int c2) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %6, 0;\n"
+      "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];\n"
+      "}\n" ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(issue)
+      : "memory");
+}
 __device__ __forceinline__ void tma_load_im2col_4d_if(uint32_t issue, uint32_t dst, const void* tmap, uint32_t bar, int c, int w,
                                                       int h, int n, uint16_t off_w, uint16_t off_h) {
   asm volatile(
@@ -618,12 +630,12 @@ __device__ __forceinline__ void tmem_st_wait() {
 //   [49,52) base offset (0: stage buffers are 1024-B aligned)   [61,64) swizzle mode
 // Swizzle modes: 0 none, 2 = 128 B, 4 = 64 B, 6 = 32 B.
 // Instruction descriptor (32-bit) for kind::f16 / kind::tf32, dense, fp32 accumulate,
-// both operands K-major.
+// A K-major.
 //   [4,6) D format (1 = f32)   [7,10) A format   [10,13) B format
 //   (kind::f16: 0 = f16, 1 = bf16; kind::tf32: 2 = tf32)
-//   [15] A major, [16] B major (0 = K-major)   [17,23) N >> 3   [24,29) M >> 4
-__host__ __device__ constexpr uint32_t make_idesc(uint32_t ab_format, uint32_t m, uint32_t n) {
-  return (1u << 4) | (ab_format << 7) | (ab_format << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
+//   [15] A major, [16] B major (0 = K-major, 1 = N contiguous)   [17,23) N >> 3   [24,29) M >> 4
+__host__ __device__ constexpr uint32_t make_idesc(uint32_t ab_format, uint32_t m, uint32_t n, uint32_t b_n_major = 0) {
+  return (1u << 4) | (ab_format << 7) | (ab_format << 10) | (b_n_major << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
 }  // namespace ptx

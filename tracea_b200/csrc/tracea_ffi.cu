@@ -1203,6 +1203,14 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
       b_jump_r = sr - S * ss;
     }
   }
+  // A row-major 16-bit B of a matrix product: the MMA takes a B with N contiguous, so it is read in place too, at the price of a
+  // copy for every 64 columns of a stage. Against a repack per call, bf16: 2048 x 2048 x 1024 13.9 -> 11.7 us, 256 x 4096 x 4096
+  // 27.4 -> 14.3, 8192 x 4096 x 4096 191 -> 171, 1000 x 512 x 512 6.7 -> 4.9, 16000 x 64 x 256 6.5 -> 4.8; K-major B of the same
+  // sizes is at most 4 % faster.
+  const bool w_n_major = !w_direct && !window && es == 2 && R == 1 && S == 1 && w_in.stride[0] == 1 && chunk_bytes == 128 &&
+                         (w_in.stride[1] * es) % 16 == 0 && w_in.stride[1] >= K && aligned16(w_in.ptr) && K > 1 &&
+                         knobs().force_chunk == 0 && knobs().tiled_a == 0;
+  if (w_n_major) w_direct = true;
   const bool stage_w = !w_direct || window;
   {
     // one block of scratch and one launch for both operands
@@ -1282,6 +1290,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     const long long m_tiles_64 = (M + tb200::kSmallM - 1) / tb200::kSmallM;
     for (int b = 64; b >= 32; b >>= 1) {
       if (m_tiles_64 * ((K + b - 1) / b) > st.num_sms) continue;
+      if (w_n_major && b < 64) continue;   // its columns come 64 at a time
       const long long cost = k_steps * (plain_a ? (b == 32 ? 130 : 160) : (b == 32 ? 360 : 410));
       if (cost < best) {
         best = cost;
@@ -1289,7 +1298,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
       }
     }
   }
-  const bool b_steps2 = small_bn != 0 && whole_chunks && !w_remap;
+  const bool b_steps2 = small_bn != 0 && (w_n_major || (whole_chunks && !w_remap));
   const bool a_steps2 = small_bn != 0 && plain_a;
   const int a_rows = small_bn != 0 ? tb200::kSmallM : tb200::kBlockM;
 
@@ -1392,6 +1401,10 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
       a.b_mma_off[k] = 2u * k * b_chunk;
     }
   }
+  if (w_n_major) {   // 64 columns x 64 rows of K a block: 8 rows are 1024 bytes (SBO), the next 64 columns follow behind (LBO)
+    a.b_lbo = 64u * 128u;
+    for (int k = 0; k < 4; ++k) a.b_mma_off[k] = 16u * 128u * k;
+  }
   a.out = out.ptr;
   a.out_sn = out.stride[0];
   a.out_sc = out.stride[1];
@@ -1485,6 +1498,17 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   const uint32_t fmt = x.dtype == TRACEA_DTYPE_FLOAT16 ? 0u : (x.dtype == TRACEA_DTYPE_BFLOAT16 ? 1u : 2u);
 
   auto encode_w = [&](CUtensorMap* m, int box_rows) {
+    if (w_n_major) {   // {output channel, k, 1}; the small-tile kernel brings in two k-steps at once
+      const cuuint64_t gdim[3] = {(cuuint64_t)K, (cuuint64_t)C, 1u};
+      const cuuint64_t gstr[2] = {(cuuint64_t)(w_in.stride[1] * es), (cuuint64_t)(w_in.stride[1] * es)};
+      const cuuint32_t box[3] = {64u, small_bn != 0 ? 128u : 64u, 1u};
+      const cuuint32_t estr[3] = {1u, 1u, 1u};
+      CUresult r = g_encode_tiled(m, tmap_dtype(x.dtype), 3, const_cast<void*>(w_ptr), gdim, gstr, box, estr,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      if (r != CUDA_SUCCESS) TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled (row-major B) failed with %d", (int)r);
+      return;
+    }
     if (b_steps2) {   // {column in chunk, output channel, chunk of Kgemm}
       const cuuint64_t gdim[3] = {(cuuint64_t)chunk_elems, (cuuint64_t)K, (cuuint64_t)total_chunks_ll};
       const cuuint64_t gstr[2] = {(cuuint64_t)(Kgemm * es), 128};
@@ -1559,7 +1583,8 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     la.shared_bias = a.bias == nullptr ? 0 : (n_tiles * bn <= tb200::kSharedBiasColumns ? bn : -1);
     la.bias_bytes = bias_bytes;
     la.staging_depth = depth;
-    la.idesc = tb200::ptx::make_idesc(fmt, pair_v ? 2 * tb200::kBlockM : tb200::kBlockM, bn);
+    la.idesc = tb200::ptx::make_idesc(fmt, pair_v ? 2 * tb200::kBlockM : tb200::kBlockM, bn, w_n_major ? 1u : 0u);
+    la.b_n_groups = w_n_major ? (pair_v ? bn / 2 : bn) / 64 : 0;
     const long long tiles = m_tiles * n_tiles;
     const long long workers_max = pair_v ? st.num_sms / 2 : st.num_sms;   // CTAs, or CTA pairs
     long long workers = std::min<long long>(tiles, workers_max);
@@ -1657,7 +1682,8 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     a.num_n_tiles = static_cast<int>(tiles_n);
     const long long stages_needed = (total_chunks_ll + 1) / 2;   // two 128-byte k-steps each
     a.num_stages = static_cast<int>(std::min<long long>(tb200::small_stages(small_bn), stages_needed));
-    a.idesc = tb200::ptx::make_idesc(fmt, tb200::kSmallM, small_bn);
+    a.idesc = tb200::ptx::make_idesc(fmt, tb200::kSmallM, small_bn, w_n_major ? 1u : 0u);
+    a.b_n_groups = w_n_major ? 1 : 0;
     a.a_steps2 = a_steps2 ? 1 : 0;
     a.b_steps2 = b_steps2 ? 1 : 0;
     a.b_prefetch = b_steps2 && !stage_w ? 1 : 0;

@@ -171,7 +171,8 @@ def conv2d(x, w, bias=None, residual=None, epilogue=None, stride=1, padding=0, d
 def gemm(x, w, bias=None, epilogue=None, residual=None):
     """tracea.ops.gemm (tracea-python/python/tracea/ops.py:12-35): x (M, K) @ w (K, N) -> (M, N) with the conv
     epilogue. Any strides; a ``w`` whose memory is [N][K] (``weight.t()`` of a Linear layer, or the result of
-    ``prepack_gemm_b``) is read in place, a row-major one is transposed into scratch on every call."""
+    ``prepack_gemm_b``) is read in place, and so is a row-major one of 16-bit elements whose rows start on 16-byte
+    boundaries; any other is transposed into scratch on every call."""
     if x.ndim != 2 or w.ndim != 2:
         raise ValueError("Expected 2D tensors: x (M, K), w (K, N)")
     if x.shape[1] != w.shape[0]:
