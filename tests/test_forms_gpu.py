@@ -72,3 +72,28 @@ def test_row_major_b_is_read_in_place(dtype, M):
     assert torch.equal(ops.gemm(a, part), ops.gemm(a, part.t().contiguous().t()))
     odd = wide[:, 1:100]             # no 16-byte rows: repacked as ever
     assert torch.equal(ops.gemm(a, odd), ops.gemm(a, odd.t().contiguous().t()))
+
+
+# Filter rows as k-chunks: channel counts around the pixel pitches of 16 and 32 bytes and around whole chunks, both memory formats
+# that are staged (NCHW, channels-last of odd channel counts), strides, no padding, narrow and one-pixel images, every filter width.
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+def test_filter_rows_as_chunks(dtype):
+    for case in ((3, 20, 31, 23, 50, 5, 1, 2, "gelu", False), (2, 33, 17, 40, 100, 3, 2, 1, "bias+relu", False),
+                 (1, 12, 40, 41, 64, 7, 2, 3, "bias+relu", False), (2, 96, 14, 15, 72, 3, 1, 1, "bias+residual+relu", False),
+                 (2, 50, 9, 11, 33, 3, 1, 1, "residual+relu", True), (1, 17, 1, 1, 20, 3, 1, 1, "bias", False),
+                 (2, 25, 8, 6, 40, 2, 1, 0, "relu", False), (1, 200, 12, 12, 130, 3, 1, 0, "bias+silu", False),
+                 (40, 40, 28, 28, 64, 3, 1, 1, "bias+relu", False), (1, 11, 30, 30, 9, 16, 1, 8, "bias", False),
+                 (2, 9, 5, 7, 70, 5, 3, 2, "bias", True)):
+        check(case, dtype)
+
+
+# The phases of a transposed convolution pad front and back differently.
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+def test_filter_rows_in_the_phases_of_a_transposed_convolution(dtype):
+    for N, C, H, W, K, R, stride, pad, opad in ((2, 20, 9, 13, 24, 4, 2, 1, 0), (1, 33, 7, 6, 40, 5, 2, 2, 1), (1, 50, 5, 8, 17, 5, 3, 1, 2)):
+        x = torch.from_numpy(cc.normal((N, H, W, C), 59, "ct/x")).to(TORCH_DT[dtype]).cuda()
+        w = torch.from_numpy(cc.normal((K, R, R, C), 59, "ct/w", (C * R * R) ** -0.5)).to(TORCH_DT[dtype]).cuda()
+        got = ops.conv_transpose2d(x, w, None, None, None, stride, pad, opad)
+        want = torch.nn.functional.conv_transpose2d(x.double().permute(0, 3, 1, 2), w.double().permute(3, 0, 1, 2), stride=stride,
+                                                    padding=pad, output_padding=opad).permute(0, 2, 3, 1)
+        assert float((got.double() - want).abs().max() / want.abs().max()) <= cc.tol_for(dtype)

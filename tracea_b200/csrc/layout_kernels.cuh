@@ -10,7 +10,8 @@ namespace tb200 {
 
 // One copy src[n][c][p] (element strides) -> dst[n][p][Cp], channels C .. Cp-1 zero-filled: an activation tensor (p: its
 // pixels), a filter bank (n: output channels, p: taps) or a matrix. Cp * sizeof(T) is a multiple of 16 bytes and dst is
-// 16-byte aligned, except in kCopyElements.
+// 16-byte aligned, except in kCopyElements. With pad_lo / pad_hi > 0 (never in kCopyTaps) every row of W pixels is written
+// with that many zero pixels in front of and behind it.
 enum : int {
   kCopyPlanes = 0,     // pixels contiguous (NCHW): 128-byte x 64-pixel tiles transposed through shared memory
   kCopyTaps = 1,       // pixels contiguous, few of them, and channels right behind one another (OIHW filters): a group of
@@ -24,6 +25,7 @@ struct CopyJob {
   int mode;
   int vec;             // elements per source access (kCopyPlanes: along pixels, kCopyRows: along channels)
   int C, Cp, P, W;     // W: pixels per row of the source (pixel p is at (p / W) * sh + (p % W) * sw)
+  int pad_lo, pad_hi;
   long long N;
   long long sn, sc, sh, sw;
   long long blocks;
@@ -69,6 +71,22 @@ __device__ __forceinline__ void copy_tile_in(const CopyJob& j, T* tile, const T*
     for (int k = 0; k < kVec; ++k) tile[(p + k) * kCopyPitch<T> + c] = e[k];
   }
 }
+// The destination pixel of pixel p of image n.
+__device__ __forceinline__ long long copy_dst_pixel(const CopyJob& j, long long n, int p) {
+  if ((j.pad_lo | j.pad_hi) == 0) return n * j.P + p;
+  const int h = p / j.W;
+  return (n * (j.P / j.W) + h) * (j.W + j.pad_lo + j.pad_hi) + j.pad_lo + (p - h * j.W);
+}
+// The zero pixels beside a row's first / last pixel are written by whoever writes that one, at `at`: one V of each.
+template <typename T, typename V>
+__device__ __forceinline__ void copy_pad(const CopyJob& j, T* at, int p) {
+  if ((j.pad_lo | j.pad_hi) == 0) return;
+  const int w = p % j.W;
+  if (w == 0)
+    for (int k = 1; k <= j.pad_lo; ++k) *reinterpret_cast<V*>(at - static_cast<long long>(k) * j.Cp) = V{};
+  if (w == j.W - 1)
+    for (int k = 1; k <= j.pad_hi; ++k) *reinterpret_cast<V*>(at + static_cast<long long>(k) * j.Cp) = V{};
+}
 // 16 bytes of one tile row (4-byte aligned).
 template <typename T>
 __device__ __forceinline__ uint4 tile_chunk(const T* row, int chunk) {
@@ -107,8 +125,11 @@ __global__ void __launch_bounds__(kCopyThreads) copy_channels_last_kernel(const 
     __syncthreads();
     for (int i = tid; i < kCopyTileP * 8; i += kCopyThreads) {   // 8 lanes write one pixel's 128 bytes
       const int p = i >> 3, c = c0 + (i & 7) * kChunk;
-      if (p0 + p < j.P && c < j.Cp)
-        *reinterpret_cast<uint4*>(dst + (n * j.P + p0 + p) * j.Cp + c) = tile_chunk(tile + p * kCopyPitch<T>, i & 7);
+      if (p0 + p < j.P && c < j.Cp) {
+        T* at = dst + copy_dst_pixel(j, n, p0 + p) * j.Cp + c;
+        *reinterpret_cast<uint4*>(at) = tile_chunk(tile + p * kCopyPitch<T>, i & 7);
+        copy_pad<T, uint4>(j, at, p0 + p);
+      }
     }
   } else if (j.mode == kCopyTaps) {
     // one block: one group of 128 bytes of channels of as many images (output channels) as fill the tile
@@ -158,7 +179,9 @@ __global__ void __launch_bounds__(kCopyThreads) copy_channels_last_kernel(const 
       for (int k = 0; k < kChunk; ++k)
         if (c + k < j.C) e[k] = s[k];
     }
-    *reinterpret_cast<uint4*>(dst + i * kChunk) = out;
+    T* at = dst + copy_dst_pixel(j, n, p) * j.Cp + c;
+    *reinterpret_cast<uint4*>(at) = out;
+    copy_pad<T, uint4>(j, at, p);
   } else {
     const int tiles_p = (j.P + 31) / 32, tiles_c = (j.Cp + 31) / 32;
     const int p0 = static_cast<int>(b % tiles_p) * 32;
@@ -177,7 +200,11 @@ __global__ void __launch_bounds__(kCopyThreads) copy_channels_last_kernel(const 
     __syncthreads();
     const int c = c0 + tx;
     for (int i = ty; i < 32; i += kCopyThreads / 32)
-      if (p0 + i < j.P && c < j.Cp) dst[(n * j.P + p0 + i) * j.Cp + c] = tile[tx * 33 + i];
+      if (p0 + i < j.P && c < j.Cp) {
+        T* at = dst + copy_dst_pixel(j, n, p0 + i) * j.Cp + c;
+        *at = tile[tx * 33 + i];
+        copy_pad<T, T>(j, at, p0 + i);
+      }
   }
 }
 

@@ -394,6 +394,21 @@ int pick_chunk_bytes(long long row_bytes) {
   return chunk;
 }
 
+// Whether the S taps of a filter row, as one run of channels, take fewer k-chunks than tap by tap -- a k-chunk is a copy of
+// either operand, and with few channels those are what a walk takes its time for; returns the channels per pixel of that form, 0
+// if not. Pixels start on 32-byte sectors where that takes no chunk more (40 channels would: 15.2 us exact, 21.7 rounded up;
+// 24 channels 15.4 and 13.6). NCHW calls, tap by tap and by filter rows, us: 5x5 20->50 + GELU on 3 images of 72x72 19.0 and
+// 13.2; 3x3 20->50 13.9 and 11.7; 3x3 40->64 on 8 images of 56x56 20.8 and 15.2; 3x3 80->128 on 8 of 28x28 13.3 and 12.4; 5x5
+// 48->96 36.7 and 29.7; 7x7/2 12->64 fp32 on 8 of 112x112 43.7 and 23.3; 3x3 104->128 on 32 of 28x28 26.5 and 23.6.
+long long filter_row_channels(long long Cp, int es, long long S) {
+  if (S < 2 || S > 16) return 0;
+  auto chunks = [](long long bytes) { const int c = pick_chunk_bytes(bytes); return (bytes + c - 1) / c; };
+  const long long aligned = (Cp * es + 31) / 32 * 32 / es;
+  const long long by_tap = S * chunks(Cp * es), exact = chunks(S * Cp * es), wide = chunks(S * aligned * es);
+  if (std::min(exact, wide) >= by_tap) return 0;
+  return wide <= exact ? aligned : Cp;
+}
+
 int pick_stages(int bn, bool pair, bool rows2, int staging_depth, int bias_bytes) {
   const int fixed = tb200::conv_smem_bytes(bn, 0, pair, rows2, staging_depth, bias_bytes);
   const int stage_bytes = tb200::conv_smem_bytes(bn, 1, pair, rows2, staging_depth, bias_bytes) - fixed;
@@ -612,17 +627,19 @@ NoAllocState& noalloc_state(int dev) {
 }
 
 // ------------------------------------------------------------------ layout adapters
-// src[n, c, h, w] through element strides -> dst[n][h * W + w][Cp], channels C .. Cp-1 zero-filled. The mode is the widest
-// access both sides allow: see CopyJob.
+// src[n, c, h, w] through element strides -> dst[n][h * W + w][Cp], channels C .. Cp-1 zero-filled, or with zero pixels
+// around every row, dst[n][h][pad_lo + w][Cp]. The mode is the widest access both sides allow: see CopyJob.
 tb200::CopyJob copy_job(const void* src, void* dst, int es, long long N, long long C, long long Cp, long long H, long long W,
-                        long long sn, long long sc, long long sh, long long sw) {
-  if (H * W == 1) {   // a matrix: its rows are the pixels of one image
+                        long long sn, long long sc, long long sh, long long sw, long long pad_lo = 0, long long pad_hi = 0) {
+  const bool padded = pad_lo + pad_hi > 0;
+  if (H * W == 1 && !padded) {   // a matrix: its rows are the pixels of one image
     W = N; sw = sn; sh = 0; N = 1; sn = 0;
   }
   tb200::CopyJob j;
   memset(&j, 0, sizeof(j));
   j.src = src; j.dst = dst;
   j.N = N; j.C = (int)C; j.Cp = (int)Cp; j.P = (int)(H * W); j.W = (int)W;
+  j.pad_lo = (int)pad_lo; j.pad_hi = (int)pad_hi;
   j.sn = sn; j.sc = sc; j.sh = sh; j.sw = sw;
   j.vec = 1;
   const long long P = H * W, chunk = 16 / es;
@@ -633,7 +650,7 @@ tb200::CopyJob copy_job(const void* src, void* dst, int es, long long N, long lo
   } else if (sc == 1 || C == 1) {
     j.mode = tb200::kCopyRows;
     if (es == 2 && C > 1 && C % 2 == 0 && addr % 4 == 0 && sn % 2 == 0 && sh % 2 == 0 && sw % 2 == 0) j.vec = 2;
-  } else if (planar && P <= tb200::kCopyMaxTaps && sc == P && N > 1) {
+  } else if (planar && P <= tb200::kCopyMaxTaps && sc == P && N > 1 && !padded) {
     j.mode = tb200::kCopyTaps;
   } else if (planar) {
     j.mode = tb200::kCopyPlanes;
@@ -1150,30 +1167,42 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   // cost it nearly twice the time (3x3 C->128 on 32 images of 28x28: C = 104 25.1 us, C = 112 13.9).
   long long Cs = Cp * es > 16 ? (Cp * es + 31) / 32 * 32 / es : Cp;
   // (the built-in scratch of the no-alloc entry is small: there the padding is left out when only that makes the copies fit)
-  if (arena != nullptr && arena->used + (N * H * W + K * R * S) * Cs * es + 1024 > static_cast<long long>(arena->capacity)) Cs = Cp;
+  auto scratch_holds = [&](long long elems) {
+    return arena == nullptr || static_cast<long long>(arena->used) + elems * es + 1024 <= static_cast<long long>(arena->capacity);
+  };
+  if (!scratch_holds((N * H * W + K * R * S) * Cs)) Cs = Cp;
+  // ---- whole filter rows as k-chunks (see filter_rows_pay): the staged copy carries its horizontal padding, so the S taps of
+  // a filter row are S adjacent pixels, one run of S * Cr channels that the k-chunks cut without regard to the taps
+  const long long W_padded = W + static_cast<long long>(p.padding_w) + p.pad_w_hi;
+  const long long Cr = filter_row_channels(Cp, es, S);
+  const bool frow = stage_x && Cr != 0 && p.dilation_w == 1 && W_padded < (1LL << 30) && knobs().force_chunk == 0 &&
+                    scratch_holds((N * H * W_padded + K * R * S) * Cr);
+  if (frow) Cs = Cr;
   if (stage_x) {   // its address is filled in below, where the weights' form is known too
-    x.stride[0] = H * W * Cs;
+    const long long row = (frow ? W_padded : W) * Cs;
+    x.stride[0] = H * row;
     x.stride[1] = 1;
-    x.stride[2] = W * Cs;
+    x.stride[2] = row;
     x.stride[3] = Cs;
   }
 
   // ---- k-chunking: how many bytes of one pixel's channels one copy brings in (see pick_chunk_bytes)
-  // In window mode the kernel sees a conv with one tap per filter row over "pixels" of 8 * Cp channels.
-  const long long Cg = window ? 8 * Cp : Cp;      // channel extent of the kernel's view
-  const long long Sg = window ? 1 : S;            // taps per filter row of the kernel's view
+  // In window mode the kernel sees a conv with one tap per filter row over "pixels" of 8 * Cp channels, with filter rows as
+  // k-chunks one over "pixels" of S * Cr.
+  const long long Cg = window ? 8 * Cp : (frow ? S * Cr : Cp);   // channel extent of the kernel's view
+  const long long Sg = window || frow ? 1 : S;                   // taps per filter row of the kernel's view
   const long long row_bytes = Cg * es;
   int chunk_bytes = pick_chunk_bytes(row_bytes);
   const int forced_chunk = knobs().force_chunk;
   if (forced_chunk == 16 || forced_chunk == 32 || forced_chunk == 64 || forced_chunk == 128) chunk_bytes = forced_chunk;
   const int chunk_elems = chunk_bytes / es;
   const int chunks_per_tap = static_cast<int>((Cg + chunk_elems - 1) / chunk_elems);
-  const bool w_dense = C == Cp && (w_in.stride[1] == 1) && w_in.stride[3] == C &&
+  const bool w_dense = C == Cp && (!frow || Cr == Cp) && (w_in.stride[1] == 1) && w_in.stride[3] == C &&
                        w_in.stride[2] == S * C && w_in.stride[0] == R * S * C && aligned16(w_in.ptr);
   // Where the last chunk of a tap is partly past the channels, the TMA unit fills the activations' channels >= C with zeros,
   // but the weights need a map with one row per tap, unless there is only one tap. So do weights that are repacked with
   // padded taps, whatever the chunk (chunks that divide an unpadded tap then only come from TRACEA_B200_FORCE_CHUNK).
-  const bool ragged_taps = (row_bytes % chunk_bytes != 0 || (!w_dense && !window && Cs != Cp)) && R * Sg > 1;
+  const bool ragged_taps = (row_bytes % chunk_bytes != 0 || (!w_dense && !window && !frow && Cs != Cp)) && R * Sg > 1;
   const long long total_chunks_ll = R * Sg * chunks_per_tap;
   if (total_chunks_ll > 0x7fffffffLL / 128) TB_FAIL(TRACEA_UNSUPPORTED_CONFIG, "R*S*C too large");
 
@@ -1186,7 +1215,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   Scratch op_scratch;
   long long w_row_elems = R * S * C, w_pitch = R * S * C, b_k0 = 0, b_jump_s = 0, b_jump_r = 0;
   bool w_direct = w_dense, w_remap = false;
-  if (!w_dense && !window && C == Cp && w_in.stride[1] == 1 && chunk_bytes == 128 && !ragged_taps) {
+  if (!w_dense && !window && !frow && C == Cp && w_in.stride[1] == 1 && chunk_bytes == 128 && !ragged_taps) {
     const long long ss = S == 1 ? C : w_in.stride[3], sr = R == 1 ? S * ss : w_in.stride[2], sk = w_in.stride[0];
     const long long lo = std::min(0LL, (R - 1) * sr) + std::min(0LL, (S - 1) * ss);
     const long long hi = std::max(0LL, (R - 1) * sr) + std::max(0LL, (S - 1) * ss) + C;
@@ -1215,7 +1244,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   {
     // one block of scratch and one launch for both operands
     const long long Sd = window ? 8 : S;   // tap slots per filter row in the packed weights
-    const size_t x_bytes = stage_x ? (static_cast<size_t>(N * H * W * Cs) * es + 255) / 256 * 256 : 0;
+    const size_t x_bytes = stage_x ? (static_cast<size_t>(N * x.stride[0]) * es + 255) / 256 * 256 : 0;
     const size_t w_bytes = stage_w ? static_cast<size_t>(K * R * Sd * (window ? Cp : Cs)) * es : 0;
     tb200::CopyJob jobs[2];
     int count = 0;
@@ -1224,7 +1253,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
       if (stage_x) {
         x.ptr = base;
         jobs[count++] = copy_job(x_in.ptr, x.ptr, es, N, C, Cs, H, W, x_in.stride[0], x_in.stride[1], x_in.stride[2],
-                                 x_in.stride[3]);
+                                 x_in.stride[3], frow ? p.padding_w : 0, frow ? p.pad_w_hi : 0);
       }
       if (stage_w) {
         w_ptr = base + x_bytes;
@@ -1241,7 +1270,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   {
     const bool ovec = (out.stride[1] == 1) && aligned16(out.ptr) && (out.stride[0] * es) % 16 == 0 &&
                       (out.stride[2] * es) % 16 == 0 && (out.stride[3] * es) % 16 == 0 && (K % vec_elems) == 0;
-    if (!window && !w_remap && Cp == 64 && C == 64 && st.status != nullptr &&
+    if (!window && !frow && !w_remap && Cp == 64 && C == 64 && st.status != nullptr &&
         try_resident_filter_conv(st, x, w_ptr, bias, out, p, epi, K, R, S, ovec, stream))
       return;
   }
@@ -1332,13 +1361,14 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     if (r != CUDA_SUCCESS) TB_FAIL(TRACEA_CUDA_ERROR, "cuTensorMapEncodeTiled (A) failed with %d", (int)r);
   } else {
     // window mode: "pixel" w of the view starts at padded pixel w and spans 8 of them (pitch 16 B, extent
-    // 128 B, overlapping); the horizontal padding is in memory, so the W corners only trim the filter width
-    const cuuint64_t gdim[4] = {(cuuint64_t)Cg, (cuuint64_t)(window ? W + 2LL * p.padding_w : W), (cuuint64_t)H,
-                                (cuuint64_t)N};
+    // 128 B, overlapping); filter rows as k-chunks: it spans S of them. The horizontal padding is in memory then, so the W
+    // corners only trim the filter width
+    const bool wide_pixels = window || frow;
+    const cuuint64_t gdim[4] = {(cuuint64_t)Cg, (cuuint64_t)(wide_pixels ? W_padded : W), (cuuint64_t)H, (cuuint64_t)N};
     const cuuint64_t gstr[3] = {(cuuint64_t)(x.stride[3] * es), (cuuint64_t)(x.stride[2] * es),
                                 (cuuint64_t)(x.stride[0] * es)};
-    const int lower[2] = {window ? 0 : -(int)p.padding_w, -(int)p.padding_h};
-    const int upper[2] = {window ? -(int)(S - 1) : (int)p.pad_w_hi - (int)((S - 1) * p.dilation_w),
+    const int lower[2] = {wide_pixels ? 0 : -(int)p.padding_w, -(int)p.padding_h};
+    const int upper[2] = {wide_pixels ? -(int)(S - 1) : (int)p.pad_w_hi - (int)((S - 1) * p.dilation_w),
                           (int)p.pad_h_hi - (int)((R - 1) * p.dilation_h)};
     const cuuint32_t estr[4] = {1u, p.stride_w, p.stride_h, 1u};
     CUresult r = g_encode_im2col(&tmap_x, tmap_dtype(x.dtype), 4, x.ptr, gdim, gstr, lower, upper,
@@ -1363,7 +1393,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   a.stride_h = p.stride_h;
   a.stride_w = p.stride_w;
   a.pad_h = p.padding_h;
-  a.pad_w = window ? 0 : p.padding_w;
+  a.pad_w = window || frow ? 0 : p.padding_w;
   a.dil_h = p.dilation_h;
   a.dil_w = p.dilation_w;
   a.S = static_cast<int>(Sg);
@@ -1523,7 +1553,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     // {column, tap, output channel}. Repacked or dense weights: one row is the whole Kgemm axis, or one tap of it when
     // the k-chunks do not divide a tap; in-place strided taps: one row spans the taps
     const long long row_elems = w_remap ? w_row_elems : (ragged_taps ? Cg : Kgemm);
-    const long long tap_pitch = stage_w && !window ? Cs : Cg;
+    const long long tap_pitch = stage_w && !window && !frow ? Cs : Cg;
     const long long k_pitch = w_remap ? w_pitch : R * Sg * tap_pitch;
     const cuuint64_t gdim[3] = {(cuuint64_t)row_elems, (cuuint64_t)(ragged_taps ? R * Sg : 1), (cuuint64_t)K};
     const cuuint64_t gstr[2] = {(cuuint64_t)((ragged_taps ? tap_pitch : k_pitch) * es), (cuuint64_t)(k_pitch * es)};
