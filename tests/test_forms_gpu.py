@@ -97,3 +97,31 @@ def test_filter_rows_in_the_phases_of_a_transposed_convolution(dtype):
         want = torch.nn.functional.conv_transpose2d(x.double().permute(0, 3, 1, 2), w.double().permute(3, 0, 1, 2), stride=stride,
                                                     padding=pad, output_padding=opad).permute(0, 2, 3, 1)
         assert float((got.double() - want).abs().max() / want.abs().max()) <= cc.tol_for(dtype)
+
+
+# 32-wide small tiles whatever the number of k-steps: walks longer than the 31 steps up to which they used to be chosen, bit for bit against
+# the general kernel; pixels that do not start on 32-byte sectors keep it beyond a few tiles.
+LONG_WALKS = [(1, 256, 14, 14, 256, 3, 1, 1, "bias+relu", True), (2, 512, 7, 7, 520, 3, 1, 1, "bias+residual+relu", True),
+              (1, 128, 20, 20, 96, 5, 1, 2, "gelu", False), (3, 320, 9, 7, 33, 3, 2, 1, "bias", True)]
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+def test_small_tiles_for_long_walks(dtype, tmp_path):
+    got = []
+    for case in LONG_WALKS:
+        before = ffi.launch_count_of(ffi.KERNEL_SMALL_TILE)
+        got.append(check(case, dtype))
+        assert ffi.launch_count_of(ffi.KERNEL_SMALL_TILE) == before + 1, case
+    before = ffi.launch_count_of(ffi.KERNEL_GENERAL)
+    check((93, 120 if dtype != "f32" else 124, 12, 12, 128, 3, 2, 1, "bias+silu", True), dtype)
+    assert ffi.launch_count_of(ffi.KERNEL_GENERAL) == before + 1
+    here = os.path.dirname(os.path.abspath(__file__))
+    out = str(tmp_path / "general.npz")
+    code = ("import sys; sys.path.insert(0, %r); sys.path.insert(0, %r)\n"
+            "import numpy as np, test_forms_gpu as t\n"
+            "np.savez(%r, *[t.conv(c, %r)[0].float().cpu().numpy() for c in t.LONG_WALKS])\n"
+            "assert t.ffi.launch_count_of(t.ffi.KERNEL_SMALL_TILE) == 0\n" % (os.path.dirname(here), here, out, dtype))
+    subprocess.run([sys.executable, "-c", code], check=True, env=dict(os.environ, TRACEA_B200_FORCE_BN="64"), timeout=300)
+    general = np.load(out)
+    for i, g in enumerate(got):
+        assert np.array_equal(general["arr_%d" % i], g.float().cpu().numpy()), LONG_WALKS[i]

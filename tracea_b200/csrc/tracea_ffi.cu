@@ -1299,10 +1299,13 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
 
   // ---- problems of up to one wave: the small-tile kernel (conv2d_small_sm100.cuh). Where two k-steps come in one copy per
   // operand -- 1x1 convolutions and products over whole 128-byte chunks -- a k-step takes it about half the general kernel's
-  // time (2048 -> 512 channels on one 7x7 image 8.5 -> 5.2 us, 64 x 1000 x 2048 8.7 -> 5.3); with im2col copies its step is
-  // put above the general kernel's, so that the microsecond that its launch is shorter by pays for about 30 of them. (3x3, one
-  // image: 64 channels 5.3 -> 3.8, 128 channels 6.7 -> 4.7, 192 channels, 27 steps, 8.0 -> 5.6: the 360 and 410 below, from an
-  // earlier build in which 256 channels lost, 9.3 -> 9.6, look too high and have not been measured again.) More than one tile
+  // time (2048 -> 512 channels on one 7x7 image 8.5 -> 5.2 us, 64 x 1000 x 2048 8.7 -> 5.3). With im2col copies a step is
+  // 215-270 cycles against 300 and more: 32-wide tiles win whatever the number of steps (bf16, 3x3: 256 channels on one / four
+  // 14x14 images 9.2 -> 6.8 and 9.5 -> 7.3 us, 512 channels on one / eight 7x7 images 14.7 -> 11.1 and 15.2 -> 11.6; 5x5 128->128
+  // on two 28x28 images 12.4 -> 9.1). 64-wide ones win less the more of them there are (64->128 fp32 on six 28x28 images 7.1 ->
+  // 5.9, 256 channels on ten 14x14 images 9.7 -> 9.0): their step is put at 355, which leaves walks of more than 34 steps to the
+  // general kernel. Pixels that do not start on 32-byte sectors cost every copy sectors that it shares with its neighbours: 120
+  // channels, 106 / 144 tiles, 9.4 -> 10.3 and 9.6 -> 9.8; those keep the earlier costs. More than one tile
   // per SM gains nothing (1x1 64->64 at 4 images: 196 tiles, 3.65 -> 3.88). Costs in cycles.
   const bool whole_chunks = chunk_bytes == 128 && row_bytes % 128 == 0;
   const bool plain_a = whole_chunks && !window && R == 1 && S == 1 && p.stride_h == 1 && p.stride_w == 1 &&
@@ -1320,7 +1323,8 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     for (int b = 64; b >= 32; b >>= 1) {
       if (m_tiles_64 * ((K + b - 1) / b) > st.num_sms) continue;
       if (w_n_major && b < 64) continue;   // its columns come 64 at a time
-      const long long cost = k_steps * (plain_a ? (b == 32 ? 130 : 160) : (b == 32 ? 360 : 410));
+      const long long im2col = x.stride[3] * es % 32 == 0 ? (b == 32 ? 240 : 355) : (b == 32 ? 360 : 410);
+      const long long cost = k_steps * (plain_a ? (b == 32 ? 130 : 160) : im2col);
       if (cost < best) {
         best = cost;
         small_bn = b;
