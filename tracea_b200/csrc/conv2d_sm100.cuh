@@ -1170,8 +1170,12 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
     constexpr int kLdPerGroup = kGroupCols / 32;
     constexpr int kChunksPerLd = 32 / kVec;        // 16-byte chunks produced per 32-column TMEM load
     // with a shared copy every warp writes the same values to the same words before it reads them
-    float* bias_w = reinterpret_cast<float*>(smem_gen + bias_off) + (args.shared_bias >= 0 ? 0 : ew * BN);
-    uint32_t bias_w_s = smem_base + bias_off + (args.shared_bias >= 0 ? 0u : static_cast<uint32_t>(ew) * BN * 4u);
+    // the tile's columns of the shared copy start bias_step floats further down per column tile; every warp writes the same values
+    // there before it reads them
+    const int bias_slot = args.shared_bias >= 0 ? 0 : ew * BN;
+    const int bias_step = args.shared_bias > 0 ? args.shared_bias : 0;
+    float* bias_w = reinterpret_cast<float*>(smem_gen + bias_off) + bias_slot;
+    const uint32_t bias_w_s = smem_base + bias_off + static_cast<uint32_t>(bias_slot) * 4u;
     const uint32_t stg0 = staging_base + static_cast<uint32_t>(ew * args.staging_depth) * kStagingBoxBytes;
     const uint32_t box_flip = args.staging_depth == 2 ? 1u : 0u;
     // this lane's 16-byte chunk c of its staging row lives at row*128 + ((c ^ (row & 7)) << 4): the
@@ -1327,12 +1331,9 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
       // this warp's fp32 copy of the tile's bias (zeros when there is none / past K_out); the values
       // were fetched into registers during the previous tile, and the next tile's are fetched now
       if (n_tile != bias_tile) {
-        const int move = args.shared_bias > 0 ? (n_tile - max(bias_tile, 0)) * args.shared_bias : 0;   // to the tile's own columns
-        bias_w += move;
-        bias_w_s += static_cast<uint32_t>(move) * 4u;
         __syncwarp();
 #pragma unroll
-        for (int j = 0; j < kBiasPerLane; ++j) bias_w[j * 32 + lane] = bias_next[j];
+        for (int j = 0; j < kBiasPerLane; ++j) bias_w[n_tile * bias_step + j * 32 + lane] = bias_next[j];
         __syncwarp();
         bias_tile = n_tile;
       }
@@ -1456,7 +1457,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
           for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[h][j]);
 #pragma unroll
           for (int j4 = 0; j4 < 8; ++j4) {
-            const float4 b4 = ld_shared_f4(bias_w_s + static_cast<uint32_t>(g * kGroupCols + h * 32 + j4 * 4) * 4u);
+            const float4 b4 = ld_shared_f4(bias_w_s + static_cast<uint32_t>(n_tile * bias_step + g * kGroupCols + h * 32 + j4 * 4) * 4u);
             add2(f[j4 * 4 + 0], f[j4 * 4 + 1], b4.x, b4.y);
             add2(f[j4 * 4 + 2], f[j4 * 4 + 3], b4.z, b4.w);
           }
