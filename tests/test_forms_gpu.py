@@ -125,3 +125,14 @@ def test_small_tiles_for_long_walks(dtype, tmp_path):
     general = np.load(out)
     for i, g in enumerate(got):
         assert np.array_equal(general["arr_%d" % i], g.float().cpu().numpy()), LONG_WALKS[i]
+
+
+# The resident-filter kernel's tile height follows the number of tiles: heights for one to four blocks of pixels, with and without a
+# shorter tile at the bottom, odd tile counts.
+@pytest.mark.parametrize("case", [(32, 64, 56, 56, 64, 3, 1, 1, "bias+relu", True), (21, 64, 56, 56, 48, 3, 1, 1, "silu", True),
+                                  (39, 64, 40, 40, 64, 3, 1, 1, "bias", True), (37, 64, 37, 46, 56, 3, 1, 1, "gelu", True),
+                                  (13, 64, 112, 112, 64, 3, 1, 1, "relu", True), (80, 64, 56, 56, 8, 3, 1, 1, "bias", True)])
+def test_resident_filter_tile_heights(case):
+    before = ffi.launch_count_of(ffi.KERNEL_RESIDENT_FILTER)
+    check(case, "bf16")
+    assert ffi.launch_count_of(ffi.KERNEL_RESIDENT_FILTER) == before + 1

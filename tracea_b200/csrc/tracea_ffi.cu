@@ -972,28 +972,54 @@ bool try_resident_filter_conv(DeviceState& st, const View4& x, const void* w_ptr
   const long long Wp = W + p.padding_w, dummy = Wp - Wo;
   if (dummy < 0) return false;
   const uint32_t w_bytes = static_cast<uint32_t>(R * S) * 4096u;
-  long long ht = 0, nblk = 0, slot_bytes = 0, box_rows = 0;
-  for (long long nb = tb200::kWinMaxBlocks; nb >= 1; --nb) {
-    long long h = std::min<long long>((128 * nb + dummy) / Wp, Ho);
-    if (h < 1 || h + R - 1 > 256) continue;
-    const long long rows = (h + R - 1) * Wp;                            // what a window copy fills
-    const long long reach = 128 * nb + (R - 1) * Wp + (S - 1);         // what the MMAs of nb blocks read
-    const long long slot = (std::max(rows + p.pad_w_hi, reach) * 128 + 1023) / 1024 * 1024;
-    if (tb200::window_smem_bytes(w_bytes, static_cast<uint32_t>(slot)) > 232448u) continue;
-    ht = h; nblk = nb; slot_bytes = slot; box_rows = rows;
-    break;
-  }
-  if (ht == 0) return false;
-  const long long nblk_full = (ht * Wp - dummy + 127) / 128;
-  const long long tiles_per_img = Ho / ht, ht_short = Ho % ht;
-  const long long nblk_short = ht_short > 0 ? (ht_short * Wp - dummy + 127) / 128 : 0;
+  // Rows of a tile: what up to kWinMaxBlocks blocks of 128 pixels hold.
+  struct Plan {
+    long long ht, slot_bytes, box_rows, nblk_full, tiles_per_img, ht_short, nblk_short, n_full, n_short, pair_full, pair_tiles;
+  };
+  auto plan = [&](long long nb, Plan& q) {
+    q.ht = std::min<long long>((128 * nb + dummy) / Wp, Ho);
+    if (q.ht < 1 || q.ht + R - 1 > 256) return false;
+    q.box_rows = (q.ht + R - 1) * Wp;                                   // what a window copy fills
+    const long long reach = 128 * nb + (R - 1) * Wp + (S - 1);          // what the MMAs of nb blocks read
+    q.slot_bytes = (std::max(q.box_rows + p.pad_w_hi, reach) * 128 + 1023) / 1024 * 1024;
+    if (tb200::window_smem_bytes(w_bytes, static_cast<uint32_t>(q.slot_bytes)) > 232448u) return false;
+    q.nblk_full = (q.ht * Wp - dummy + 127) / 128;
+    q.tiles_per_img = Ho / q.ht;
+    q.ht_short = Ho % q.ht;
+    q.nblk_short = q.ht_short > 0 ? (q.ht_short * Wp - dummy + 127) / 128 : 0;
+    q.n_full = N * q.tiles_per_img;
+    q.n_short = q.ht_short > 0 ? N : 0;
+    q.pair_full = (q.n_full + 1) / 2;
+    q.pair_tiles = q.pair_full + (q.n_short + 1) / 2;
+    return true;
+  };
+  Plan q;
+  long long nb = tb200::kWinMaxBlocks;
+  while (nb >= 1 && !plan(nb, q)) --nb;
+  if (nb < 1) return false;
   // worth it only when the 128-row MMA blocks are mostly real pixels and the launch fills the GPU at least once
-  const long long blocks_per_img = tiles_per_img * nblk_full + nblk_short;
-  if (Ho * Wo * 100 < blocks_per_img * 128 * 85) return false;
-  const long long n_full = N * tiles_per_img, n_short = ht_short > 0 ? N : 0;
-  const long long pair_full = (n_full + 1) / 2, pair_tiles = pair_full + (n_short + 1) / 2;
-  if (pair_tiles < st.num_sms / 2 || pair_tiles > 0x3fffffffLL) return false;
-  (void)nblk;
+  const long long pairs = st.num_sms / 2;
+  if (Ho * Wo * 100 < (q.tiles_per_img * q.nblk_full + q.nblk_short) * 128 * 85) return false;
+  if (q.pair_tiles < pairs || q.pair_tiles > 0x3fffffffLL) return false;
+  // Tall tiles read the least halo, but few of them leave pairs idle, and what runs before the first tile's epilogue grows with a
+  // tile: shorter ones where that shortens the busiest pair's walk, in cycles -- 3800 for a block's epilogue, two blocks at a
+  // time, the first window's copy and the first tile's MMAs on top. Measured with nine taps; with four, where epilogues compete
+  // with fewer MMAs, shorter tiles lose (2x2 on 80 images of 56x56: 20.5 -> 23.2 us). (3x3 64->64, tiles of 9 and 4 rows at
+  // 56x56 on 32 images 15.1 and 13.4 us, of 12 and 6 rows at 40x40 on 40 images 12.0 and 10.9; on 64 images of 56x56 both take
+  // 18.6.)
+  auto cost = [&](const Plan& v) {
+    const long long block = 3800, full = (v.nblk_full + 1) / 2 * block, part = (v.nblk_short + 1) / 2 * block;
+    const long long busiest = (v.pair_full + pairs - 1) / pairs * full;
+    const long long mean = (v.pair_full * full + (v.pair_tiles - v.pair_full) * part + pairs - 1) / pairs;
+    return std::max(busiest, mean) + v.box_rows * 128 / 80 + v.nblk_full * 1550;
+  };
+  for (long long k = nb - 1; k >= 1 && R * S == 9; --k) {
+    Plan v;
+    if (plan(k, v) && v.pair_tiles <= 0x3fffffffLL && cost(v) * 100 < cost(q) * 96) q = v;
+  }
+  const long long ht = q.ht, slot_bytes = q.slot_bytes, box_rows = q.box_rows, nblk_full = q.nblk_full, ht_short = q.ht_short,
+                  nblk_short = q.nblk_short, tiles_per_img = q.tiles_per_img, n_full = q.n_full, n_short = q.n_short,
+                  pair_full = q.pair_full, pair_tiles = q.pair_tiles;
 
   auto encode_x = [&](CUtensorMap* m, long long box_h) {
     const int es = 2;
