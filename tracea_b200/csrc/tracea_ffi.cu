@@ -359,24 +359,59 @@ const Knobs& knobs() {
 }
 
 // ------------------------------------------------------------------ tile selection
-// Relative cost of one 128-byte k-step of a 128-row x BN tile on one SM, measured on the ResNet-50 layers rather
-// than derived: the tensor pipe alone would give 512 / 256 / 192 cycles (BN/2 per MMA, 48 at BN = 64 where the
-// shared-memory operand reads bind), but the narrower tiles pull (128 + BN) * 128 bytes per step through L2 -> SM
-// paths that deliver ~70 B/cycle/SM when every SM loads, so a BN = 128 step costs ~400 and a BN = 64 step ~300.
-// The widest tile wins ties: it re-reads A least. (Measured while one thread each issued the copies and the MMAs, at 420-505
-// cycles a stage; a stage issues in 290-320 now, and the costs have not been measured again.)
-int pick_bn(long long m_tiles, int k_out, int num_sms) {
-  const int bns[3] = {256, 128, 64};
-  const int step_cost[3] = {512, 400, 300};
+struct Tiling {
+  int bn = 64;
+  bool pair = false, rows2 = false;
+};
+
+// The tiling of the general kernel with the shortest walk of the busiest CTA (or pair), in cycles:
+//  * a k-step (128 bytes of K) takes what its MMAs and copies take to issue, or, if that is more, what bringing in its operands
+//    takes: all SMs together get about 87 B/cycle/SM from L2, and fewer working SMs more each. Per step: 64 / 128 / 256
+//    columns 300 / 315 / 530 cycles for 24 / 32 / 48 KB, two row blocks of 64 / 128 columns 440 / 580 for 40 / 48 KB, a CTA
+//    of a pair 495 for 32 KB;
+//  * a tile hides the epilogue of the one before it (640 cycles per 128 bytes of columns, a quarter more with a residual, a fifth
+//    more for per-lane stores; two groups take alternate tiles, or a row block each), or waits for it, and costs 420 on top;
+//  * the first tile's walk and the last one's epilogue have nothing to hide them or hide behind; a pair costs 1040 once.
+// Two row blocks from 7 k-steps on and pairs from 8 on: below, the epilogue sets the pace, and both tie more of it together.
+// (Fitted to 91 layers and products in all six tilings; the pick is 0.9 % above the best of the six on average. The rule before it,
+// which only counted waves, took: 3x3 192->192 on 16 images of 28x28 13.9 -> 11.4 us, 1x1 512->2048 + residual on 64 of 7x7 12.4
+// -> 10.2, 1x1 64->256 on 8 NCHW images of 56x56 13.3 -> 11.1, 1x1 64->320 fp32 on 19 of 70x70 108 -> 72, 8192 x 512 x 512 8.8
+// -> 7.9, 1500 x 3072 x 768 10.4 -> 9.3.)
+Tiling pick_tiling(long long M, long long K_out, long long k_steps, int es, bool residual, bool per_lane, bool whole_stage,
+                   int num_sms, int forced_bn, int pair_env, int rows2_env) {
+  struct Form {
+    int bn;
+    bool pair, rows2;
+    int step, kbytes;
+  };
+  const Form forms[] = {{256, true, false, 495, 32}, {256, false, false, 530, 48}, {128, false, true, 580, 48},
+                        {128, false, false, 315, 32}, {64, false, true, 440, 40},  {64, false, false, 300, 24}};
+  Tiling best;
   long long best_cost = -1;
-  int best = 64;
-  for (int i = 0; i < 3; ++i) {
-    const long long n_tiles = (k_out + bns[i] - 1) / bns[i];
-    const long long waves = (m_tiles * n_tiles + num_sms - 1) / num_sms;
-    const long long cost = waves * step_cost[i];
+  for (const Form& f : forms) {
+    if (forced_bn != 0 && f.bn != forced_bn) continue;
+    if ((f.pair || f.rows2) && !whole_stage) continue;          // narrow k-chunks: several copies a stage
+    if (f.pair && (num_sms < 2 || pair_env == 0 || (pair_env != 1 && k_steps < 8))) continue;
+    if (f.rows2 && (rows2_env == 0 || (rows2_env != 1 && k_steps < 7))) continue;
+    // a form that was asked for is taken wherever it fits
+    if (!f.pair && f.bn == 256 && pair_env == 1 && whole_stage && num_sms >= 2) continue;
+    if (!f.rows2 && f.bn <= 128 && rows2_env == 1 && whole_stage) continue;
+    const long long rows = f.pair || f.rows2 ? 2 * tb200::kBlockM : tb200::kBlockM;
+    const long long tiles = (M + rows - 1) / rows * ((K_out + f.bn - 1) / f.bn);
+    const long long workers = f.pair ? num_sms / 2 : num_sms;
+    const long long waves = (tiles + workers - 1) / workers;
+    const long long busy = std::min<long long>(num_sms, tiles * (f.pair ? 2 : 1) / waves);
+    const long long walk = k_steps * std::max<long long>(f.step, f.kbytes * 1024 * busy / (87LL * num_sms));
+    long long epi = 640LL * f.bn * es / 128;
+    if (residual) epi = epi * 5 / 4;
+    if (per_lane) epi = epi * 6 / 5;
+    if (!f.rows2) epi /= 2;
+    const long long cost = (f.pair ? 1040 : 0) + waves * (std::max(walk, epi) + 420) + std::min(walk, epi) + epi * 4 / 5;
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
-      best = bns[i];
+      best.bn = f.bn;
+      best.pair = f.pair;
+      best.rows2 = f.rows2;
     }
   }
   return best;
@@ -481,8 +516,7 @@ void launch_tiling(DeviceState& st, int dt_idx, int bn, bool pair, bool rows2, c
     return;
   }
   if (pair) {
-    if (bn == 128) launch_one<OutT, 128, true, false, kStore>(st, dt_idx, 1, tx, tw, to, tr, args, grid, smem, stream);
-    else launch_one<OutT, 256, true, false, kStore>(st, dt_idx, 2, tx, tw, to, tr, args, grid, smem, stream);
+    launch_one<OutT, 256, true, false, kStore>(st, dt_idx, 2, tx, tw, to, tr, args, grid, smem, stream);
     return;
   }
   switch (bn) {
@@ -1301,27 +1335,17 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
       return;
   }
 
-  // ---- tiling of the whole problem
+  // ---- tiling of the whole problem. TRACEA_B200_FORCE_BN / _PAIR / _ROWS2 narrow the choice.
   const long long m_tiles_128 = (M + tb200::kBlockM - 1) / tb200::kBlockM;
-  int bn = pick_bn(m_tiles_128, static_cast<int>(K), st.num_sms);
-  const int forced_bn = knobs().force_bn;
-  if (forced_bn == 64 || forced_bn == 128 || forced_bn == 256) bn = forced_bn;
-  // CTA pairs (cta_group::2): a pair of SMs owns a 256 x bn tile and each CTA brings in only half of B's rows
-  // Worth it when the main loop is long enough to dominate the tile (>= 8 k-steps); short-K, epilogue-bound
-  // layers lose more from coupling two SMs' epilogues than they gain. TRACEA_B200_PAIR=0/1 forces the choice.
-  const int pair_env = knobs().pair;
-  const bool pair_ok = chunk_bytes == 128 && bn == 256 && st.num_sms >= 2;
-  const bool pair = pair_ok && (pair_env == 1 || (pair_env != 0 && total_chunks_ll >= 8));
-  // Two row blocks per CTA for narrow outputs (bn <= 128): twice the tensor work per barrier probe and per tile.
-  const int rows2_env = knobs().rows2;
-  // A 256-row tile costs an SM about 1.6x what a 128-row tile costs it (measured with the issue loops that pick_bn's costs
-  // are from; the narrow tile was bound by the shared-memory fill rate, which B's reuse across two row blocks relieves):
-  // taken when it shortens the launch, wave quantisation included.
+  const int forced_bn = knobs().force_bn == 64 || knobs().force_bn == 128 || knobs().force_bn == 256 ? knobs().force_bn : 0;
+  const int pair_env = knobs().pair, rows2_env = knobs().rows2;
+  const Tiling tiling = pick_tiling(M, K, (total_chunks_ll * chunk_bytes + 127) / 128, es, epi.residual, out.stride[1] != 1,
+                                    chunk_bytes == 128, st.num_sms, forced_bn, pair_env, rows2_env);
+  const int bn = tiling.bn;
+  const bool pair = tiling.pair, rows2 = tiling.rows2;
   const long long n_tiles = (K + bn - 1) / bn;
   const long long waves_128 = (m_tiles_128 * n_tiles + st.num_sms - 1) / st.num_sms;
   const long long waves_256 = ((m_tiles_128 + 1) / 2 * n_tiles + st.num_sms - 1) / st.num_sms;
-  const bool rows2 = !pair && chunk_bytes == 128 && bn <= 128 && rows2_env != 0 &&
-                     (rows2_env == 1 || (total_chunks_ll >= 7 && 8 * waves_256 < 5 * waves_128));
 
   // ---- problems of up to one wave: the small-tile kernel (conv2d_small_sm100.cuh). Where two k-steps come in one copy per
   // operand -- 1x1 convolutions and products over whole 128-byte chunks -- a k-step takes it about half the general kernel's
