@@ -136,3 +136,15 @@ def test_resident_filter_tile_heights(case):
     before = ffi.launch_count_of(ffi.KERNEL_RESIDENT_FILTER)
     check(case, "bf16")
     assert ffi.launch_count_of(ffi.KERNEL_RESIDENT_FILTER) == before + 1
+
+
+# The copy in front of the RGB stem: odd and even padding, rows that are no multiple of a block's eight, widths over and under a block's
+# 128 pixel pairs, images of a wider batch, rows that start on odd elements (the general copy).
+@pytest.mark.parametrize("case", [(2, 3, 33, 160, 64, 7, 2, 3, "bias+relu", True), (3, 3, 21, 166, 48, 5, 2, 2, "relu", True),
+                                  (1, 3, 40, 600, 64, 3, 2, 1, "bias", True), (5, 3, 17, 170, 16, 7, 2, 0, "bias", True),
+                                  (2, 3, 30, 165, 64, 7, 2, 3, "bias+relu", True)])
+def test_rgb_stem_copies(case):
+    before = ffi.launch_count_of(ffi.KERNEL_ROW_BAND)
+    check(case, "bf16")
+    check(case, "f16")
+    assert ffi.launch_count_of(ffi.KERNEL_ROW_BAND) == before + 2

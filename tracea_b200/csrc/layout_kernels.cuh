@@ -237,29 +237,6 @@ __global__ void to_channels_last_wpad_kernel(const T* __restrict__ src, T* __res
   else *reinterpret_cast<uint2*>(dst + i * kCp) = *reinterpret_cast<const uint2*>(v);   // 8-byte pixels (4 x 16 bit)
 }
 
-// The same padded copy for the one layout that matters in practice -- a dense channels-last RGB image of 16-bit
-// values (pixel pitch 3 elements) -> 4-channel pixels: a thread turns four source pixels (24 bytes, three 8-byte
-// loads) into four destination pixels (32 bytes, four 8-byte stores), and the threads past the image's width write
-// the zero pixels in front of and behind the row. One block per image row. `src_row` / `src_img`: element pitches.
-__global__ void rgb16_rows_to_padded4_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int H, int W,
-                                             int Wp, int pad, long long src_img, long long src_row) {
-  const long long row = blockIdx.x;                       // n * H + h
-  const long long n = row / H, h = row - n * H;
-  const uint2* __restrict__ s = reinterpret_cast<const uint2*>(src + n * src_img + h * src_row);
-  uint2* __restrict__ d = reinterpret_cast<uint2*>(dst + row * Wp * 4);
-  const int groups = W >> 2;
-  for (int t = threadIdx.x; t < groups; t += blockDim.x) {
-    const uint2 a = s[3 * t], b = s[3 * t + 1], c = s[3 * t + 2];   // words w0..w5 = elements e0..e11, two per word
-    uint2* o = d + pad + 4 * t;
-    o[0] = make_uint2(a.x, a.y & 0xffffu);
-    o[1] = make_uint2((a.y >> 16) | (b.x << 16), b.x >> 16);
-    o[2] = make_uint2(b.y, c.x & 0xffffu);
-    o[3] = make_uint2((c.x >> 16) | (c.y << 16), c.y >> 16);
-  }
-  const int zeros = Wp - W;                               // pad in front, the rest behind
-  for (int z = threadIdx.x; z < zeros; z += blockDim.x) d[z < pad ? z : W + z] = make_uint2(0u, 0u);
-}
-
 // w[k, c, r, s] (element strides) -> dst[k][r][s][Cp], zero-padded channels: the K-major B operand
 // whose Kgemm axis runs (r, s, c), the order the reference walks it (conv.rs:209-210).
 // `Sd` >= S is the number of tap slots per filter row in the destination (slots s >= S are zero).
@@ -276,6 +253,57 @@ __global__ void pack_weights_krsc_kernel(const T* __restrict__ src, T* __restric
   const int r = static_cast<int>(t % R);
   const long long k = t / R;
   dst[i] = (c < C && s < S) ? src[k * sk + c * sc + r * sr + s * ss] : T(0);
+}
+
+// The padded copy of a channels-last RGB image of 16-bit values (pixel pitch 3 elements) as 4-channel pixels, and its filter bank
+// packed [K][R][Sd][4], in one programmatic launch in front of the row-band kernel. Bound by the memory system: a thread turns the
+// source of two neighbouring destination pixels into one 16-byte store, so that a warp's store covers 512 consecutive bytes (as
+// four 8-byte stores a thread, 32 bytes apart, a store touched every sector a quarter at a time); kStemRows rows a block, their
+// loads in flight together. Pixels outside the image are zeros. Rows of the source start on 4-byte boundaries, W and Wp are even.
+constexpr int kStemThreads = 128, kStemRows = 8;
+struct StemCopy {
+  const uint16_t* src;
+  uint16_t* dst;
+  int H, W, Wp, pad, rows, image_blocks;   // rows: N * H
+  long long src_img, src_row;
+  const uint16_t* w;
+  uint16_t* w_dst;
+  int C, R, S, Sd, w_total;                // w_total: K * R * Sd * 4
+  long long sk, sc, sr, ss;
+};
+// Pixel i of a source row as {e0 | e1 << 16, e2}, zeros outside the row.
+__device__ __forceinline__ uint2 rgb16_pixel(const uint32_t* row, int i, int W) {
+  if (i < 0 || i >= W) return make_uint2(0u, 0u);
+  const uint32_t* w = row + ((3 * i) >> 1);
+  const uint32_t a = __ldg(w), b = __ldg(w + 1);
+  return (i & 1) != 0 ? make_uint2((a >> 16) | (b << 16), b >> 16) : make_uint2(a, b & 0xffffu);
+}
+__global__ void __launch_bounds__(kStemThreads) rgb16_stem_copy_kernel(const __grid_constant__ StemCopy c) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int tid = static_cast<int>(threadIdx.x);
+  if (static_cast<int>(blockIdx.x) >= c.image_blocks) {
+    const int i = (static_cast<int>(blockIdx.x) - c.image_blocks) * kStemThreads + tid;
+    if (i >= c.w_total) return;
+    const int ch = i & 3, s = (i >> 2) % c.Sd, t = (i >> 2) / c.Sd, r = t % c.R, k = t / c.R;
+    c.w_dst[i] = ch < c.C && s < c.S ? c.w[k * c.sk + ch * c.sc + r * c.sr + s * c.ss] : uint16_t(0);
+    return;
+  }
+  const int row0 = static_cast<int>(blockIdx.x) * kStemRows;
+  const int count = min(kStemRows, c.rows - row0);
+  const int n0 = row0 / c.H, h0 = row0 - n0 * c.H;
+  for (int j = tid; j < c.Wp / 2; j += kStemThreads) {
+    int n = n0, h = h0;
+    uint4* d = reinterpret_cast<uint4*>(c.dst + static_cast<long long>(row0) * c.Wp * 4) + j;
+#pragma unroll 4
+    for (int r = 0; r < count; ++r) {
+      const uint32_t* row = reinterpret_cast<const uint32_t*>(c.src + n * c.src_img + h * c.src_row);
+      const uint2 a = rgb16_pixel(row, 2 * j - c.pad, c.W), b = rgb16_pixel(row, 2 * j + 1 - c.pad, c.W);
+      *d = make_uint4(a.x, a.y, b.x, b.y);
+      d += c.Wp / 2;
+      if (++h == c.H) { h = 0; ++n; }
+    }
+  }
 }
 
 }  // namespace tb200

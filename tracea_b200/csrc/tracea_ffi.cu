@@ -833,17 +833,37 @@ bool try_row_band_conv(DeviceState& st, Staging&& staging, const View4& x, const
   Scratch x_scratch, w_scratch;
   const long long pixels = N * H * Wpitch;
   void* x_stage = staging(x_scratch, static_cast<size_t>(pixels * px_bytes), "the padded channels-last copy of x");
-  {
+  const long long Sd = kmma * 32 / px_bytes;               // tap slots per filter row in the packed bank
+  void* w_stage = staging(w_scratch, static_cast<size_t>(K * R * Sd * px_bytes), "the packed filter bank");
+  if (C == 3 && x.stride[1] == 1 && x.stride[3] == 3 && (W % 2) == 0 && (x.stride[2] % 2) == 0 && (x.stride[0] % 2) == 0 &&
+      (reinterpret_cast<uintptr_t>(x.ptr) % 4) == 0 && N * H <= 0x3fffffffLL) {
+    tb200::StemCopy c;
+    c.src = static_cast<const uint16_t*>(x.ptr);
+    c.dst = static_cast<uint16_t*>(x_stage);
+    c.H = (int)H; c.W = (int)W; c.Wp = (int)Wpitch; c.pad = (int)p.padding_w; c.rows = (int)(N * H);
+    c.image_blocks = (int)((N * H + tb200::kStemRows - 1) / tb200::kStemRows);
+    c.src_img = x.stride[0]; c.src_row = x.stride[2];
+    c.w = static_cast<const uint16_t*>(w.ptr);
+    c.w_dst = static_cast<uint16_t*>(w_stage);
+    c.C = (int)C; c.R = (int)R; c.S = (int)S; c.Sd = (int)Sd; c.w_total = (int)(K * R * Sd * 4);
+    c.sk = w.stride[0]; c.sc = w.stride[1]; c.sr = w.stride[2]; c.ss = w.stride[3];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(c.image_blocks + (c.w_total + tb200::kStemThreads - 1) / tb200::kStemThreads));
+    cfg.blockDim = dim3(tb200::kStemThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = knobs().pdl != 0 ? 1 : 0;
+    TB_CUDA(cudaLaunchKernelEx(&cfg, tb200::rgb16_stem_copy_kernel, c));
+    TB_CUDA(cudaGetLastError());
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    g_launches_by_kind[3].fetch_add(1, std::memory_order_relaxed);
+  } else {
     const int threads = 256;
     const unsigned blocks = static_cast<unsigned>((pixels + threads - 1) / threads);
-    const bool dense_rgb = C == 3 && x.stride[1] == 1 && x.stride[3] == 3 && (W % 4) == 0 && (x.stride[2] % 4) == 0 &&
-                           (x.stride[0] % 4) == 0 && (reinterpret_cast<uintptr_t>(x.ptr) % 8) == 0 &&
-                           N * H <= 0x7fffffffLL;
-    if (dense_rgb)
-      tb200::rgb16_rows_to_padded4_kernel<<<static_cast<unsigned>(N * H), 64, 0, stream>>>(
-          static_cast<const uint16_t*>(x.ptr), static_cast<uint16_t*>(x_stage), (int)H, (int)W, (int)Wpitch,
-          (int)p.padding_w, x.stride[0], x.stride[2]);
-    else if (Cw == 4)
+    if (Cw == 4)
       tb200::to_channels_last_wpad_kernel<uint16_t, 4><<<blocks, threads, 0, stream>>>(
           static_cast<const uint16_t*>(x.ptr), static_cast<uint16_t*>(x_stage), (int)C, (int)H, (int)W, (int)Wpitch,
           (int)p.padding_w, pixels, x.stride[0], x.stride[1], x.stride[2], x.stride[3]);
@@ -854,10 +874,8 @@ bool try_row_band_conv(DeviceState& st, Staging&& staging, const View4& x, const
     TB_CUDA(cudaGetLastError());
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     g_launches_by_kind[3].fetch_add(1, std::memory_order_relaxed);
+    launch_weight_pack(w.ptr, w_stage, 2, K, C, R, S, Sd, Cw, w.stride, stream);
   }
-  const long long Sd = kmma * 32 / px_bytes;               // tap slots per filter row in the packed bank
-  void* w_stage = staging(w_scratch, static_cast<size_t>(K * R * Sd * px_bytes), "the packed filter bank");
-  launch_weight_pack(w.ptr, w_stage, 2, K, C, R, S, Sd, Cw, w.stride, stream);
 
   CUtensorMap tmap_x;
   {
