@@ -129,15 +129,16 @@ TraceaStatus tracea_conv2d_v0(TraceaTensorView x, TraceaTensorView w, const Trac
  * callers cannot afford that: a serving process that handed every free byte of the GPU to its own
  * arena at start-up (a later allocation fails, or makes the arena give memory back), or a
  * latency-critical loop where an allocation's implicit synchronisation and driver locks are not
- * acceptable. This entry point does the same work with the staging area taken from a fixed
- * 16 MiB array that is part of the library's device image; it never calls cudaMalloc / cudaFree,
+ * acceptable. This entry point does the same work, to the bit, with the staging area taken from a fixed
+ * 64 MiB array that is part of the library's device image; it never calls cudaMalloc / cudaFree,
  * the pool allocator, or any library routine that allocates.
  *
  * Limits and rules:
  *   - x, w, b, residual and out must be device tensors (device_id >= 0); host views are rejected
  *     with INVALID_PARAMS, because staging them would need an allocation.
  *   - The channels-last copy of x plus the repacked w (each rounded up to 256 bytes) must fit in
- *     16 MiB; otherwise the call returns UNSUPPORTED_CONFIG and the message states the sizes.
+ *     16 MiB; otherwise the call returns UNSUPPORTED_CONFIG and the message states the sizes. (The array is
+ *     larger because the copy of x may carry its horizontal padding; that does not count.)
  *     Channels-last x and w need no staging at all and are accepted at any size.
  *   - The first call on each device looks up the array's device address (with that device made
  *     current); issue that first call before starting any stream capture.

@@ -82,6 +82,24 @@ def test_noalloc_entry_takes_every_copy_that_fits_its_scratch_without_row_paddin
     assert torch.equal(outs[0], outs[1])
 
 
+# Filter rows as k-chunks sum in another order than tap by tap: the same form at any size, or the bits change with the batch. The
+# first is a copy that is over 16 MiB with its padding (16.1 + 0.7 MB) and under without (16.0 + 0.7); the others straddle that
+# limit too, in the number of images.
+@pytest.mark.parametrize("dtype,N,C,H,W,K", [("f16", 1, 40, 400, 500, 352), ("f16", 430, 20, 28, 28, 50), ("bf16", 395, 24, 28, 28, 8),
+                                             ("f32", 180, 20, 31, 29, 16)])
+def test_noalloc_entry_keeps_the_order_of_summation_up_to_its_limit(dtype, N, C, H, W, K):
+    dt = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}[dtype]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn((N, C, H, W), generator=g, device="cuda").to(dt)
+    w = (torch.randn((K, C, 5, 5), generator=g, device="cuda") * 0.05).to(dt)
+    run = lambda e, t: _call(e, t, w, None, None, torch.empty((t.shape[0], K, H, W), dtype=dt, device="cuda"), 1, 2,
+                             ffi.EPILOGUE_IDENTITY)
+    want, got = run("tracea_conv2d", x), run("tracea_conv2d_noalloc", x)
+    assert torch.equal(got, want)
+    for e in ("tracea_conv2d", "tracea_conv2d_noalloc"):
+        assert torch.equal(run(e, x[N - 1:].clone()), want[N - 1:])
+
+
 def test_noalloc_entry_takes_no_memory_from_the_device_or_the_pool():
     """Steady state (the kernels of this shape have run once, so the driver has loaded them): across a call
     the device's free memory does not move and the library's scratch pool hands nothing out."""

@@ -429,19 +429,27 @@ int pick_chunk_bytes(long long row_bytes) {
   return chunk;
 }
 
+constexpr long long kFilterRowBankBytes = 16LL << 20;   // larger filter banks go tap by tap
+
 // Whether the S taps of a filter row, as one run of channels, take fewer k-chunks than tap by tap -- a k-chunk is a copy of
 // either operand, and with few channels those are what a walk takes its time for; returns the channels per pixel of that form, 0
 // if not. Pixels start on 32-byte sectors where that takes no chunk more (40 channels would: 15.2 us exact, 21.7 rounded up;
 // 24 channels 15.4 and 13.6). NCHW calls, tap by tap and by filter rows, us: 5x5 20->50 + GELU on 3 images of 72x72 19.0 and
 // 13.2; 3x3 20->50 13.9 and 11.7; 3x3 40->64 on 8 images of 56x56 20.8 and 15.2; 3x3 80->128 on 8 of 28x28 13.3 and 12.4; 5x5
 // 48->96 36.7 and 29.7; 7x7/2 12->64 fp32 on 8 of 112x112 43.7 and 23.3; 3x3 104->128 on 32 of 28x28 26.5 and 23.6.
-long long filter_row_channels(long long Cp, int es, long long S) {
-  if (S < 2 || S > 16) return 0;
+// The copy carries the padding, so on images a few pixels wide it grows: not where it doubles, nor by more than 256 bytes a
+// pixel for every three filter rows that share it (64 rows high, fp32: 104 channels 3x3, 1 / 2 / 3 / 4 pixels wide, tap by tap
+// 22.1 / 40.8 / 63.2 / 72.3 us and by filter rows 26.8 / 43.5 / 65.7 / 72.0; bf16 7x7, 1 pixel 40.6 and 54.6).
+// The answer depends on the layer alone, not on the number of images: another form is another order of summation.
+long long filter_row_channels(long long Cp, int es, long long R, long long S, long long K, long long W, long long W_padded) {
+  if (S < 2 || S > 16 || W_padded > 2 * W) return 0;
   auto chunks = [](long long bytes) { const int c = pick_chunk_bytes(bytes); return (bytes + c - 1) / c; };
   const long long aligned = (Cp * es + 31) / 32 * 32 / es;
   const long long by_tap = S * chunks(Cp * es), exact = chunks(S * Cp * es), wide = chunks(S * aligned * es);
   if (std::min(exact, wide) >= by_tap) return 0;
-  return wide <= exact ? aligned : Cp;
+  const long long Cr = wide <= exact ? aligned : Cp;
+  if (3 * (W_padded - W) * Cr * es > 256 * R * W || K * R * S * Cr * es > kFilterRowBankBytes) return 0;
+  return Cr;
 }
 
 int pick_stages(int bn, bool pair, bool rows2, int staging_depth, int bias_bytes) {
@@ -597,8 +605,13 @@ CUtensorMapSwizzle tmap_swizzle(int chunk_bytes) {
 // that entry point never has to ask the CUDA allocator for anything. Every GPU that loads the
 // library carries these bytes until the process exits. The symbol below is only a host-side
 // handle; the device address kernels must be given comes from cudaGetSymbolAddress (noalloc_state).
-constexpr size_t kStaticScratchBytes = 16u << 20;   // 16 MiB
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+// What a call may stage is 16 MiB, counted as plain channels-last copies. The array is larger because filter rows as k-chunks
+// (see filter_row_channels) take a wider copy of the same input: that form sums in another order, so whether a call takes it
+// must not depend on whether the wider copy still fits -- then neither the batch size nor the entry point changes a bit. The
+// wider copy is at most 8/3 of the plain one (twice the width, 48-byte pixels as 64-byte ones) plus a bank of kFilterRowBankBytes.
+constexpr size_t kStaticScratchBytes = 16u << 20;
+constexpr size_t kStaticScratchArrayBytes = 64u << 20;
+static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchArrayBytes];
 // Error words of the kernels tracea_conv2d_noalloc launches ({code, block, detail, 0}, first error wins). The
 // allocating path keeps its words in pinned host memory; this path may not allocate, so its words live in the
 // device image as well and tracea_b200_device_status copies them back on request.
@@ -607,15 +620,17 @@ static __device__ __align__(16) uint32_t g_noalloc_status[4];
 // Bump allocator over the static array for the duration of one call.
 struct StaticArena {
   unsigned char* base = nullptr;
-  size_t capacity = 0;
+  size_t capacity = 0;   // what may be staged
+  size_t size = 0;       // bytes there are
   size_t used = 0;
-  void* take(size_t bytes, const char* what) {
+  // `counted`: what the request counts as against `capacity`
+  void* take(size_t bytes, size_t counted, const char* what) {
     const size_t start = (used + 255u) & ~static_cast<size_t>(255u);
-    if (start + bytes > capacity)
+    if (start + counted > capacity || start + bytes > size)
       TB_FAIL(TRACEA_UNSUPPORTED_CONFIG,
               "tracea_conv2d_noalloc: staging %s needs %zu bytes on top of %zu already in use, but the "
               "built-in scratch holds %zu bytes; use tracea_conv2d or pass channels-last tensors",
-              what, bytes, start, capacity);
+              what, counted, start, capacity);
     used = start + bytes;
     return base + start;
   }
@@ -1003,6 +1018,7 @@ void conv2d_device_noalloc(int dev, const View4& x_in, const View4& w_in, const 
   StaticArena arena;
   arena.base = na.scratch;
   arena.capacity = kStaticScratchBytes;
+  arena.size = kStaticScratchArrayBytes;
   conv2d_core(st, &arena, x_in, w_in, bias, residual, out, p, epi);
 }
 
@@ -1178,9 +1194,9 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   cudaStream_t stream = static_cast<cudaStream_t>(p.stream);
   // staging comes from the stream-ordered pool, or from the static scratch for the no-alloc entry
   bool staged = false;   // this call launches layout adapters in front of its conv kernel
-  auto staging = [&](Scratch& s, size_t bytes, const char* what) -> void* {
+  auto staging = [&](Scratch& s, size_t bytes, const char* what, size_t counted = 0) -> void* {
     staged = true;
-    if (arena != nullptr) return arena->take(bytes, what);
+    if (arena != nullptr) return arena->take(bytes, counted != 0 ? counted : bytes, what);
     s.alloc(st, bytes, stream);
     return s.ptr;
   };
@@ -1249,12 +1265,15 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     return arena == nullptr || static_cast<long long>(arena->used) + elems * es + 1024 <= static_cast<long long>(arena->capacity);
   };
   if (!scratch_holds((N * H * W + K * R * S) * Cs)) Cs = Cp;
-  // ---- whole filter rows as k-chunks (see filter_rows_pay): the staged copy carries its horizontal padding, so the S taps of
-  // a filter row are S adjacent pixels, one run of S * Cr channels that the k-chunks cut without regard to the taps
+  const bool w_taps_dense = C == Cp && (w_in.stride[1] == 1) && w_in.stride[3] == C && w_in.stride[2] == S * C &&
+                            w_in.stride[0] == R * S * C && aligned16(w_in.ptr);
+  // ---- whole filter rows as k-chunks (see filter_row_channels): the staged copy carries its horizontal padding, so the S taps
+  // of a filter row are S adjacent pixels, one run of S * Cr channels that the k-chunks cut without regard to the taps
   const long long W_padded = W + static_cast<long long>(p.padding_w) + p.pad_w_hi;
-  const long long Cr = filter_row_channels(Cp, es, S);
-  const bool frow = stage_x && Cr != 0 && p.dilation_w == 1 && W_padded < (1LL << 30) && knobs().force_chunk == 0 &&
-                    scratch_holds((N * H * W_padded + K * R * S) * Cr);
+  const long long Cr = filter_row_channels(Cp, es, R, S, K, W, W_padded);
+  const bool frow = stage_x && Cr != 0 && p.dilation_w == 1 && W_padded < (1LL << 30) && knobs().force_chunk == 0;
+  // the plain copies that the no-alloc entry counts
+  const long long plain_bytes = (N * H * W * Cs * es + 255) / 256 * 256 + (w_taps_dense ? 0 : K * R * S * Cs * es);
   if (frow) Cs = Cr;
   if (stage_x) {   // its address is filled in below, where the weights' form is known too
     const long long row = (frow ? W_padded : W) * Cs;
@@ -1275,8 +1294,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   if (forced_chunk == 16 || forced_chunk == 32 || forced_chunk == 64 || forced_chunk == 128) chunk_bytes = forced_chunk;
   const int chunk_elems = chunk_bytes / es;
   const int chunks_per_tap = static_cast<int>((Cg + chunk_elems - 1) / chunk_elems);
-  const bool w_dense = C == Cp && (!frow || Cr == Cp) && (w_in.stride[1] == 1) && w_in.stride[3] == C &&
-                       w_in.stride[2] == S * C && w_in.stride[0] == R * S * C && aligned16(w_in.ptr);
+  const bool w_dense = w_taps_dense && (!frow || Cr == Cp);
   // Where the last chunk of a tap is partly past the channels, the TMA unit fills the activations' channels >= C with zeros,
   // but the weights need a map with one row per tap, unless there is only one tap. So do weights that are repacked with
   // padded taps, whatever the chunk (chunks that divide an unpadded tap then only come from TRACEA_B200_FORCE_CHUNK).
@@ -1327,7 +1345,8 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     tb200::CopyJob jobs[2];
     int count = 0;
     if (stage_x || stage_w) {
-      char* base = static_cast<char*>(staging(op_scratch, x_bytes + w_bytes, "the channels-last copies of x and w"));
+      char* base = static_cast<char*>(staging(op_scratch, x_bytes + w_bytes, "the channels-last copies of x and w",
+                                              frow ? static_cast<size_t>(plain_bytes) : 0));
       if (stage_x) {
         x.ptr = base;
         jobs[count++] = copy_job(x_in.ptr, x.ptr, es, N, C, Cs, H, W, x_in.stride[0], x_in.stride[1], x_in.stride[2],
