@@ -87,6 +87,22 @@ def test_filter_rows_as_chunks(dtype):
         check(case, dtype)
 
 
+# An im2col map's corners go from -128 to 127: wider paddings are refused in every memory format, also where the padding would be copied.
+@pytest.mark.parametrize("C", [20, 24, 64])
+@pytest.mark.parametrize("last", [False, True])
+def test_paddings_beyond_the_im2col_corners_are_refused(C, last):
+    fmt = torch.channels_last if last else torch.contiguous_format
+    x = torch.randn((2, C, 9, 300), device="cuda").bfloat16().contiguous(memory_format=fmt)
+    w = torch.randn((8, C, 3, 3), device="cuda").bfloat16().contiguous(memory_format=fmt)
+    got = ops.conv2d_nchw(x, w, None, None, 1, (1, 128))
+    want = torch.nn.functional.conv2d(x.double(), w.double(), padding=(1, 128))
+    assert float((got.double() - want).abs().max() / want.abs().max()) <= cc.TOL_16BIT
+    for pad in (129, 200):
+        with pytest.raises(ffi.TraceaError) as e:
+            ops.conv2d_nchw(x, w, None, None, 1, (1, pad))
+        assert e.value.status == ffi.CUDA_ERROR and "Im2col" in e.value.message
+
+
 # The phases of a transposed convolution pad front and back differently.
 @pytest.mark.parametrize("dtype", ["bf16", "f32"])
 def test_filter_rows_in_the_phases_of_a_transposed_convolution(dtype):

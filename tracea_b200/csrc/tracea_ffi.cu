@@ -1271,7 +1271,9 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   // of a filter row are S adjacent pixels, one run of S * Cr channels that the k-chunks cut without regard to the taps
   const long long W_padded = W + static_cast<long long>(p.padding_w) + p.pad_w_hi;
   const long long Cr = filter_row_channels(Cp, es, R, S, K, W, W_padded);
-  const bool frow = stage_x && Cr != 0 && p.dilation_w == 1 && W_padded < (1LL << 30) && knobs().force_chunk == 0;
+  // (paddings that an im2col map's corners cannot hold are refused, also where this form would not need them there)
+  const bool frow = stage_x && Cr != 0 && p.dilation_w == 1 && W_padded < (1LL << 30) && p.padding_w <= 128 &&
+                    p.pad_w_hi - (S - 1) <= 127 && knobs().force_chunk == 0;
   // the plain copies that the no-alloc entry counts
   const long long plain_bytes = (N * H * W * Cs * es + 255) / 256 * 256 + (w_taps_dense ? 0 : K * R * S * Cs * es);
   if (frow) Cs = Cr;
