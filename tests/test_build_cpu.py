@@ -1,6 +1,7 @@
 """What is built, and when, without running a compiler: the library for callers of the C ABI, who have neither Python nor torch,
 and the tensor front end, which fits one interpreter and one build of torch."""
 import os
+import re
 import sys
 import types
 
@@ -67,3 +68,11 @@ def test_a_front_end_of_another_torch_is_refused(monkeypatch):
     monkeypatch.setattr(ffi, "load", lambda: None)
     with pytest.raises(ImportError, match="built for torch 1.0.0"):
         ops._native()
+
+
+def test_kernels_read_tensors_with_ordinary_loads():
+    """A programmatic launch is resident while its predecessors write what it reads, which the non-coherent loads do not allow."""
+    for path in build.SOURCES + build.HEADERS:
+        with open(path) as f:
+            code = "\n".join(line.split("//")[0] for line in f)
+        assert not re.search(r"\b__ldg\b|ld\.global\S*\.nc|__builtin_nontemporal_load|__ldlu", code), path

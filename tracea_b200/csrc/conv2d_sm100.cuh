@@ -395,12 +395,20 @@ __device__ __noinline__ void coop_load_box(uint32_t stg, const OutT* row_base, l
   const uint32_t chunk = static_cast<uint32_t>(lane) & 7u;
   const bool chunk_ok = static_cast<int>(chunk) * kVec < cols_left;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = i * 4 + (lane >> 3);
-    const long long off = __shfl_sync(0xffffffffu, row_off, r);
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (chunk_ok && ((ok_rows >> r) & 1u)) v = __ldg(reinterpret_cast<const uint4*>(row_base + off) + chunk);
-    ptx::st_shared_v4(stg + static_cast<uint32_t>(r) * 128u + ((chunk ^ (static_cast<uint32_t>(r) & 7u)) << 4), v);
+  for (int half = 0; half < 2; ++half) {   // four loads in flight: eight cost the calling kernels spilled registers
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = (half * 4 + i) * 4 + (lane >> 3);
+      const long long off = __shfl_sync(0xffffffffu, row_off, r);
+      v[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (chunk_ok && ((ok_rows >> r) & 1u)) v[i] = reinterpret_cast<const uint4*>(row_base + off)[chunk];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = (half * 4 + i) * 4 + (lane >> 3);
+      ptx::st_shared_v4(stg + static_cast<uint32_t>(r) * 128u + ((chunk ^ (static_cast<uint32_t>(r) & 7u)) << 4), v[i]);
+    }
   }
   __syncwarp();   // rows were written by other lanes than the ones that read them next
 }
@@ -1163,7 +1171,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     OutT* __restrict__ out = static_cast<OutT*>(args.out);
-    const OutT* __restrict__ res = static_cast<const OutT*>(args.residual);
+    const OutT* res = static_cast<const OutT*>(args.residual);
     constexpr int kVec = 16 / sizeof(OutT);        // elements per 16-byte vector
     constexpr int kGroupCols = 128 / sizeof(OutT); // columns per 128-byte staging row
     constexpr int kGroups = BN / kGroupCols;
@@ -1193,7 +1201,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
         const int n = nt * BN + j * 32 + lane;
         float b = 0.0f;
         if (args.bias != nullptr && n < args.K_out) {
-          b = args.bias_is_f32 ? __ldg(static_cast<const float*>(args.bias) + n)
+          b = args.bias_is_f32 ? static_cast<const float*>(args.bias)[n]
                                : OutTraits<OutT>::to_f(static_cast<const OutT*>(args.bias)[n]);
         }
         bias_next[j] = b;

@@ -218,7 +218,7 @@ conv2d_small_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gr
     const int m = m0 + quarter * 16 + lane;
     const bool row_ok = lane < 16 && m < args.M;
     OutT* __restrict__ out = static_cast<OutT*>(args.out);
-    const OutT* __restrict__ res = static_cast<const OutT*>(args.residual);
+    const OutT* res = static_cast<const OutT*>(args.residual);
     const int pq = m / args.Wo;
     const int wo = m - pq * args.Wo;
     const int img = pq / args.Ho;
@@ -235,7 +235,7 @@ conv2d_small_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gr
       const int n = n_base + h * 32 + lane;
       bias_l[h] = 0.0f;
       if (args.bias != nullptr && n < args.K_out)
-        bias_l[h] = args.bias_is_f32 ? __ldg(static_cast<const float*>(args.bias) + n)
+        bias_l[h] = args.bias_is_f32 ? static_cast<const float*>(args.bias)[n]
                                      : OutTraits<OutT>::to_f(static_cast<const OutT*>(args.bias)[n]);
 #pragma unroll
       for (int c = 0; c < kChunks; ++c) {
@@ -243,7 +243,7 @@ conv2d_small_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x, const __gr
         const int col = n_base + h * 32 + c * kVec;
         if (rows && res != nullptr && row_ok && col < args.K_out) {
           if (args.res_vec == 16) {
-            res_c[h][c] = __ldg(reinterpret_cast<const uint4*>(res + col));
+            res_c[h][c] = *reinterpret_cast<const uint4*>(res + col);
           } else {
             OutT* e = reinterpret_cast<OutT*>(&res_c[h][c]);
 #pragma unroll

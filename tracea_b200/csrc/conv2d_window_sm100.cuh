@@ -421,7 +421,7 @@ conv2d_window_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x_full,
       for (int n = lane; n < kWinBN; n += 32) {
         float b = 0.0f;
         if (args.bias != nullptr && n < args.K_out)
-          b = args.bias_is_f32 ? __ldg(static_cast<const float*>(args.bias) + n)
+          b = args.bias_is_f32 ? static_cast<const float*>(args.bias)[n]
                                : OutTraits<OutT>::to_f(static_cast<const OutT*>(args.bias)[n]);
         bias_s[n] = b;
       }

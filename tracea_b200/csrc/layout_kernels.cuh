@@ -275,7 +275,7 @@ struct StemCopy {
 __device__ __forceinline__ uint2 rgb16_pixel(const uint32_t* row, int i, int W) {
   if (i < 0 || i >= W) return make_uint2(0u, 0u);
   const uint32_t* w = row + ((3 * i) >> 1);
-  const uint32_t a = __ldg(w), b = __ldg(w + 1);
+  const uint32_t a = w[0], b = w[1];
   return (i & 1) != 0 ? make_uint2((a >> 16) | (b << 16), b >> 16) : make_uint2(a, b & 0xffffu);
 }
 __global__ void __launch_bounds__(kStemThreads) rgb16_stem_copy_kernel(const __grid_constant__ StemCopy c) {
@@ -295,13 +295,22 @@ __global__ void __launch_bounds__(kStemThreads) rgb16_stem_copy_kernel(const __g
   for (int j = tid; j < c.Wp / 2; j += kStemThreads) {
     int n = n0, h = h0;
     uint4* d = reinterpret_cast<uint4*>(c.dst + static_cast<long long>(row0) * c.Wp * 4) + j;
-#pragma unroll 4
-    for (int r = 0; r < count; ++r) {
-      const uint32_t* row = reinterpret_cast<const uint32_t*>(c.src + n * c.src_img + h * c.src_row);
-      const uint2 a = rgb16_pixel(row, 2 * j - c.pad, c.W), b = rgb16_pixel(row, 2 * j + 1 - c.pad, c.W);
-      *d = make_uint4(a.x, a.y, b.x, b.y);
-      d += c.Wp / 2;
-      if (++h == c.H) { h = 0; ++n; }
+    for (int r0 = 0; r0 < count; r0 += kStemRows / 2) {
+      uint4 v[kStemRows / 2];
+#pragma unroll
+      for (int k = 0; k < kStemRows / 2; ++k) {
+        if (r0 + k >= count) break;
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(c.src + n * c.src_img + h * c.src_row);
+        const uint2 a = rgb16_pixel(row, 2 * j - c.pad, c.W), b = rgb16_pixel(row, 2 * j + 1 - c.pad, c.W);
+        v[k] = make_uint4(a.x, a.y, b.x, b.y);
+        if (++h == c.H) { h = 0; ++n; }
+      }
+#pragma unroll
+      for (int k = 0; k < kStemRows / 2; ++k) {
+        if (r0 + k >= count) break;
+        *d = v[k];
+        d += c.Wp / 2;
+      }
     }
   }
 }

@@ -42,6 +42,9 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 // visible (at once when there is no such dependency); nothing the earlier kernel wrote may be read, and nothing it
 // reads may be overwritten, before it. `griddep_launch_dependents` lets the NEXT kernel on the stream be scheduled
 // as soon as every CTA of this grid has called it (or exited).
+// Under such a launch a kernel is resident while the launches before it still write what it is going to read. The non-coherent
+// loads (__ldg, ld.global.nc) are only specified for memory that nothing writes as long as the kernel lives: tensors, biases and
+// scratch are read with ordinary loads, behind the wait.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
