@@ -167,15 +167,17 @@ def test_rgb_stem_copies(case):
 
 
 # Calls right behind one another hand the same scratch on: the copy and the packed filter bank of one are rewritten for the next
-# while the launch that read them drains. Two banks and two images in turn, one image being the least work a launch can have.
+# while the launch that read them drains. Three banks and two inputs in turn; one image is the least work a launch can have, and with 300
+# the copy is more than a wave, which the next launch does not start beside.
+@pytest.mark.parametrize("images", [1, 300])
 @pytest.mark.parametrize("dtype", ["bf16", "f16"])
-def test_rgb_stems_behind_one_another(dtype):
-    xs = [torch.from_numpy(cc.normal((1, 40, 66, 3), 61 + i, "stems/x")).to(TORCH_DT[dtype]).cuda() for i in range(2)]
+def test_rgb_stems_behind_one_another(dtype, images):
+    xs = [torch.from_numpy(cc.normal((images, 40, 66, 3), 61 + i, "stems/x")).to(TORCH_DT[dtype]).cuda() for i in range(2)]
     ws = [torch.from_numpy(cc.normal((64, 7, 7, 3), 63 + i, "stems/w", 0.1)).to(TORCH_DT[dtype]).cuda() for i in range(3)]
     want = {}
     for i, x in enumerate(xs):
         for k, w in enumerate(ws):
             want[i, k] = ops.conv2d(x, w, None, None, "relu", 2, 3)
             torch.cuda.synchronize()
-    got = [(n % 2, n % 3, ops.conv2d(xs[n % 2], ws[n % 3], None, None, "relu", 2, 3)) for n in range(240)]
+    got = [(n % 2, n % 3, ops.conv2d(xs[n % 2], ws[n % 3], None, None, "relu", 2, 3)) for n in range(240 if images == 1 else 24)]
     assert all(torch.equal(out, want[i, k]) for i, k, out in got)

@@ -260,11 +260,16 @@ __global__ void pack_weights_krsc_kernel(const T* __restrict__ src, T* __restric
 // source of two neighbouring destination pixels into one 16-byte store, so that a warp's store covers 512 consecutive bytes (as
 // four 8-byte stores a thread, 32 bytes apart, a store touched every sector a quarter at a time); kStemRows rows a block, their
 // loads in flight together. Pixels outside the image are zeros. Rows of the source start on 4-byte boundaries, W and Wp are even.
+// Whole calls of the 7x7/2 stem at 224x224, bf16, with the copy and the packing as two ordinary launches (four pixels a thread) and
+// with this one: 1 image 9.2 -> 9.0 us replayed and 15.8 -> 12.2 issued one by one, 32 images 29.7 -> 28.8, 256 173 -> 163, 512 337 -> 316.
+// The launch behind it may only come up beside its last blocks while the copy is about a wave (`early`): with more, calls issued one
+// behind another took 181 us at 256 images and 350 at 512 (1 image without: 9.4). Why is not established.
 constexpr int kStemThreads = 128, kStemRows = 8;
 struct StemCopy {
   const uint16_t* src;
   uint16_t* dst;
   int H, W, Wp, pad, rows, image_blocks;   // rows: N * H
+  int early;                               // let the next launch start before this one is done
   long long src_img, src_row;
   const uint16_t* w;
   uint16_t* w_dst;
@@ -279,7 +284,7 @@ __device__ __forceinline__ uint2 rgb16_pixel(const uint32_t* row, int i, int W) 
   return (i & 1) != 0 ? make_uint2((a >> 16) | (b << 16), b >> 16) : make_uint2(a, b & 0xffffu);
 }
 __global__ void __launch_bounds__(kStemThreads) rgb16_stem_copy_kernel(const __grid_constant__ StemCopy c) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (c.early != 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int tid = static_cast<int>(threadIdx.x);
   if (static_cast<int>(blockIdx.x) >= c.image_blocks) {

@@ -864,6 +864,7 @@ bool try_row_band_conv(DeviceState& st, Staging&& staging, const View4& x, const
     c.sk = w.stride[0]; c.sc = w.stride[1]; c.sr = w.stride[2]; c.ss = w.stride[3];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(c.image_blocks + (c.w_total + tb200::kStemThreads - 1) / tb200::kStemThreads));
+    c.early = static_cast<long long>(cfg.gridDim.x) <= 8LL * st.num_sms ? 1 : 0;
     cfg.blockDim = dim3(tb200::kStemThreads);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
