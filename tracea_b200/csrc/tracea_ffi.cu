@@ -687,7 +687,7 @@ tb200::CopyJob copy_job(const void* src, void* dst, int es, long long N, long lo
   tb200::CopyJob j;
   memset(&j, 0, sizeof(j));
   j.src = src; j.dst = dst;
-  j.N = N; j.C = (int)C; j.Cp = (int)Cp; j.P = (int)(H * W); j.W = (int)W;
+  j.N = N; j.C = (int)C; j.Cp = (int)Cp; j.P = (int)(H * W); j.W = (int)W; j.H = (int)H;
   j.pad_lo = (int)pad_lo; j.pad_hi = (int)pad_hi;
   j.sn = sn; j.sc = sc; j.sh = sh; j.sw = sw;
   j.vec = 1;
@@ -740,8 +740,13 @@ void launch_copies(const tb200::CopyJob* jobs, int count, int es, cudaStream_t s
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = knobs().pdl != 0 ? 1 : 0;
-  if (es == 2) TB_CUDA(cudaLaunchKernelEx(&cfg, tb200::copy_channels_last_kernel<uint16_t>, pack));
-  else TB_CUDA(cudaLaunchKernelEx(&cfg, tb200::copy_channels_last_kernel<uint32_t>, pack));
+  const bool padded = (pack.job[0].pad_lo | pack.job[0].pad_hi) != 0;   // x, if there is padding, is the first job
+  if (es == 2)
+    TB_CUDA(padded ? cudaLaunchKernelEx(&cfg, tb200::copy_channels_last_kernel<uint16_t, true>, pack)
+                   : cudaLaunchKernelEx(&cfg, tb200::copy_channels_last_kernel<uint16_t, false>, pack));
+  else
+    TB_CUDA(padded ? cudaLaunchKernelEx(&cfg, tb200::copy_channels_last_kernel<uint32_t, true>, pack)
+                   : cudaLaunchKernelEx(&cfg, tb200::copy_channels_last_kernel<uint32_t, false>, pack));
   TB_CUDA(cudaGetLastError());
   g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
   g_launches_by_kind[3].fetch_add(1, std::memory_order_relaxed);
