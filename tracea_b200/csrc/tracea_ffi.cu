@@ -372,13 +372,17 @@ struct Tiling {
 //  * a tile hides the epilogue of the one before it (640 cycles per 128 bytes of columns, a quarter more with a residual, a fifth
 //    more for per-lane stores; two groups take alternate tiles, or a row block each), or waits for it, and costs 420 on top;
 //  * the first tile's walk and the last one's epilogue have nothing to hide them or hide behind; a pair costs 1040 once.
+//  * where a filter tap's pixels start inside 128-byte lines (C * element size no multiple of 128, taps one by one), every row of
+//    an operand is two lines to fetch: a k-step takes at least 24 cycles per KB (3 per row), however few SMs are at work.
 // Two row blocks from 7 k-steps on and pairs from 8 on: below, the epilogue sets the pace, and both tie more of it together.
 // (Fitted to 91 layers and products in all six tilings; the pick is 0.9 % above the best of the six on average. The rule before it,
 // which only counted waves, took: 3x3 192->192 on 16 images of 28x28 13.9 -> 11.4 us, 1x1 512->2048 + residual on 64 of 7x7 12.4
 // -> 10.2, 1x1 64->256 on 8 NCHW images of 56x56 13.3 -> 11.1, 1x1 64->320 fp32 on 19 of 70x70 108 -> 72, 8192 x 512 x 512 8.8
-// -> 7.9, 1500 x 3072 x 768 10.4 -> 9.3.)
+// -> 7.9, 1500 x 3072 x 768 10.4 -> 9.3. 18 more layers whose pixels are no whole lines, all forms: without the last rule the
+// pick is 9.6 % above the best, with it 0.2 % -- 3x3 328->320 on 80 images of 14x14 70.5 -> 51.1 us, 232->256 51.6 -> 37.6, 264->704
+// dilated 66.3 -> 48.8, 168->200 /2 on 60 of 28x28 23.4 -> 19.1 -- and 95 drawn ones do not change.)
 Tiling pick_tiling(long long M, long long K_out, long long k_steps, int es, bool residual, bool per_lane, bool whole_stage,
-                   int num_sms, int forced_bn, int pair_env, int rows2_env) {
+                   bool split_lines, int num_sms, int forced_bn, int pair_env, int rows2_env) {
   struct Form {
     int bn;
     bool pair, rows2;
@@ -401,7 +405,8 @@ Tiling pick_tiling(long long M, long long K_out, long long k_steps, int es, bool
     const long long workers = f.pair ? num_sms / 2 : num_sms;
     const long long waves = (tiles + workers - 1) / workers;
     const long long busy = std::min<long long>(num_sms, tiles * (f.pair ? 2 : 1) / waves);
-    const long long walk = k_steps * std::max<long long>(f.step, f.kbytes * 1024 * busy / (87LL * num_sms));
+    const long long step = split_lines ? std::max(f.step, 24 * f.kbytes) : f.step;
+    const long long walk = k_steps * std::max<long long>(step, f.kbytes * 1024 * busy / (87LL * num_sms));
     long long epi = 640LL * f.bn * es / 128;
     if (residual) epi = epi * 5 / 4;
     if (per_lane) epi = epi * 6 / 5;
@@ -1384,8 +1389,9 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   const long long m_tiles_128 = (M + tb200::kBlockM - 1) / tb200::kBlockM;
   const int forced_bn = knobs().force_bn == 64 || knobs().force_bn == 128 || knobs().force_bn == 256 ? knobs().force_bn : 0;
   const int pair_env = knobs().pair, rows2_env = knobs().rows2;
+  const bool split_lines = !window && !frow && R * S > 1 && x.stride[3] * es % 128 != 0;
   const Tiling tiling = pick_tiling(M, K, (total_chunks_ll * chunk_bytes + 127) / 128, es, epi.residual, out.stride[1] != 1,
-                                    chunk_bytes == 128, st.num_sms, forced_bn, pair_env, rows2_env);
+                                    chunk_bytes == 128, split_lines, st.num_sms, forced_bn, pair_env, rows2_env);
   const int bn = tiling.bn;
   const bool pair = tiling.pair, rows2 = tiling.rows2;
   const long long n_tiles = (K + bn - 1) / bn;
