@@ -83,7 +83,8 @@ def test_filter_rows_as_chunks(dtype):
                  (2, 50, 9, 11, 33, 3, 1, 1, "residual+relu", True), (1, 17, 1, 1, 20, 3, 1, 1, "bias", False),
                  (2, 25, 8, 6, 40, 2, 1, 0, "relu", False), (1, 200, 12, 12, 130, 3, 1, 0, "bias+silu", False),
                  (40, 40, 28, 28, 64, 3, 1, 1, "bias+relu", False), (1, 11, 30, 30, 9, 16, 1, 8, "bias", False),
-                 (2, 9, 5, 7, 70, 5, 3, 2, "bias", True)):
+                 (2, 9, 5, 7, 70, 5, 3, 2, "bias", True), (2, 104, 11, 13, 40, 7, 1, 3, "bias+relu", False),
+                 (1, 200, 9, 10, 33, 5, 2, 2, "bias", False), (3, 100, 10, 9, 70, 7, 1, 3, "silu", False)):
         check(case, dtype)
 
 

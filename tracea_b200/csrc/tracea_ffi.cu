@@ -438,8 +438,9 @@ constexpr long long kFilterRowBankBytes = 16LL << 20;   // larger filter banks g
 
 // Whether the S taps of a filter row, as one run of channels, take fewer k-chunks than tap by tap -- a k-chunk is a copy of
 // either operand, and with few channels those are what a walk takes its time for; returns the channels per pixel of that form, 0
-// if not. Pixels start on 32-byte sectors where that takes no chunk more (40 channels would: 15.2 us exact, 21.7 rounded up;
-// 24 channels 15.4 and 13.6). NCHW calls, tap by tap and by filter rows, us: 5x5 20->50 + GELU on 3 images of 72x72 19.0 and
+// if not. Pixels start on 32-byte sectors where that takes at most a chunk in nine more (40 channels, 3x3, would take half as many
+// more: 15.2 us exact, 21.7 rounded up; 24 channels 15.4 and 13.6; 7x7, 200 -> 64 on 4 images of 28x28 51.8 and 25.9, tap by tap
+// 49.4; 7x7 104->64 on 9 32.3 and 25.0; 5x5 200->64 on 9 32.9 and 25.9, tap by tap 31.2). NCHW calls, tap by tap and by filter rows, us: 5x5 20->50 + GELU on 3 images of 72x72 19.0 and
 // 13.2; 3x3 20->50 13.9 and 11.7; 3x3 40->64 on 8 images of 56x56 20.8 and 15.2; 3x3 80->128 on 8 of 28x28 13.3 and 12.4; 5x5
 // 48->96 36.7 and 29.7; 7x7/2 12->64 fp32 on 8 of 112x112 43.7 and 23.3; 3x3 104->128 on 32 of 28x28 26.5 and 23.6.
 // The copy carries the padding, so on images a few pixels wide it grows: not where it doubles, nor by more than 256 bytes a
@@ -452,7 +453,7 @@ long long filter_row_channels(long long Cp, int es, long long R, long long S, lo
   const long long aligned = (Cp * es + 31) / 32 * 32 / es;
   const long long by_tap = S * chunks(Cp * es), exact = chunks(S * Cp * es), wide = chunks(S * aligned * es);
   if (std::min(exact, wide) >= by_tap) return 0;
-  const long long Cr = wide <= exact ? aligned : Cp;
+  const long long Cr = wide < by_tap && 8 * wide <= 9 * exact ? aligned : Cp;
   if (3 * (W_padded - W) * Cr * es > 256 * R * W || K * R * S * Cr * es > kFilterRowBankBytes) return 0;
   return Cr;
 }
