@@ -278,7 +278,7 @@ uint64_t tracea_b200_launch_count(void);
 /* The same count for one kind of kernel: 0 the general implicit-GEMM conv kernel, 1 its instantiations that cut tiles
  * over K, 2 the resident-filter kernel (stride-1 small filters over 64-channel activations), 3 layout adapters,
  * 4 the row-band kernel (few-channel 16-bit images such as the RGB stem), 5 the small-tile kernel (problems of up to one
- * wave of 64-row tiles).
+ * wave of 64-row tiles); and 6, those of 0, 1 and 5 that read a copied input by whole filter rows instead of tap by tap.
  * Lets tests and benchmarks see which path a call took. 0 for any other `kind`. No counterpart in the reference. */
 uint64_t tracea_b200_launch_count_of(int32_t kind);
 

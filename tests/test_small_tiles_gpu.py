@@ -19,8 +19,8 @@ TORCH_DT = {"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}
 
 # N, C, H, W, K, R, stride, pad, epilogue, channels-last: tile and k-step edges -- one to three and many k-steps (two share a
 # stage, four stages are in flight), 1 / 63 / 64 / 65 pixels, 1 / 31 / 33 / 64 / 65 / 130 output channels, ragged channel
-# counts, a plain matrix and an im2col A operand, both memory formats. With im2col copies the kernel is chosen for up to 31
-# k-steps of 128 bytes.
+# counts, a plain matrix and an im2col A operand, both memory formats. With im2col copies 32-wide tiles are chosen whatever the number
+# of k-steps, 64-wide ones up to 34 of 128 bytes.
 CASES = [
     (1, 64, 1, 1, 64, 1, 1, 0, "bias", True), (1, 128, 7, 9, 33, 1, 1, 0, "relu", True),
     (1, 192, 8, 8, 65, 1, 1, 0, "bias+residual+relu", True), (5, 64, 13, 1, 31, 1, 1, 0, "gelu", True),
@@ -36,7 +36,7 @@ CASES = [
     (2, 192, 14, 14, 1000, 1, 1, 0, "bias+residual+relu", False), (2, 96, 14, 14, 1000, 1, 1, 0, "gelu", True),
     (1, 128, 24, 24, 600, 2, 1, 0, "bias+residual", True),
 ]
-# 64-wide tiles with an im2col operand, the ring filled twice and more: up to 17 k-steps of 128 bytes
+# 64-wide tiles with an im2col operand, the ring filled twice and more: 16 and 9 k-steps of 128 bytes
 CASES_OF = {
     2: [(1, 256, 24, 24, 600, 2, 1, 0, "bias+silu", True), (1, 64, 24, 24, 601, 3, 1, 1, "bias+residual+relu", False)],
     4: [(1, 128, 24, 24, 600, 2, 1, 0, "bias+silu", True), (1, 32, 24, 24, 601, 3, 1, 1, "bias+residual+relu", False)],

@@ -94,7 +94,9 @@ def test_noalloc_entry_keeps_the_order_of_summation_up_to_its_limit(dtype, N, C,
     w = (torch.randn((K, C, 5, 5), generator=g, device="cuda") * 0.05).to(dt)
     run = lambda e, t: _call(e, t, w, None, None, torch.empty((t.shape[0], K, H, W), dtype=dt, device="cuda"), 1, 2,
                              ffi.EPILOGUE_IDENTITY)
+    before = ffi.launch_count_of(ffi.FORM_FILTER_ROWS)
     want, got = run("tracea_conv2d", x), run("tracea_conv2d_noalloc", x)
+    assert ffi.launch_count_of(ffi.FORM_FILTER_ROWS) == before + 2
     assert torch.equal(got, want)
     for e in ("tracea_conv2d", "tracea_conv2d_noalloc"):
         assert torch.equal(run(e, x[N - 1:].clone()), want[N - 1:])

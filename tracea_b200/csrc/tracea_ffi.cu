@@ -111,8 +111,8 @@ std::atomic<int> g_test_producer_stop{-1};
 std::atomic<bool> g_attr_set[kMaxDevices][3][3][3 * (tb200::kNumStores + 2)];
 std::atomic<unsigned long long> g_kernel_launches{0};   // every kernel this library has launched (conv + layout adapters)
 // the same, by kind: 0 general implicit-GEMM kernel, 1 its K-split instantiations, 2 resident-filter kernel, 3 layout adapters,
-// 4 row-band kernel, 5 small-tile kernel
-constexpr int kLaunchKinds = 6;
+// 4 row-band kernel, 5 small-tile kernel; and 6, those of 0, 1 and 5 whose k-chunks run over whole filter rows
+constexpr int kLaunchKinds = 7;
 std::atomic<unsigned long long> g_launches_by_kind[kLaunchKinds];
 EncodeTiledFn g_encode_tiled = nullptr;
 EncodeIm2colFn g_encode_im2col = nullptr;
@@ -1374,6 +1374,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
     }
     launch_copies(jobs, count, es, stream);
   }
+  if (frow) g_launches_by_kind[6].fetch_add(1, std::memory_order_relaxed);
 
   const long long Kgemm = R * Sg * Cg;
 

@@ -218,11 +218,11 @@ def conv_transpose2d_raw(x, w, bias, residual, out, stride=(1, 1), padding=(0, 0
 
 
 (KERNEL_GENERAL, KERNEL_SPLIT_K, KERNEL_RESIDENT_FILTER, KERNEL_LAYOUT, KERNEL_ROW_BAND,
- KERNEL_SMALL_TILE) = range(6)
+ KERNEL_SMALL_TILE, FORM_FILTER_ROWS) = range(7)
 
 
 def launch_count_of(kind):
-    """Launches so far of one kind of kernel (KERNEL_* above)."""
+    """Launches so far of one kind of kernel (KERNEL_* above; FORM_FILTER_ROWS: those whose k-chunks are whole filter rows)."""
     return int(load().tracea_b200_launch_count_of(kind))
 
 
