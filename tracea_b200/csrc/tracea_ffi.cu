@@ -1388,7 +1388,6 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   }
 
   // ---- tiling of the whole problem. TRACEA_B200_FORCE_BN / _PAIR / _ROWS2 narrow the choice.
-  const long long m_tiles_128 = (M + tb200::kBlockM - 1) / tb200::kBlockM;
   const int forced_bn = knobs().force_bn == 64 || knobs().force_bn == 128 || knobs().force_bn == 256 ? knobs().force_bn : 0;
   const int pair_env = knobs().pair, rows2_env = knobs().rows2;
   const bool split_lines = !window && !frow && R * S > 1 && x.stride[3] * es % 128 != 0;
@@ -1397,8 +1396,6 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   const int bn = tiling.bn;
   const bool pair = tiling.pair, rows2 = tiling.rows2;
   const long long n_tiles = (K + bn - 1) / bn;
-  const long long waves_128 = (m_tiles_128 * n_tiles + st.num_sms - 1) / st.num_sms;
-  const long long waves_256 = ((m_tiles_128 + 1) / 2 * n_tiles + st.num_sms - 1) / st.num_sms;
 
   // ---- problems of up to one wave: the small-tile kernel (conv2d_small_sm100.cuh). Where two k-steps come in one copy per
   // operand -- 1x1 convolutions and products over whole 128-byte chunks -- a k-step takes it about half the general kernel's
@@ -1409,7 +1406,10 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   // 5.9, 256 channels on ten 14x14 images 9.7 -> 9.0): their step is put at 355, which leaves walks of more than 34 steps to the
   // general kernel. Pixels that do not start on 32-byte sectors cost every copy sectors that it shares with its neighbours: 120
   // channels, 106 / 144 tiles, 9.4 -> 10.3 and 9.6 -> 9.8; those keep the earlier costs. More than one tile
-  // per SM gains nothing (1x1 64->64 at 4 images: 196 tiles, 3.65 -> 3.88). Costs in cycles.
+  // per SM gains nothing (1x1 64->64 at 4 images: 196 tiles, 3.65 -> 3.88). Costs in cycles. What they are compared with is one wave of
+  // the general kernel's single 64-column tiles: where 64-row tiles fit the SMs, pick_tiling takes no other form (23 million draws of
+  // rows, columns, steps and forms of output). Its 300 cycles a step and 1900 for what its epilogue takes longer are this rule's own
+  // scale, on which the costs above were fitted to calls timed in both kernels.
   const bool whole_chunks = chunk_bytes == 128 && row_bytes % 128 == 0;
   const bool plain_a = whole_chunks && !window && R == 1 && S == 1 && p.stride_h == 1 && p.stride_w == 1 &&
                        p.padding_h == 0 && p.padding_w == 0 && p.pad_h_hi == 0 && p.pad_w_hi == 0 &&
@@ -1418,10 +1418,7 @@ void conv2d_core(DeviceState& st, StaticArena* arena, const View4& x_in, const V
   if (chunk_bytes == 128 && forced_bn == 0 && pair_env == -1 && rows2_env == -1 && knobs().split_k == 0 &&
       knobs().tiled_a == 0) {
     const long long k_steps = total_chunks_ll;
-    const long long pair_waves = ((m_tiles_128 + 1) / 2 * n_tiles + st.num_sms / 2 - 1) / std::max(1, st.num_sms / 2);
-    const long long general = pair ? pair_waves * 512 : (rows2 ? waves_256 * (bn == 128 ? 640 : 480)
-                                                              : waves_128 * (bn == 256 ? 512 : (bn == 128 ? 400 : 300)));
-    long long best = general * k_steps + 1900;
+    long long best = k_steps * 300 + 1900;   // one wave of the general kernel's 64-column tiles
     const long long m_tiles_64 = (M + tb200::kSmallM - 1) / tb200::kSmallM;
     for (int b = 64; b >= 32; b >>= 1) {
       if (m_tiles_64 * ((K + b - 1) / b) > st.num_sms) continue;
