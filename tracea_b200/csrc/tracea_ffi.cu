@@ -1083,8 +1083,10 @@ bool try_resident_filter_conv(DeviceState& st, const View4& x, const void* w_ptr
   if (q.pair_tiles < pairs || q.pair_tiles > 0x3fffffffLL) return false;
   // Tall tiles read the least halo, but few of them leave pairs idle, and what runs before the first tile's epilogue grows with a
   // tile: shorter ones where that shortens the busiest pair's walk, in cycles -- 3800 for a block's epilogue, two blocks at a
-  // time, the first window's copy and the first tile's MMAs on top. Measured with nine taps; with four, where epilogues compete
-  // with fewer MMAs, shorter tiles lose (2x2 on 80 images of 56x56: 20.5 -> 23.2 us). (3x3 64->64, tiles of 9 and 4 rows at
+  // time, the first window's copy and the first tile's MMAs on top. For nine taps only: with fewer, where epilogues compete with fewer
+  // MMAs, shorter tiles lose on larger batches (2x2 on 80 images of 56x56: 20.5 -> 23.2 us; 2x3 21.8 -> 25.9, on 20 of 112x112
+  // 22.5 -> 24.9; 3x2 21.9 -> 25.0 and 21.8 -> 22.9), although six taps gain on small ones (2x3 / 3x2 on 32 of 56x56 14.7 -> 14.4 /
+  // 14.4 -> 13.9, on 40 of 40x40 10.4 -> 9.3 / 10.9 -> 9.8). (3x3 64->64, tiles of 9 and 4 rows at
   // 56x56 on 32 images 15.1 and 13.4 us, of 12 and 6 rows at 40x40 on 40 images 12.0 and 10.9; on 64 images of 56x56 both take
   // 18.6.)
   auto cost = [&](const Plan& v) {
