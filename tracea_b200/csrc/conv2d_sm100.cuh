@@ -1177,7 +1177,6 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
     constexpr int kGroups = BN / kGroupCols;
     constexpr int kLdPerGroup = kGroupCols / 32;
     constexpr int kChunksPerLd = 32 / kVec;        // 16-byte chunks produced per 32-column TMEM load
-    // with a shared copy every warp writes the same values to the same words before it reads them
     // the tile's columns of the shared copy start bias_step floats further down per column tile; every warp writes the same values
     // there before it reads them
     const int bias_slot = args.shared_bias >= 0 ? 0 : ew * BN;
@@ -1201,7 +1200,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
         const int n = nt * BN + j * 32 + lane;
         float b = 0.0f;
         if (args.bias != nullptr && n < args.K_out) {
-          b = args.bias_is_f32 ? static_cast<const float*>(args.bias)[n]
+          b = args.bias_is_f32 ? ld_global_f32(static_cast<const float*>(args.bias) + n)
                                : OutTraits<OutT>::to_f(static_cast<const OutT*>(args.bias)[n]);
         }
         bias_next[j] = b;
@@ -1333,6 +1332,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
       const int g_step = shared ? 2 : 1;
       const uint32_t use = static_cast<uint32_t>(local_tile >> 1);
       const int n_base = n_tile * BN;
+      const uint32_t bias_tile_s = bias_w_s + static_cast<uint32_t>(n_tile * bias_step) * 4u;
       const int row_block = kPair ? static_cast<int>(cta_rank) : (kRows2 ? egroup : 0);   // which 128 rows of the tile
       const int m_row0 = args.m_begin + m_tile * kTileM + row_block * kBlockM + quarter * 32;
 
@@ -1465,7 +1465,7 @@ conv2d_igemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_x,
           for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[h][j]);
 #pragma unroll
           for (int j4 = 0; j4 < 8; ++j4) {
-            const float4 b4 = ld_shared_f4(bias_w_s + static_cast<uint32_t>(n_tile * bias_step + g * kGroupCols + h * 32 + j4 * 4) * 4u);
+            const float4 b4 = ld_shared_f4(bias_tile_s + static_cast<uint32_t>(g * kGroupCols + h * 32 + j4 * 4) * 4u);
             add2(f[j4 * 4 + 0], f[j4 * 4 + 1], b4.x, b4.y);
             add2(f[j4 * 4 + 2], f[j4 * 4 + 3], b4.z, b4.w);
           }
